@@ -25,7 +25,8 @@ struct BatchMember {
     Geo g;
     float dx, dt;
     double dtd;
-    int S, adv_den, nzone, pad;
+    int S, adv_den, nzone, epoch;
+    int *flags;
     const float *u, *v, *w, *rho, *jac, *ju, *jv, *jw, *dz;
     float *Um, *Vm, *Wm, *Gc, *DJR, *Wp;
     const float *filter;
@@ -91,12 +92,15 @@ __global__ void k_batch_prep(const BatchMember *__restrict__ mem, const int *__r
     if (j >= nj) return;
     const int adv_den = m.adv_den;
     const float dt = m.dt, dx = m.dx;
+    bool bad = false, tie = false;
     if (j < g.ny) {
         size_t c = ix(g, i, k, j);
         if (i >= 1 && i <= g.nx - 1) {
             float rr = adv_den ? m.rho[c] : 1.0f;
             float rl = adv_den ? m.rho[c - 1] : 1.0f;
-            m.Um[c] = m.u[c] * dt * (rr + rl) * 0.5f * m.ju[c] / dx;
+            const float um = m.u[c] * dt * (rr + rl) * 0.5f * m.ju[c] / dx;
+            m.Um[c] = um;
+            bad |= !exact_wind(um);
         } else {
             m.Um[c] = 0.0f;
         }
@@ -111,9 +115,12 @@ __global__ void k_batch_prep(const BatchMember *__restrict__ mem, const int *__r
             }
             m.Wm[c] = wm;
             const float d = m.dz[c], jj = m.jac[c], rh = m.rho[c];
-            m.Gc[c] = jj * rh;
-            m.DJR[c] = d * jj * rh;
-            m.Wp[c] = wm / d;
+            const float G = jj * rh, D = d * jj * rh, wp = wm / d;
+            m.Gc[c] = G;
+            m.DJR[c] = D;
+            m.Wp[c] = wp;
+            bad |= !exact_wind(wp) || !(fabsf(wm) < 0x1p20f) || !exact_metric(G) || !exact_metric(D) || !exact_metric(d);
+            tie |= tie_divisor(G) || tie_divisor(D);
         }
     }
     if (i < g.nx) {
@@ -121,11 +128,15 @@ __global__ void k_batch_prep(const BatchMember *__restrict__ mem, const int *__r
         if (j >= 1 && j <= g.ny - 1) {
             float rr = adv_den ? m.rho[c] : 1.0f;
             float rl = adv_den ? m.rho[ix(g, i, k, j - 1)] : 1.0f;
-            m.Vm[c] = m.v[c] * dt * (rr + rl) * 0.5f * m.jv[c] / dx;
+            const float vm = m.v[c] * dt * (rr + rl) * 0.5f * m.jv[c] / dx;
+            m.Vm[c] = vm;
+            bad |= !exact_wind(vm);
         } else {
             m.Vm[c] = 0.0f;
         }
     }
+    if (bad && m.flags) m.flags[FLAG_IEEE] = m.epoch;
+    if (tie && m.flags) m.flags[FLAG_TIE] = m.epoch;
 }
 
 // Donor-cell pass of every member: prefix over members of

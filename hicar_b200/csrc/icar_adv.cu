@@ -100,7 +100,10 @@ struct icar_adv_domain {
     std::vector<const float *> map_tag[2];
     int map_next = 0;
     int *op_err = nullptr;
+    int *op_flags = nullptr;   // icar::N_FLAGS words the prep kernels set to a step's epoch
+    int op_epoch = 0;
     bool op_ready = false;
+    int nsm = 148;     // SMs of the device
     int mp_shape = 1;  // tile shape of the fused correction kernel (icar::mp_shape_ty)
     int sp_group = 0;  // species per thread of the fused upwind pass (0 = all)
     // diagnostics: launch counter and optional event timing of the species kernels
@@ -721,7 +724,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tma_encoder()
     return fn;
 }
 
-// Descriptor of one pitched 3-D field (rows = ny or ny+1) for 64 x 1 x 32
+// Descriptor of one pitched 3-D field (rows = ny or ny+1) for 64 x 1 x 28
 // plane boxes; cached per device address.
 int plane_map(icar_adv_t *h, const float *base, int rows, const CUtensorMap **out)
 {
@@ -786,13 +789,13 @@ int onepass_maps(icar_adv_t *h, const CUtensorMap **out)
     return ICAR_ADV_OK;
 }
 
-template <bool EXACT>
+template <int M>
 cudaError_t onepass_attr()
 {
-    cudaError_t e = cudaFuncSetAttribute(icar::k_mpdata_onepass<EXACT, true>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)icar::op::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(icar::k_mpdata_onepass<M, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)icar::op::SMEM);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(icar::k_mpdata_onepass<EXACT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        e = cudaFuncSetAttribute(icar::k_mpdata_onepass<M, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)icar::op::SMEM);
     return e;
 }
@@ -811,8 +814,13 @@ int ensure_onepass(icar_adv_t *h)
             CUDA_TRY(h, dev_alloc(h, (void **)&h->op_err, sizeof(int)));
             CUDA_TRY(h, cudaMemsetAsync(h->op_err, 0, sizeof(int), h->stream));
         }
-        cudaError_t ce = onepass_attr<true>();
-        if (ce == cudaSuccess) ce = onepass_attr<false>();
+        if (!h->op_flags) {
+            CUDA_TRY(h, dev_alloc(h, (void **)&h->op_flags, icar::N_FLAGS * sizeof(int)));
+            CUDA_TRY(h, cudaMemsetAsync(h->op_flags, 0, icar::N_FLAGS * sizeof(int), h->stream));
+        }
+        cudaError_t ce = onepass_attr<icar::opx::A_EXACT>();
+        if (ce == cudaSuccess) ce = onepass_attr<icar::opx::A_FAST>();
+        if (ce == cudaSuccess) ce = cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, h->desc.device);
         if (ce != cudaSuccess) return fail(h, ICAR_ADV_CUDA_ERROR, "cudaFuncSetAttribute: %s", cudaGetErrorString(ce));
         h->op_ready = true;
     }
@@ -840,10 +848,15 @@ int mpdata_onepass_group(icar_adv_t *h, int s0, int s1)
     prm.DJR = h->DJR.p;
     prm.dz = h->dz.p;
     prm.err = h->op_err;
+    prm.flags = h->op_flags;
+    prm.epoch = h->op_epoch;
+    prm.nzero = -0.0f;
     prm.g = g;
     prm.nspecies = S;
     prm.tiles_x = onepass_tiles_x(g);
-    const unsigned grid = (unsigned)(onepass_tiles_x(g) * onepass_tiles_y(g) * S);
+    const int tiles = onepass_tiles_x(g) * onepass_tiles_y(g) * S;
+    prm.klen = icar::op::levels_per_cta(tiles, g.nz, h->nsm);
+    const unsigned grid = (unsigned)tiles * (unsigned)((g.nz + prm.klen - 1) / prm.klen);
     const bool exact = h->path != 3, fct = h->opts.mpdata_fct != 0;
     cudaEvent_t c0 = nullptr, c1 = nullptr;
     if (h->profiling) {
@@ -851,10 +864,12 @@ int mpdata_onepass_group(icar_adv_t *h, int s0, int s1)
         cudaEventCreate(&c1);
         cudaEventRecord(c0, h->stream);
     }
-    if (exact && fct) icar::k_mpdata_onepass<true, true><<<grid, icar::op::NT, icar::op::SMEM, h->stream>>>(prm);
-    else if (exact) icar::k_mpdata_onepass<true, false><<<grid, icar::op::NT, icar::op::SMEM, h->stream>>>(prm);
-    else if (fct) icar::k_mpdata_onepass<false, true><<<grid, icar::op::NT, icar::op::SMEM, h->stream>>>(prm);
-    else icar::k_mpdata_onepass<false, false><<<grid, icar::op::NT, icar::op::SMEM, h->stream>>>(prm);
+    using icar::opx::A_EXACT;
+    using icar::opx::A_FAST;
+    if (exact && fct) icar::k_mpdata_onepass<A_EXACT, true><<<grid, icar::op::NT, icar::op::SMEM, h->stream>>>(prm);
+    else if (exact) icar::k_mpdata_onepass<A_EXACT, false><<<grid, icar::op::NT, icar::op::SMEM, h->stream>>>(prm);
+    else if (fct) icar::k_mpdata_onepass<A_FAST, true><<<grid, icar::op::NT, icar::op::SMEM, h->stream>>>(prm);
+    else icar::k_mpdata_onepass<A_FAST, false><<<grid, icar::op::NT, icar::op::SMEM, h->stream>>>(prm);
     if (h->profiling) {
         cudaEventRecord(c1, h->stream);
         h->corr_events.emplace_back(c0, c1);
@@ -872,7 +887,8 @@ int mpdata_prep(icar_adv_t *h, float dt)
     const size_t nf = (size_t)(g.nx + 1) * g.nz * (g.ny + 1);
     icar::k_mp_prep<<<blocks_for(nf, 256), 256, 0, h->stream>>>(
         g, h->desc.dx, dt, h->opts.advect_density, h->u.p, h->v.p, h->w.p, h->rho.p, h->jac.p, h->jac_u.p,
-        h->jac_v.p, h->jac_w.p, h->dz.p, h->Um.p, h->Vm.p, h->Wm.p, h->Gc.p, h->DJR.p, h->Wp.p);
+        h->jac_v.p, h->jac_w.p, h->dz.p, h->Um.p, h->Vm.p, h->Wm.p, h->Gc.p, h->DJR.p, h->Wp.p, h->op_flags,
+        ++h->op_epoch);
     if (h->opts.debug &&
         icar::check_courant(h->stream, h->g, h->Um.p, h->Vm.p, h->Wm.p, h->dz.p, h->jac.p, h->rho.p, 1))
         return fail(h, ICAR_ADV_CFL_VIOLATION, "a Courant number >= 1 was found (debug check)");
@@ -1227,6 +1243,7 @@ int icar_adv_destroy(icar_adv_t *h)
     dev_free(h->acc_precip, st);
     dev_free(h->mp_stop, st);
     dev_free(h->op_err, st);
+    dev_free(h->op_flags, st);
     for (auto *m : h->map_dev) dev_free(m, st);
     for (auto &b : h->q) release(b, st);
     for (auto &b : h->qn) release(b, st);
@@ -1927,6 +1944,8 @@ void fill_member(icar::BatchMember &m, icar_adv_t *h, double dt, int parity)
     m.Um = h->Um.p; m.Vm = h->Vm.p; m.Wm = h->Wm.p; m.Gc = h->Gc.p; m.DJR = h->DJR.p; m.Wp = h->Wp.p;
     m.filter = h->filter_dev;
     m.zone = h->zone_dev;
+    m.flags = h->op_flags;
+    m.epoch = h->op_epoch;
     for (int s = 0; s < m.S; s++) {
         // parity 0: current state in q, next in qn; parity 1 the other way round
         float *cur = parity == 0 ? h->q[s].p : h->qn[s].p;
@@ -1954,7 +1973,12 @@ int build_tables(icar_adv_batch_t *b)
     std::vector<icar::OnePassParams> opp[2];
     std::vector<CUtensorMap> maps;
     std::vector<size_t> map_base[2];
+    std::vector<int> klen(M, 0);   // levels per single-pass item of each member
     if (onepass) {
+        long tiles = 0;
+        for (icar_adv_t *h : b->members)
+            tiles += (long)onepass_tiles_x(h->g) * onepass_tiles_y(h->g) * h->desc.n_species;
+        for (int m = 0; m < M; m++) klen[m] = icar::op::levels_per_cta(tiles, b->members[m]->g.nz, b->nsm);
         opp[0].resize(std::max(M, 1));
         opp[1].resize(std::max(M, 1));
         map_base[0].resize(M);
@@ -1969,6 +1993,7 @@ int build_tables(icar_adv_batch_t *b)
         if (onepass) {
             int r = ensure_onepass(h);
             if (r) return bfail(b, r, "member scratch: %s", h->err.c_str());
+            h->op_epoch++;   // one epoch for every step these tables serve
             // descriptors of both parities: species inputs, then U_m, V_m, W_m/dz, J*rho
             for (int pp = 0; pp < 2; pp++) {
                 map_base[pp][m] = maps.size();
@@ -2000,11 +2025,12 @@ int build_tables(icar_adv_batch_t *b)
             }
         }
         if (onepass) {
-            const int tx = onepass_tiles_x(g), tyn = onepass_tiles_y(g);
+            const int tx = onepass_tiles_x(g), tyn = onepass_tiles_y(g), parts = (g.nz + klen[m] - 1) / klen[m];
             for (int s = 0; s < h->desc.n_species; s++)
                 for (int a = 0; a < tyn; a++)
                     for (int c = 0; c < tx; c++)
-                        items.push_back(make_int4(m, s, c, a * icar::op::TY));
+                        for (int k = 0; k < parts; k++)
+                            items.push_back(make_int4(m, s + icar::op::MAXS * k, c, a * icar::op::TY));
         } else {
             const int tx = icar::mp_tiles_x(g), tyn = icar::mp_tiles_y(g, ty);
             for (int s = 0; s < h->desc.n_species; s++)
@@ -2035,9 +2061,13 @@ int build_tables(icar_adv_batch_t *b)
                 q.DJR = h->DJR.p;
                 q.dz = h->dz.p;
                 q.err = b->d_operr;
+                q.flags = h->op_flags;
+                q.epoch = h->op_epoch;
+                q.nzero = -0.0f;
                 q.g = h->g;
                 q.nspecies = S;
                 q.tiles_x = onepass_tiles_x(h->g);
+                q.klen = klen[m];
             }
         if ((size_t)std::max(M, 1) > b->opp_cap || !b->d_opp[0]) {
             for (int pp = 0; pp < 2; pp++) {
@@ -2050,9 +2080,10 @@ int build_tables(icar_adv_batch_t *b)
             b->opp_cap = cap;
         }
     }
-    // longest columns first (cost ~ nz per tile), so the tail of the
+    // longest columns first (cost ~ levels per item), so the tail of the
     // launch is made of short items
     std::stable_sort(items.begin(), items.end(), [&](const int4 &x, const int4 &y) {
+        if (onepass) return klen[x.x] > klen[y.x];
         return b->members[x.x]->g.nz > b->members[y.x]->g.nz;
     });
     b->n_prep = prep[M];
@@ -2145,10 +2176,10 @@ void enqueue_step(icar_adv_batch_t *b, int p, cudaStream_t st)
             const int n = b->n_items;
             const size_t sm = icar::op::SMEM;
             const int4 *it = b->d_items;
-            if (b->path == 2 && b->fct) icar::k_batch_onepass_items<true, true><<<n, icar::op::NT, sm, st>>>(opp, it);
-            else if (b->path == 2) icar::k_batch_onepass_items<true, false><<<n, icar::op::NT, sm, st>>>(opp, it);
-            else if (b->fct) icar::k_batch_onepass_items<false, true><<<n, icar::op::NT, sm, st>>>(opp, it);
-            else icar::k_batch_onepass_items<false, false><<<n, icar::op::NT, sm, st>>>(opp, it);
+            if (b->path == 2 && b->fct) icar::k_batch_onepass_items<icar::opx::A_EXACT, true><<<n, icar::op::NT, sm, st>>>(opp, it);
+            else if (b->path == 2) icar::k_batch_onepass_items<icar::opx::A_EXACT, false><<<n, icar::op::NT, sm, st>>>(opp, it);
+            else if (b->fct) icar::k_batch_onepass_items<icar::opx::A_FAST, true><<<n, icar::op::NT, sm, st>>>(opp, it);
+            else icar::k_batch_onepass_items<icar::opx::A_FAST, false><<<n, icar::op::NT, sm, st>>>(opp, it);
         }
         return;
     }
@@ -2165,13 +2196,13 @@ cudaError_t batch_onepass_setup()
 {
     const int sm = (int)icar::op::SMEM;
     cudaError_t e =
-        cudaFuncSetAttribute(icar::k_batch_onepass_items<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+        cudaFuncSetAttribute(icar::k_batch_onepass_items<icar::opx::A_EXACT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(icar::k_batch_onepass_items<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+        e = cudaFuncSetAttribute(icar::k_batch_onepass_items<icar::opx::A_EXACT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(icar::k_batch_onepass_items<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+        e = cudaFuncSetAttribute(icar::k_batch_onepass_items<icar::opx::A_FAST, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(icar::k_batch_onepass_items<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+        e = cudaFuncSetAttribute(icar::k_batch_onepass_items<icar::opx::A_FAST, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     return e;
 }
 
@@ -2596,7 +2627,7 @@ extern "C" int icar_adv_advect_noalloc(const icar_adv_noalloc_args *a)
     const size_t nf = (size_t)(g.nx + 1) * g.nz * (g.ny + 1);
     icar::k_mp_prep<<<blocks_for(nf, 256), 256, 0, st>>>(g, a->dx, a->dt, a->advect_density, a->u, a->v, a->w,
                                                        a->density, a->jacobian, a->jacobian_u, a->jacobian_v,
-                                                       a->jacobian_w, a->advection_dz, Um, Vm, Wm, Gc, DJR, Wp);
+                                                       a->jacobian_w, a->advection_dz, Um, Vm, Wm, Gc, DJR, Wp, nullptr, 0);
     // the column-march donor-cell pass of the handle path, one species at a
     // time through the one pass-1 field of the scratch
     const dim3 gu((unsigned)((g.nx + icar::upf::BX - 1) / icar::upf::BX),

@@ -31,12 +31,34 @@ namespace icar {
 // --------------------------------------------------------------------------
 // per-step species-independent fields
 // --------------------------------------------------------------------------
+// What the prep kernels report about the fields of a step, for the exact
+// arithmetic of the single-pass kernel: flags[f] is set to the step's epoch
+// (so nothing has to be cleared between steps) when
+//   FLAG_IEEE  a wind or metric term lies outside the range its branch-free
+//              quotients are exact for (non-finite, huge, or a face Courant
+//              number that is tiny but not zero), so the tiles take IEEE
+//              division;
+//   FLAG_TIE   J*rho or dz*J*rho is an even integer other than a power of
+//              two somewhere, so that a subnormal quotient can lie exactly
+//              halfway between two floats.
+enum { FLAG_IEEE = 0, FLAG_TIE = 1, N_FLAGS = 2 };
+__device__ __forceinline__ bool exact_wind(float x)
+{
+    const float a = fabsf(x);
+    return a < 0x1p10f && (a >= 0x1p-80f || a == 0.0f);
+}
+__device__ __forceinline__ bool exact_metric(float x) { return x >= 0x1p-20f && x <= 0x1p20f; }
+__device__ __forceinline__ bool tie_divisor(float x)
+{
+    return x >= 4.0f && rintf(0.5f * x) * 2.0f == x && (__float_as_int(x) & 0x7fffff) != 0;
+}
+
 __global__ void k_mp_prep(Geo g, float dx, float dt, int adv_den, const float *__restrict__ u,
                           const float *__restrict__ v, const float *__restrict__ w, const float *__restrict__ rho,
                           const float *__restrict__ jac, const float *__restrict__ ju, const float *__restrict__ jv,
                           const float *__restrict__ jw, const float *__restrict__ dz, float *__restrict__ Um,
                           float *__restrict__ Vm, float *__restrict__ Wm, float *__restrict__ Gc,
-                          float *__restrict__ DJR, float *__restrict__ Wp)
+                          float *__restrict__ DJR, float *__restrict__ Wp, int *flags, int epoch)
 {
     size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int ni = g.nx + 1, nk = g.nz, nj = g.ny + 1;
@@ -45,12 +67,15 @@ __global__ void k_mp_prep(Geo g, float dx, float dt, int adv_den, const float *_
     const int k = (int)(rest % (size_t)nk);
     const int j = (int)(rest / (size_t)nk);
     if (j >= nj) return;
+    bool bad = false, tie = false;
     if (j < g.ny) {
         size_t c = ix(g, i, k, j);
         if (i >= 1 && i <= g.nx - 1) {
             float rr = adv_den ? rho[c] : 1.0f;
             float rl = adv_den ? rho[c - 1] : 1.0f;
-            Um[c] = u[c] * dt * (rr + rl) * 0.5f * ju[c] / dx;
+            const float um = u[c] * dt * (rr + rl) * 0.5f * ju[c] / dx;
+            Um[c] = um;
+            bad |= !exact_wind(um);
         } else {
             Um[c] = 0.0f;
         }
@@ -65,9 +90,12 @@ __global__ void k_mp_prep(Geo g, float dx, float dt, int adv_den, const float *_
             }
             Wm[c] = wm;
             const float d = dz[c], jj = jac[c], rh = rho[c];
-            Gc[c] = jj * rh;
-            DJR[c] = d * jj * rh;
-            Wp[c] = wm / d;
+            const float G = jj * rh, D = d * jj * rh, wp = wm / d;
+            Gc[c] = G;
+            DJR[c] = D;
+            Wp[c] = wp;
+            bad |= !exact_wind(wp) || !(fabsf(wm) < 0x1p20f) || !exact_metric(G) || !exact_metric(D) || !exact_metric(d);
+            tie |= tie_divisor(G) || tie_divisor(D);
         }
     }
     if (i < g.nx) {
@@ -75,11 +103,15 @@ __global__ void k_mp_prep(Geo g, float dx, float dt, int adv_den, const float *_
         if (j >= 1 && j <= g.ny - 1) {
             float rr = adv_den ? rho[c] : 1.0f;
             float rl = adv_den ? rho[ix(g, i, k, j - 1)] : 1.0f;
-            Vm[c] = v[c] * dt * (rr + rl) * 0.5f * jv[c] / dx;
+            const float vm = v[c] * dt * (rr + rl) * 0.5f * jv[c] / dx;
+            Vm[c] = vm;
+            bad |= !exact_wind(vm);
         } else {
             Vm[c] = 0.0f;
         }
     }
+    if (bad && flags) flags[FLAG_IEEE] = epoch;
+    if (tie && flags) flags[FLAG_TIE] = epoch;
 }
 
 // Species pointer tables for the multi-species launches.

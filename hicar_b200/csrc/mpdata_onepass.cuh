@@ -1,41 +1,74 @@
 // Single-pass MPDATA step (mpdata_order 2, FCT on or off): one launch per
-// advect call for every species, each CTA one 56 x 26 column tile of one
-// species marching up the column.  Per level it
+// advect call for every species, each CTA one 56 x 22 column tile of one
+// species marching up the column (or up a range of its levels).  Per level it
 //
-//   P0  recomputes the donor-cell pass q0 -> q1 one level ahead on the tile
-//       plus a two-cell halo (upwind_advection, adv_mpdata.f90:43-103), so
-//       q1 never goes through HBM;
+//   P0  recomputes the donor-cell pass q0 -> q1 two levels ahead on the tile
+//       plus its halo (upwind_advection, adv_mpdata.f90:43-103), so q1 never
+//       goes through HBM;
 //   P1  forms the antidiffusive pseudo-velocities u2, v2, w2 with their
 //       cross terms (mpdata_fluxes, adv_mpdata.f90:105-252), scaled by 0.5
 //       and 0.5*dz (:378-380);
 //   P2  forms the FCT limiter's per-cell bounds, in/out flux sums and beta
 //       factors in x, y and z (flux_limiter, adv_mpdata.f90:254-350, in the
 //       per-cell form of adv_mpdata_FCT_core.f90:47-116, first and last cells
-//       of every line included);
-//   P3  limits each face with the betas of the two cells beside it and
-//       applies the corrective donor-cell pass (adv_mpdata.f90:384): the
-//       horizontal part at this level, the vertical part one level down.
+//       of every line included), limits the vertical face below, finishes
+//       the corrective donor-cell pass (adv_mpdata.f90:384) one level down
+//       and stores it;
+//   P3  limits the horizontal faces of the level below with the betas of the
+//       two cells beside each.
 //
 // Data movement.  The level planes of q0 and of the per-step fields (U_m,
-// V_m, W_m/dz, J*rho) arrive in shared memory by TMA (64 x 32 boxes of
+// V_m, W_m/dz, J*rho) arrive in shared memory by TMA (64 x 28 boxes of
 // this GPU's own arrays, each CTA loading its own) one level ahead of use,
-// completing on mbarriers; W_m, dz*J*rho and dz of the thread's own columns
-// come by plain
-// loads one level ahead.  Each thread owns an x-pair of columns in two rows
-// and works on the pair with packed f32x2 arithmetic; x neighbours come by
-// warp shuffles, y neighbours from the shared planes.
+// completing on mbarriers; W_m, dz*J*rho and dz of the thread's own
+// columns come by plain loads one level ahead.  Each thread owns an x-pair of
+// columns in two adjacent rows and works on the pairs with packed f32x2
+// arithmetic; x neighbours come by warp shuffles, y neighbours from the shared
+// planes.
 //
-// Arithmetic.  EXACT = true evaluates the reference's FP32 expressions in
-// their order with IEEE division and no contraction (the translation unit is
-// built with -fmad=false), so results equal the CPU oracle bit for bit.
-// EXACT = false (the fast variant) rewrites the same scheme for throughput:
-// reciprocals by the hardware approximation, fused multiply-adds, donor-cell
-// fluxes as U * (U > 0 ? l : r), and each face's pair sums shared between
-// its ratio and cross terms; its results differ from the exact ones by
-// rounding only (the tolerance is stated by the tests).
+// Arithmetic (the template argument M).
+//   A_EXACT  the reference's FP32 expressions in their order, every operation
+//            rounded as the reference rounds it, so results equal the CPU
+//            oracle bit for bit.  The work is packed and has no branch: a
+//            quotient is formed from the hardware reciprocal approximation,
+//            one Newton step (which makes the reciprocal correctly rounded)
+//            and Markstein's residual correction (P. Markstein, "Computation
+//            of elementary functions on the IBM RISC System/6000 processor",
+//            IBM J. Res. Dev. 34, 1990), with the residual scaled by a power
+//            of two so that it stays exact for subnormal operands.  The
+//            conditions under which that equals IEEE division are checked
+//            (see `worst` and the prep kernels' flags); a tile that does not
+//            meet them is redone with A_IEEE before the CTA ends.
+//   A_IEEE   the same expressions with the compiler's IEEE division: any
+//            operand, including infinities and NaN.
+//   A_FAST   the same scheme rewritten for throughput: reciprocals by the
+//            hardware approximation, fused multiply-adds, reassociated pair
+//            sums.  Its results differ from the reference in the last bits;
+//            the tolerance is stated where it is tested.
+//
+// What bounds it, and why this shape.  Nothing here is near the HBM roofline
+// (8 + 28/S bytes per cell-species): the kernel is bound by issue and latency.
+// Two adjacent rows per thread (12 warps, 168 registers) load each operand
+// once for both rows and form the faces between them once: 11.1
+// warp-instructions per cell-species in A_FAST at 52 % of the issue slots,
+// where one row per warp on 24 warps took 14.2 at 61 % and two rows 16 apart,
+// reloaded for every face, on 16 warps 14.5 at 58 %.  A y face between two
+// warps is formed once too and its flux passed through a plane.  The rings
+// are deep enough for the donor pass to run two levels ahead, so a level needs
+// two block barriers.  An iteration in the middle of the march is compiled
+// without its level conditions: the few large blocks it becomes are what lets
+// the scheduler interleave the rows (A_FAST 2.85 -> 2.36 ms at 512x512x40x12).
+// The signs of a flux are split, not selected (3.26 -> 2.81 ms).  What runs beside the row warps (the halo rows, the
+// TMA issue) is kept short, for the instruction cache (2.36 -> 2.32 ms).
+// At 512x512x40x12: A_FAST 2.73 -> 2.32 ms per launch, A_EXACT 10.8 (IEEE
+// division) -> 3.58 ms; at 187x301x33x5 A_FAST 0.338 -> 0.260 ms.
+//
+// Reference: src/physics/adv_mpdata.f90:43-413, adv_mpdata_FCT_core.f90:47-116.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "tma.cuh"
@@ -44,25 +77,23 @@ namespace icar {
 
 namespace op {
 constexpr int PW = 64;               // plane width (floats): x from x0 to x0+63
-constexpr int PH = 32;               // plane rows: y from j0-3 to j0+28
-constexpr int NW = 16;               // warps per CTA
-constexpr int NT = NW * 32;
-constexpr int RPW = PH / NW;         // rows per warp (warp w owns rows w and w+NW)
+constexpr int PH = 28;               // plane rows: y from j0-3 to j0+24
+constexpr int NC = 11;               // row warps: warp w owns the output rows 2w+3 and 2w+4 of the plane
+constexpr int NT = (NC + 1) * 32;    // the last warp takes the halo rows 1, 2 and 25, 26
 constexpr int TX = PW - 8;           // 56 output columns of an inner column tile: plane x 4..59
-constexpr int TY = PH - 6;           // 26 output rows: plane y 3..28
+constexpr int TY = PH - 6;           // 22 output rows: plane y 3..24
+static_assert(TY == 2 * NC, "two output rows per warp");
+constexpr int YB = PH - 3;           // first of the halo rows above the output rows
 constexpr int PLANE = PW * PH;
 constexpr uint32_t PLANE_BYTES = PLANE * sizeof(float);
-// TMA-filled slots (ring index = level mod ring length)
-constexpr int S_Q0 = 0;              // q0, 5 levels (t-1 .. t+3)
-constexpr int S_U = 5;               // U_m, 3 levels
-constexpr int S_V = 8;               // V_m, 3 levels
-constexpr int S_WP = 11;             // W_m/dz, 3 levels
-constexpr int S_G = 14;              // J*rho, 3 levels
-// thread-written slots
-constexpr int S_Q1 = 17;             // q1, 5 levels (t-3 .. t+1)
-constexpr int S_V2 = 22;             // unlimited v2 of the current level
-constexpr int S_BYI = 23, S_BYO = 24;  // y-limiter betas of the current level
-constexpr int NPLANES = 25;
+// Planes.  The fields of a level sit side by side in a ring of four levels
+// (powers of two: a level's slot is one mask), so a level costs a thread one
+// address and every field of it a constant offset from there.
+constexpr int F_U = 0, F_V = 1, F_G = 2, F_WP = 3, F_Q1 = 4, N4 = 5;   // U_m, V_m, J*rho, W_m/dz, q1: t-1 .. t+2
+constexpr int S_Q0 = 4 * N4;                        // q0, eight levels: t-1 .. t+4
+constexpr int S_FV = S_Q0 + 8, S_FY = S_FV + 1;     // unlimited flux through the south faces of level t, limited v2 there of t-1
+constexpr int S_BYI = S_FY + 1, S_BYO = S_BYI + 1;  // y-limiter betas
+constexpr int NPLANES = S_BYO + 1;
 constexpr size_t SMEM = (size_t)NPLANES * PLANE * sizeof(float) + 128;
 constexpr uint64_t WAIT_NS = 2000000000ull;  // a TMA wait gives up after 2 s
 constexpr int MAXS = 32;             // species per launch
@@ -93,9 +124,17 @@ __device__ __forceinline__ void xtile(int nx, int tx, int ntx, int &x0, int &xlo
         }
     }
 }
+
+// Levels per CTA for a launch of `tiles` (column tile, species) pairs of nz
+// levels on `sms` SMs (one CTA each): whole columns.
+inline int levels_per_cta(long tiles, int nz, int sms)
+{
+    (void)tiles, (void)sms;
+    return nz;
+}
 }  // namespace op
 
-// Kernel parameters.  The tensor maps (64 x 1 x 32 boxes over (x, z, y))
+// Kernel parameters.  The tensor maps (64 x 1 x 28 boxes over (x, z, y))
 // live in a device table (cudaMalloc'd, so every 128-byte map is 64-byte
 // aligned as TMA requires): q0maps[s] for the species inputs, fmaps[0..3]
 // for U_m, V_m, W_m/dz and J*rho.
@@ -105,22 +144,31 @@ struct OnePassParams {
     float *out[op::MAXS];
     const float *Wm, *DJR, *dz;
     int *err;            // 1: a TMA wait gave up; 2: a TMA operand was misaligned (loads skipped)
+    const int *flags;    // what the prep kernel found in the winds and metrics (FLAG_*), by epoch
     Geo g;
     int nspecies;
     int tiles_x;
+    int klen;            // levels per CTA
+    int epoch;           // flags[i] == epoch: the condition holds for this step's fields
+    float nzero;         // -0.0f, not a compile-time constant (see opx::mul2_sep)
 };
 
 namespace opx {
 
+enum Arith { A_FAST = 0, A_EXACT = 1, A_IEEE = 2 };
 constexpr unsigned FULL = 0xffffffffu;
+constexpr float S48 = 0x1p48f, R48 = 0x1p-48f, S51 = 0x1p51f, R51 = 0x1p-51f;
+// Bound of the magnitudes A_EXACT accepts (q0, pseudo-velocities, results).
+constexpr float EXACT_MAX = 0x1p40f;
 
-__device__ __forceinline__ float2 ld2(const float *plane, int Y, int X)
+// pair of plane f at dy rows from the position `at` addresses in plane 0
+__device__ __forceinline__ float2 ld2(const float *at, int f, int dy = 0)
 {
-    return *reinterpret_cast<const float2 *>(plane + Y * op::PW + X);
+    return *reinterpret_cast<const float2 *>(at + f * op::PLANE + dy * op::PW);
 }
-__device__ __forceinline__ void st2(float *plane, int Y, int X, float2 v)
+__device__ __forceinline__ void st2(float *at, int f, float2 v, int dy = 0)
 {
-    *reinterpret_cast<float2 *>(plane + Y * op::PW + X) = v;
+    *reinterpret_cast<float2 *>(at + f * op::PLANE + dy * op::PW) = v;
 }
 __device__ __forceinline__ float up(float v) { return __shfl_up_sync(FULL, v, 1); }     // lane-1's value
 __device__ __forceinline__ float dn(float v) { return __shfl_down_sync(FULL, v, 1); }   // lane+1's value
@@ -129,11 +177,11 @@ __device__ __forceinline__ float2 lft(float2 v) { return make_float2(up(v.y), v.
 __device__ __forceinline__ float2 rgt(float2 v) { return make_float2(v.y, dn(v.x)); }
 
 // Hardware reciprocal approximation, flushing subnormal operands and results.
-// Every divisor of the fast variant is a metric term (J*rho, dz*J*rho and
-// their face sums), a sum of tracer values plus 1e-10, or a flux sum plus
-// 1e-15: none is subnormal or above 2^126, so flushing changes no result,
-// and it spares the multi-instruction subnormal handling around each
-// reciprocal that the non-flushing form needs.
+// Every divisor is a metric term (J*rho, dz*J*rho and their face sums), a
+// sum of tracer values plus 1e-10, or a flux sum plus 1e-15: none is
+// subnormal or above 2^126 (A_EXACT's checks catch one that is), and the
+// non-flushing form needs a multi-instruction subnormal handling around each
+// reciprocal.
 __device__ __forceinline__ float rcp_approx(float x)
 {
     float r;
@@ -142,213 +190,291 @@ __device__ __forceinline__ float rcp_approx(float x)
 }
 __device__ __forceinline__ float2 rcp2(float2 b) { return make_float2(rcp_approx(b.x), rcp_approx(b.y)); }
 __device__ __forceinline__ float2 div2x(float2 a, float2 b) { return make_float2(a.x / b.x, a.y / b.y); }
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+__device__ __forceinline__ float2 max2(float2 a, float2 b) { return make_float2(fmaxf(a.x, b.x), fmaxf(a.y, b.y)); }
+__device__ __forceinline__ float2 min2(float2 a, float2 b) { return make_float2(fminf(a.x, b.x), fminf(a.y, b.y)); }
 
-// donor-cell flux, exact form ((U+|U|)*l + (U-|U|)*r)/2 (adv_mpdata.f90:23-41)
-__device__ __forceinline__ float2 flux_x(float2 l, float2 r, float2 U)
+// a*b rounded by itself: ptxas may contract a packed multiply into a packed
+// add that consumes it, so a product that feeds an add directly is written
+// as a fused multiply-add with a -0.0 the compiler cannot see.
+__device__ __forceinline__ float2 mul2_sep(float2 a, float2 b, float2 nz) { return fma2(a, b, nz); }
+
+// max(m, |a|, |b|), NaN if any is NaN
+__device__ __forceinline__ void worst_of(float &m, float2 v)
 {
-    const float2 a = abs2(U);
-    return mul2x(add2x(mul2x(add2x(U, a), l), mul2x(sub2x(U, a), r)), splat2(0.5f));
+    asm("max.NaN.abs.f32 %0, %0, %1, %2;\n" : "+f"(m) : "f"(v.x), "f"(v.y));
 }
-// the same flux as U times the upwind value (equal but for rounding of
-// subnormal products)
-__device__ __forceinline__ float2 flux_f(float2 l, float2 r, float2 U)
+
+// ---- A_EXACT quotients -----------------------------------------------------
+// Everything works on the negated reciprocal and yields the negated quotient,
+// which spares the sign flips.  nrcp(b) = -RN(1/b): the approximation is good
+// to an ulp, and one Newton step from there rounds correctly for every
+// significand (checked exhaustively on the device).
+__device__ __forceinline__ float2 nrcp(float2 b)
 {
-    return mul2(U, make_float2(U.x > 0.0f ? l.x : r.x, U.y > 0.0f ? l.y : r.y));
+    const float2 r0 = make_float2(rcp_approx(-b.x), rcp_approx(-b.y));
+    return fma2(r0, fma2(b, r0, splat2(1.0f)), r0);
 }
-// pair arithmetic of the variant: exact (never contracted) or packed
-template <bool EXACT>
+// -(a*2^48)/b correctly rounded, for quotients that are normal numbers: the
+// numerator is scaled first, so the residual A + b*nq is exact even for the
+// smallest subnormal numerator.
+__device__ __forceinline__ float2 nquot48(float2 a, float2 b)
+{
+    const float2 nr = nrcp(b);
+    const float2 A = mul2(a, splat2(S48));
+    const float2 nq = mul2(A, nr);
+    return fma2(fma2(b, nq, A), nr, nq);
+}
+// A divisor that several quotients share, scaled by 2^K for the residual.
+struct ExDiv {
+    float2 bs, nrs, nr;   // b*2^K, -2^-K/b, -1/b
+};
+__device__ __forceinline__ ExDiv exdiv(float2 b, float s, float r)
+{
+    ExDiv d;
+    d.nr = nrcp(b);
+    d.bs = mul2(b, splat2(s));
+    d.nrs = mul2(d.nr, splat2(r));
+    return d;
+}
+// -(a/b) where the quotient may be subnormal: the trial quotient is unscaled
+// and the residual scaled, so the last operation rounds once at the
+// quotient's own granularity.  It is correct unless the quotient is
+// subnormal and lies exactly halfway between two floats, which needs b to be
+// an even integer other than a power of two (b = B*2^e with B odd and
+// e <= 0 keeps every quotient at least 2^-25 ulp off a midpoint, more than
+// the error of the product of residual and reciprocal).  `tie` says that
+// such a divisor occurs (FLAG_TIE); then the halfway case is rounded to
+// even by hand.
+__device__ __forceinline__ float tie_even(float nq, float nq0, float rem, float bs)
+{
+    if (fabsf(nq0) < 0x1p-125f && fabsf(rem) == bs * 0x1p-75f * 0x1p-75f)
+        return (__float_as_int(nq0) & 1) ? nq0 - copysignf(0x1p-149f, rem) : nq0;
+    return nq;
+}
+__device__ __forceinline__ float2 nquot(float2 a, const ExDiv &d, bool tie)
+{
+    const float2 nq0 = mul2(a, d.nr);
+    const float2 rem = fma2(d.bs, nq0, mul2(a, splat2(S48)));
+    float2 nq = fma2(rem, d.nrs, nq0);
+    if (__builtin_expect(tie, 0)) nq = make_float2(tie_even(nq.x, nq0.x, rem.x, d.bs.x), tie_even(nq.y, nq0.y, rem.y, d.bs.y));
+    return nq;
+}
+
+// ---- pair arithmetic of the variants -----------------------------------------
+// A_IEEE: scalar operations, never contracted.  A_EXACT and A_FAST: packed
+// (in A_EXACT, ml must not feed an add; mul2_sep does).
+template <int M>
 __device__ __forceinline__ float2 ad(float2 a, float2 b)
 {
-    if constexpr (EXACT) return add2x(a, b);
+    if constexpr (M == A_IEEE) return add2x(a, b);
     else return add2(a, b);
 }
-template <bool EXACT>
+template <int M>
 __device__ __forceinline__ float2 sb(float2 a, float2 b)
 {
-    if constexpr (EXACT) return sub2x(a, b);
+    if constexpr (M == A_IEEE) return sub2x(a, b);
     else return sub2(a, b);
 }
-template <bool EXACT>
+template <int M>
 __device__ __forceinline__ float2 ml(float2 a, float2 b)
 {
-    if constexpr (EXACT) return mul2x(a, b);
+    if constexpr (M == A_IEEE) return mul2x(a, b);
     else return mul2(a, b);
 }
 
-template <bool EXACT>
-__device__ __forceinline__ float2 flux(float2 l, float2 r, float2 U)
+// A face velocity as its two signed parts, doubled: U+|U| and U-|U| (A_IEEE: the
+// velocity itself, in p).  Using both parts instead of selecting the upwind
+// one spares a comparison and moves per face.
+struct Split {
+    float2 p, n;
+};
+template <int M>
+__device__ __forceinline__ Split split(float2 U)
 {
-    if constexpr (EXACT) return flux_x(l, r, U);
-    else return flux_f(l, r, U);
+    if constexpr (M == A_IEEE) return {U, U};
+    const float2 a = abs2(U);
+    return {add2(U, a), sub2(U, a)};
+}
+// Donor-cell flux ((U+|U|)*l + (U-|U|)*r)/2 (adv_mpdata.f90:23-41).  One of the
+// two products is zero, so fusing the other with the sum rounds as the
+// reference does.  A_FAST leaves the flux doubled (half_of takes the factor
+// into the reciprocal the flux divergence is multiplied with).
+template <int M>
+__device__ __forceinline__ float2 flux(float2 l, float2 r, Split s, float2 nz)
+{
+    if constexpr (M == A_IEEE) {
+        const float2 a = abs2(s.p);
+        return mul2x(add2x(mul2x(add2x(s.p, a), l), mul2x(sub2x(s.p, a), r)), splat2(0.5f));
+    }
+    const float2 f = fma2(s.p, l, mul2(s.n, r));
+    if constexpr (M == A_EXACT) return mul2_sep(f, splat2(0.5f), nz);
+    else return f;
+}
+__device__ __forceinline__ float2 half_of(float2 a) { return mul2(a, splat2(0.5f)); }
+// A cell's y difference, the flux through its north face (l: the cell, r: the
+// one north of it) less the one through its south face.  A_FAST fuses the
+// subtraction.
+template <int M>
+__device__ __forceinline__ float2 north_less(float2 l, float2 r, Split s, float2 south, float2 nz)
+{
+    if constexpr (M == A_FAST) return fma2(s.p, l, fma2(s.n, r, neg2(south)));
+    else return sb<M>(flux<M>(l, r, s, nz), south);
+}
+// The flux as the limiter uses it, doubled in A_EXACT and A_FAST (its sums are
+// halved in the same operation that adds 1e-15).
+template <int M>
+__device__ __forceinline__ float2 lflux(float2 l, float2 r, float2 U, float2 nz)
+{
+    const Split s = split<M>(U);
+    if constexpr (M == A_IEEE) return flux<M>(l, r, s, nz);
+    else return fma2(s.p, l, mul2(s.n, r));
 }
 
-// FCT beta num/den (den > 0): min(1, num/den) as the reference uses it; a
-// quotient >= 1 is returned as 1 without dividing, num == 0 gives 0.
-template <bool EXACT>
-__device__ __forceinline__ float beta(float num, float den)
+// FCT beta num/den (den > 0): min(1, num/den) as the reference uses it.
+// A_IEEE returns a quotient >= 1 as 1 without dividing and 0 for num == 0.
+__device__ __forceinline__ float beta_ieee(float num, float den)
 {
-    if constexpr (EXACT) {
-        if (num >= den) return 1.0f;
-        if (num == 0.0f) return 0.0f;
-        return num / den;
+    if (num >= den) return 1.0f;
+    if (num == 0.0f) return 0.0f;
+    return num / den;
+}
+// The limiter terms of a pair of cells in one direction from their bounds and
+// the fluxes through their two faces (as lflux gives them).
+template <int M>
+__device__ __forceinline__ void betas(float2 qmax, float2 qmin, float2 qc, float2 fl, float2 fr, float2 &bin,
+                                      float2 &bout)
+{
+    const float2 z = splat2(0.0f), e15 = splat2(1e-15f), one = splat2(1.0f);
+    const float2 fin = sb<M>(max2(z, fl), min2(z, fr)), fout = sb<M>(max2(z, fr), min2(z, fl));
+    const float2 a = sb<M>(qmax, qc), b = sb<M>(qc, qmin);
+    if constexpr (M == A_IEEE) {
+        const float2 di = add2x(fin, e15), dout = add2x(fout, e15);
+        bin = make_float2(beta_ieee(a.x, di.x), beta_ieee(a.y, di.y));
+        bout = make_float2(beta_ieee(b.x, dout.x), beta_ieee(b.y, dout.y));
+    } else if constexpr (M == A_EXACT) {
+        // never subnormal: a num below 2^-126*den would need values so small
+        // that den is its 1e-15
+        bin = min2(one, mul2(nquot48(a, fma2(fin, splat2(0.5f), e15)), splat2(-R48)));
+        bout = min2(one, mul2(nquot48(b, fma2(fout, splat2(0.5f), e15)), splat2(-R48)));
     } else {
-        return fminf(1.0f, num * rcp_approx(den));
+        bin = min2(one, mul2(a, rcp2(fma2(fin, splat2(0.5f), e15))));
+        bout = min2(one, mul2(b, rcp2(fma2(fout, splat2(0.5f), e15))));
     }
 }
 
-// Limited pseudo-velocity at a face (adv_mpdata_FCT_core.f90:103-115).
-// The fast variant's betas are already at most 1, and its form is a select.
-template <bool EXACT>
-__device__ __forceinline__ float limit(float u, float bin_r, float bout_l, float bin_l, float bout_r)
+// Limited face velocity (adv_mpdata_FCT_core.f90:103-115): times the factor of
+// its sign, min(bin_r, bout_l) for u > 0, min(bin_l, bout_r) otherwise (betas
+// are at most 1).  Twice the limited velocity rounds as the limited velocity
+// does (where it is subnormal, its flux is too small to change a cell).
+template <int M>
+__device__ __forceinline__ Split limit(float2 u, float2 bin_r, float2 bout_l, float2 bin_l, float2 bout_r)
 {
-    if constexpr (EXACT) {
-        if (u > 0.0f) return fminf(fminf(1.0f, bin_r), bout_l) * u;
-        if (u < 0.0f) return fminf(fminf(1.0f, bin_l), bout_r) * u;
-        return u;
-    } else {
-        return (u > 0.0f ? fminf(bin_r, bout_l) : fminf(bin_l, bout_r)) * u;
+    if constexpr (M == A_IEEE) {
+        auto one = [](float u, float br, float ol, float bl, float orr) {
+            if (u > 0.0f) return fminf(fminf(1.0f, br), ol) * u;
+            if (u < 0.0f) return fminf(fminf(1.0f, bl), orr) * u;
+            return u;
+        };
+        const float2 w = make_float2(one(u.x, bin_r.x, bout_l.x, bin_l.x, bout_r.x),
+                                     one(u.y, bin_r.y, bout_l.y, bin_l.y, bout_r.y));
+        return {w, w};
     }
+    const Split s = split<M>(u);
+    return {mul2(s.p, min2(bin_r, bout_l)), mul2(s.n, min2(bin_l, bout_r))};
+}
+// A split velocity through a plane: as one value and back.
+template <int M>
+__device__ __forceinline__ float2 join(Split s)
+{
+    if constexpr (M == A_IEEE) return s.p;
+    else return add2(s.p, s.n);   // one part is zero
+}
+template <int M>
+__device__ __forceinline__ Split unjoin(float2 w)
+{
+    if constexpr (M == A_IEEE) return {w, w};
+    const Split s = split<M>(w);
+    return {half_of(s.p), half_of(s.n)};
 }
 
-// Limited flux through a pair of faces in the fast variant: the face
-// velocity u times the limiter factor of its sign (min(bin_r, bout_l) for
-// u > 0, min(bin_l, bout_r) otherwise) times the upwind cell's value; one
-// comparison per face serves both selects.
-__device__ __forceinline__ float2 lim_flux2(float2 u, float2 ql, float2 qr, float2 bin_r, float2 bout_l, float2 bin_l,
-                                            float2 bout_r)
-{
-    const bool px = u.x > 0.0f, py = u.y > 0.0f;
-    const float2 b = make_float2(fminf(px ? bin_r.x : bin_l.x, px ? bout_l.x : bout_r.x),
-                                 fminf(py ? bin_r.y : bin_l.y, py ? bout_l.y : bout_r.y));
-    const float2 q = make_float2(px ? ql.x : qr.x, py ? ql.y : qr.y);
-    return mul2(mul2(u, b), q);
-}
-
-// Per-cell limiter terms of one direction (the carried form of the FCT
-// sweep): bounds over the cell and its two line neighbours, in/out flux sums
-// from the fluxes on its two faces, with the reference's first/last-cell
-// cases.  pos: 0 interior, 1 first cell, 2 last cell.  w lines (flux_is_w)
-// keep the end fluxes; x/y lines use 0 there.
-template <bool EXACT>
-__device__ __forceinline__ void fct_cell(float q1m, float q1c, float q1p, float q0m, float q0c, float q0p, float fl,
-                                         float fr, int pos, bool wline, float &bin, float &bout)
-{
-    float qmax, qmin, fin, fout;
-    if (pos == 1) {
-        qmax = fmaxf(fmaxf(q1c, q1p), fmaxf(q0c, q0p));
-        qmin = fminf(fminf(q1c, q1p), fminf(q0c, q0p));
-        if (wline) {
-            fin = 0.0f - fminf(0.0f, fr);
-            fout = fmaxf(0.0f, fr);
-        } else {
-            fin = 0.0f;
-            fout = 0.0f;
-        }
-    } else if (pos == 2) {
-        qmax = fmaxf(fmaxf(q1m, q1c), q0m);
-        qmin = fminf(fminf(q1m, q1c), q0m);
-        if (wline) {
-            fin = fmaxf(0.0f, fl) - fminf(0.0f, fl);
-            fout = fin;
-        } else {
-            fin = 0.0f;
-            fout = 0.0f;
-        }
-    } else {
-        qmax = fmaxf(fmaxf(fmaxf(q1m, q1c), q1p), fmaxf(fmaxf(q0m, q0c), q0p));
-        qmin = fminf(fminf(fminf(q1m, q1c), q1p), fminf(fminf(q0m, q0c), q0p));
-        fin = fmaxf(0.0f, fl) - fminf(0.0f, fr);
-        fout = fmaxf(0.0f, fr) - fminf(0.0f, fl);
-    }
-    const float e15 = 1e-15f;
-    bin = beta<EXACT>(qmax - q1c, fin + e15);
-    bout = beta<EXACT>(q1c - qmin, fout + e15);
-}
-
-// The same terms for a pair of interior cells (pos 0) in the fast
-// variant's packed arithmetic.
-__device__ __forceinline__ void fct_pair_fast(float2 q1m, float2 q1c, float2 q1p, float2 q0m, float2 q0c, float2 q0p,
-                                              float2 fl, float2 fr, float2 &bin, float2 &bout)
-{
-    const float2 qmax = make_float2(fmaxf(fmaxf(fmaxf(q1m.x, q1c.x), q1p.x), fmaxf(fmaxf(q0m.x, q0c.x), q0p.x)),
-                                    fmaxf(fmaxf(fmaxf(q1m.y, q1c.y), q1p.y), fmaxf(fmaxf(q0m.y, q0c.y), q0p.y)));
-    const float2 qmin = make_float2(fminf(fminf(fminf(q1m.x, q1c.x), q1p.x), fminf(fminf(q0m.x, q0c.x), q0p.x)),
-                                    fminf(fminf(fminf(q1m.y, q1c.y), q1p.y), fminf(fminf(q0m.y, q0c.y), q0p.y)));
-    const float2 fin = sub2(make_float2(fmaxf(0.0f, fl.x), fmaxf(0.0f, fl.y)),
-                            make_float2(fminf(0.0f, fr.x), fminf(0.0f, fr.y)));
-    const float2 fout = sub2(make_float2(fmaxf(0.0f, fr.x), fmaxf(0.0f, fr.y)),
-                             make_float2(fminf(0.0f, fl.x), fminf(0.0f, fl.y)));
-    const float2 e15 = splat2(1e-15f);
-    const float2 a = mul2(sub2(qmax, q1c), rcp2(add2(fin, e15)));
-    const float2 b = mul2(sub2(q1c, qmin), rcp2(add2(fout, e15)));
-    bin = make_float2(fminf(1.0f, a.x), fminf(1.0f, a.y));
-    bout = make_float2(fminf(1.0f, b.x), fminf(1.0f, b.y));
-}
-
-// The first and last cells of an x or y line in the fast variant, as the
-// interior form on substituted operands: a neighbour the reference's bounds
-// leave out takes a value already in them (the first cell's bounds omit the
-// cell before it; the last cell's take q1 of the cell before it and of
-// itself and q0 of the cell before it only), and both fluxes are zero (the
-// x and y lines carry no flux sums at their ends).
-__device__ __forceinline__ void fct_edge_sub(bool first, bool last, float &q1m, float q1c, float &q1p, float &q0m,
-                                             float &q0c, float &q0p, float &fl, float &fr)
-{
-    if (first) {
-        q1m = q1c;
-        q0m = q0c;
-    }
-    if (last) {
-        q1p = q1c;
-        q0c = q0m;
-        q0p = q0m;
-    }
-    if (first || last) fl = fr = 0.0f;
-}
-
-// Cross-term ratio (((a-b)+c)-d) / (den + 1e-10) with the reference's
-// operand order for the denominator chosen by the caller.
-__device__ __forceinline__ float2 xnum(float2 a, float2 b, float2 c, float2 d) { return sub2x(add2x(sub2x(a, b), c), d); }
-__device__ __forceinline__ float2 xden(float2 p, float2 q, float2 r, float2 s)
-{
-    return add2x(add2x(add2x(add2x(p, q), r), s), splat2(1e-10f));
-}
-// 0.25 * (((a + b) + c) + d)
-__device__ __forceinline__ float2 avg4(float2 a, float2 b, float2 c, float2 d)
-{
-    return mul2x(splat2(0.25f), add2x(add2x(add2x(a, b), c), d));
-}
-
-// Pseudo-velocity of a face, exact form: |U|(1-|U|/(0.5*Gs)) (r-l)/(r+l+eps)
-__device__ __forceinline__ float2 base_x(float2 U, float2 Gs, float2 r, float2 l)
+// ---- pseudo-velocity of a face -------------------------------------------------
+// |U|(1-|U|/(0.5*Gs)) (hi-lo)/(hi+lo+eps), minus a cross term
+// 0.5*U*ev*eq/Gs per tangential direction, in the reference's order.
+template <int M>
+__device__ __forceinline__ float2 base_o(float2 U, float2 Gs, const ExDiv &d, float2 hi, float2 lo)
 {
     const float2 a = abs2(U);
-    float2 v = mul2x(a, sub2x(splat2(1.0f), div2x(a, mul2x(splat2(0.5f), Gs))));
-    return div2x(mul2x(v, sub2x(r, l)), add2x(add2x(r, l), splat2(1e-10f)));
+    if constexpr (M == A_IEEE) {
+        const float2 v = mul2x(a, sub2x(splat2(1.0f), div2x(a, mul2x(splat2(0.5f), Gs))));
+        return div2x(mul2x(v, sub2x(hi, lo)), add2x(add2x(hi, lo), splat2(1e-10f)));
+    } else {
+        // |U|/(0.5*Gs) = 2|U|/Gs; where it is too small for an exact residual,
+        // one minus it is 1 either way
+        const float2 a2 = add2(a, a);
+        const float2 nq = mul2(a2, d.nr);
+        const float2 nx = fma2(fma2(Gs, nq, a2), d.nr, nq);
+        const float2 F = mul2(a, add2(splat2(1.0f), nx));
+        const float2 den = add2(add2(hi, lo), splat2(1e-10f));
+        // not subnormal for |U| >= 2^-80 or zero
+        return mul2(nquot48(mul2(F, sub2(lo, hi)), den), splat2(R48));
+    }
 }
-// minus the cross term 0.5*U*ev*eq/Gs, exact form
-__device__ __forceinline__ float2 cross_x(float2 v, float2 U, float2 ev, float2 eq, float2 Gs)
+// ev = 0.25*S, eq = (((a-b)+c)-d)/(den4+1e-10)
+template <int M>
+__device__ __forceinline__ float2 cross_term(float2 U, float2 Gs, const ExDiv &d, float2 S, float2 a, float2 b, float2 c,
+                                             float2 dd, float2 den4)
 {
-    return sub2x(v, div2x(mul2x(mul2x(mul2x(splat2(0.5f), U), ev), eq), Gs));
+    const float2 den = ad<M>(den4, splat2(1e-10f));
+    if constexpr (M == A_IEEE) {
+        const float2 eq = div2x(sub2x(add2x(sub2x(a, b), c), dd), den);
+        return neg2(div2x(mul2x(mul2x(mul2x(splat2(0.5f), U), mul2x(splat2(0.25f), S)), eq), Gs));
+    } else {
+        // eq48 = 2^48 eq (the numerator with its sign turned), then
+        // U*S*eq48 = 2^51 times the reference's 0.5*U*(0.25*S)*eq, divided by
+        // Gs with the 2^51 taken out by the scaled divisor.  Where the
+        // reference's product is subnormal it has fewer bits than this one,
+        // but the term is then below 2^-120 and cannot change the sum with a
+        // base term of a face with |U| >= 2^-80 that moves anything.
+        const float2 eq48 = nquot48(add2(sub2(sub2(b, a), c), dd), den);
+        const float2 A = mul2(mul2(U, S), eq48);
+        const float2 nq = mul2(A, d.nrs);
+        return fma2(fma2(d.bs, nq, A), d.nrs, nq);   // minus the term
+    }
+}
+template <int M>
+__device__ __forceinline__ float2 sum4(float2 a, float2 b, float2 c, float2 d)
+{
+    return ad<M>(ad<M>(ad<M>(a, b), c), d);
 }
 
 }  // namespace opx
 
-// One tile's march.  INT: the whole 64 x 32 plane lies inside the domain's
-// interior (x in [1, nx-2], y in [1, ny-2]), so no cell of the tile meets a
-// domain edge: the edge cases of the reference (boundary ring, first/last
-// cells of the limiter lines, faces that do not exist) drop out at compile
-// time.  Tiles that touch an edge take the general form.
-// bars: two mbarriers initialised once per CTA; ph[0], ph[1] count the
-// phases each has completed so far (a CTA may run several tiles), and are
-// advanced here by the phases this tile completes.  Returns false when a
+// One tile's march over output levels [ka, kb).  INT: the whole 64 x 28 plane
+// lies inside the domain's interior (x in [1, nx-2], y in [1, ny-2]), so no
+// cell of the tile meets a domain edge: the edge cases of the reference
+// (boundary ring, first/last cells of the limiter lines, faces that do not
+// exist) drop out at compile time.  Tiles that touch an edge take the general
+// form.  bars: two mbarriers with no phase completed.  Returns false when a
 // TMA wait gave up (the flag in p.err is then set and the CTA must stop).
-template <bool EXACT, bool FCT, bool INT>
-__device__ __forceinline__ bool onepass_tile(float *sm, uint64_t *bars, uint32_t *ph, const OnePassParams &p, int s,
-                                             int x0, int xlo, int xhi, int j0)
+// worst: the largest magnitude A_EXACT met (NaN if it met one).
+//
+// Iteration t does, between two block barriers each,
+//   I1  the limited horizontal faces of level t-1 (P3), P0 of level t+2, P1 of
+//       level t;
+//   I2  P2 of level t, then the update of level t-1 and its store.
+// A y face is formed once, by the row north of it, and its flux passed to the
+// row south of it through a plane.  A march from ka > 0 starts two levels
+// below it (the limited flux through the bottom of ka needs the z betas of
+// ka-1 and the w2 below that); the horizontal terms are formed for the
+// output levels only.
+template <int M, bool FCT, bool INT>
+__device__ __forceinline__ bool onepass_tile(float *sm, uint64_t *bars, const OnePassParams &p, int s, int x0, int xlo,
+                                             int xhi, int j0, int ka, int kb, bool tie, float &worst)
 {
     using namespace op;
     using namespace opx;
+    constexpr int R = 2;   // rows per thread
     const Geo g = p.g;
     const int nx = g.nx, ny = g.ny, nz = g.nz;
     const int y0 = j0 - 3;
@@ -360,598 +486,686 @@ __device__ __forceinline__ bool onepass_tile(float *sm, uint64_t *bars, uint32_t
     const int ia = x0 + X, ib = ia + 1;   // global x of the pair
     const CUtensorMap *mq = p.q0maps + s;
     const CUtensorMap *mU = p.fmaps, *mV = p.fmaps + 1, *mW = p.fmaps + 2, *mG = p.fmaps + 3;
-    float *__restrict__ outg = p.out[s];
-    auto P = [&](int slot) { return sm + (size_t)slot * PLANE; };
-    auto sq0 = [&](int l) { return P(S_Q0 + (l + 5) % 5); };       // level -1 maps to a valid slot
-    auto sU = [&](int l) { return P(S_U + l % 3); };
-    auto sV = [&](int l) { return P(S_V + l % 3); };
-    auto sW = [&](int l) { return P(S_WP + (l + 3) % 3); };   // level -1 maps to a valid slot
-    auto sG = [&](int l) { return P(S_G + l % 3); };
-    auto sQ1 = [&](int l) { return P(S_Q1 + (l + 5) % 5); };       // levels -2, -1 map to valid slots
+    const float2 zero2 = splat2(0.0f), nz2 = splat2(p.nzero);
 
-    // ---- TMA issue: the loads a level adds (elected thread only)
-    // TMA operands must be aligned (map 64 B, destination 128 B, barrier
-    // 8 B); a misaligned one is reported (flag 2) and its batch is skipped,
-    // so the CTA finishes instead of faulting
-    auto tma_ok = [&](uint64_t *bar) {
-        const bool good = (((uintptr_t)mq | (uintptr_t)p.fmaps) & 63u) == 0 && (smem_u32(sm) & 127u) == 0 &&
-                          (smem_u32(bar) & 7u) == 0;
-        if (!good) atomicExch(p.err, 2);
-        return good;
+    // levels: iterations t0..kb, limiter and faces up to tl, q1 up to l1
+    const int t0 = max(ka - 2, 0), f0 = max(t0 - 1, 0);
+    const int tl = min(kb, nz - 1), l1 = min(kb + 1, nz - 1), lq = min(kb + 2, nz - 1);
+
+    // ---- TMA issue (elected thread only): the loads of iteration t, on
+    // bars[(t - t0) & 1].  TMA operands must be aligned (map 64 B, destination
+    // 128 B, barrier 8 B); misaligned ones are reported (flag 2) and the loads
+    // skipped, so the CTA finishes instead of faulting.
+    const bool aligned = (((uintptr_t)mq | (uintptr_t)p.fmaps) & 63u) == 0 && ((smem_u32(sm) & 127u) | (smem_u32(bars) & 7u)) == 0;
+    auto load_q0 = [&](int l, uint64_t *bar) { tma_load_3d(sm + (S_Q0 + (l & 7)) * PLANE, mq, x0, l, y0, bar); };
+    auto load_uvg = [&](int l, uint64_t *bar) {
+        float *to = sm + (l & 3) * (N4 * PLANE);
+        tma_load_3d(to + F_U * PLANE, mU, x0, l, y0, bar);
+        tma_load_3d(to + F_V * PLANE, mV, x0, l, y0, bar);
+        tma_load_3d(to + F_G * PLANE, mG, x0, l, y0, bar);
     };
-    auto issue = [&](uint64_t *bar, int lq0, int lu, int lv, int lw, int lg) {
-        if (!tma_ok(bar)) {
+    auto load_w = [&](int l, uint64_t *bar) { tma_load_3d(sm + ((l & 3) * N4 + F_WP) * PLANE, mW, x0, l, y0, bar); };
+    auto issue = [&](int t) {
+        uint64_t *bar = &bars[(t - t0) & 1];
+        if (!aligned) {
             mbar_arrive_expect_tx(bar, 0);
             return;
         }
-        uint32_t n = 0;
-        n += lq0 < nz;
-        n += lu < nz;
-        n += lv < nz;
-        n += (lw >= 0 && lw < nz);
-        n += lg < nz;
-        mbar_arrive_expect_tx(bar, n * PLANE_BYTES);
-        if (lq0 < nz) tma_load_3d(sq0(lq0), mq, x0, lq0, y0, bar);
-        if (lu < nz) tma_load_3d(sU(lu), mU, x0, lu, y0, bar);
-        if (lv < nz) tma_load_3d(sV(lv), mV, x0, lv, y0, bar);
-        if (lw >= 0 && lw < nz) tma_load_3d(sW(lw), mW, x0, lw, y0, bar);
-        if (lg < nz) tma_load_3d(sG(lg), mG, x0, lg, y0, bar);
+        const bool q = t + 3 <= lq, u = t + 2 <= l1, w = t + 1 <= tl;
+        mbar_arrive_expect_tx(bar, ((q ? 1u : 0u) + (u ? 3u : 0u) + (w ? 1u : 0u)) * PLANE_BYTES);
+        if (q) load_q0(t + 3, bar);
+        if (u) load_uvg(t + 2, bar);
+        if (w) load_w(t + 1, bar);
     };
-    bool ok = true;
-    // The batch waited for at iteration t was issued on bars[t & 1]: the
-    // prologue's on bars[0], iteration t-1's otherwise.  Its phase number is
-    // the barrier's count at tile start plus the batches issued on it since.
-    const uint32_t b0 = ph[0], b1 = ph[1];
-    auto phase_of = [&](int t) -> uint32_t { return (t & 1) ? b1 + (uint32_t)(t - 1) / 2 : b0 + (uint32_t)t / 2; };
-    // bounded wait on the batch of iteration t, by every thread; a thread
+    // the first iteration's: everything it and the donor pass before it read
+    auto issue_first = [&]() {
+        if (!aligned) {
+            atomicExch(p.err, 2);
+            mbar_arrive_expect_tx(bars, 0);
+            return;
+        }
+        const int qb = min(t0 + 3, lq), ub = min(t0 + 2, l1), wb = min(t0 + 1, tl);
+        mbar_arrive_expect_tx(bars, (uint32_t)(qb - f0 + 1 + 3 * (ub - t0 + 1) + (wb - t0 + 1)) * PLANE_BYTES);
+        for (int l = f0; l <= qb; l++) load_q0(l, bars);
+        for (int l = t0; l <= ub; l++) load_uvg(l, bars);
+        for (int l = t0; l <= wb; l++) load_w(l, bars);
+    };
+    // bounded wait on the batch of iteration n, by every thread; a thread
     // whose wait gave up raises the flag and reports false (the CTA then
-    // agrees at its next barrier to stop, after draining with a bound what
-    // it issued)
-    auto wait_mine = [&](int t) {
-        const bool mine = mbar_wait_bounded(&bars[t & 1], phase_of(t) & 1u, WAIT_NS);
+    // agrees at its next barrier to stop)
+    auto wait_mine = [&](int n) {
+        const bool mine = mbar_wait_bounded(&bars[n & 1], (uint32_t)(n >> 1) & 1u, WAIT_NS);
         if (!mine) atomicExch(p.err, 1);
         return mine;
     };
-    // every batch completes a phase (one arrival, possibly zero bytes): the
-    // prologue and the odd iterations on bars[0], the even ones on bars[1]
-    ph[0] = b0 + 1 + (uint32_t)(nz + 1) / 2;
-    ph[1] = b1 + (uint32_t)nz / 2 + 1;
-
-    if (threadIdx.x == 0) tma_prefetch_map(mq);
+    // a wait gave up: wait (bounded) for the batch so no copy is left in
+    // flight into this CTA's shared memory, then stop
+    auto drain = [&](int n) {
+        mbar_wait_bounded(&bars[n & 1], (uint32_t)(n >> 1) & 1u, WAIT_NS);
+        return false;
+    };
     if (threadIdx.x == 0) {
-        // iteration 0 (and the level-0 donor pass before it) needs q0 at
-        // levels 0..2, U_m, V_m and J*rho at 0..1 and W_m/dz at 0 (nz >= 3)
-        uint32_t cnt = 0;
-        for (int l = 0; l < 3; l++) cnt += l < nz;
-        for (int l = 0; l < 2; l++) cnt += 3 * (l < nz);
-        cnt += 1;
-        const bool good = tma_ok(&bars[0]);
-        mbar_arrive_expect_tx(&bars[0], good ? cnt * PLANE_BYTES : 0u);
-        for (int l = 0; good && l < 3; l++)
-            if (l < nz) tma_load_3d(sq0(l), mq, x0, l, y0, &bars[0]);
-        for (int l = 0; good && l < 2; l++) {
-            if (l >= nz) continue;
-            tma_load_3d(sU(l), mU, x0, l, y0, &bars[0]);
-            tma_load_3d(sV(l), mV, x0, l, y0, &bars[0]);
-            tma_load_3d(sG(l), mG, x0, l, y0, &bars[0]);
-        }
-        if (good) tma_load_3d(sW(0), mW, x0, 0, y0, &bars[0]);
+        tma_prefetch_map(mq);
+        issue_first();
     }
 
-    // ---- per-row constants and carried state --------------------------
-    int rowY[RPW], rowj[RPW];
-    size_t rowc[RPW];      // global offset of (ia, level 0, j) (clamped into the array)
-    bool rowin[RPW];       // row inside the domain
-#pragma unroll
-    for (int r = 0; r < RPW; r++) {
-        rowY[r] = warp + NW * r;
-        rowj[r] = y0 + rowY[r];
-        rowin[r] = rowj[r] >= 0 && rowj[r] < ny;
-        const int ci = max(min(ia, g.P - 2), 0), cj = max(min(rowj[r], ny - 1), 0);
-        rowc[r] = ix(g, ci, 0, cj);
-    }
+    // ---- rows
+    const bool halo = warp == NC;               // warp-uniform
+    const int Y = halo ? 1 : 2 * warp + 3;      // first plane row
+    const int j = y0 + Y;
+    float *const own = sm + Y * PW + X, *const top = sm + YB * PW + X;   // top: the halo warp's upper rows
+    auto at4 = [&](float *at, int l) { return at + (l & 3) * (N4 * PLANE); };
+    auto atq = [&](float *at, int l) { return at + (S_Q0 + (l & 7)) * PLANE; };
+    auto row_offset = [&](int jj) {   // of (ia, level 0, jj), clamped into the array (fewer than 2^32 elements)
+        return (uint32_t)ix(g, max(min(ia, g.P - 2), 0), 0, max(min(jj, ny - 1), 0));
+    };
+    const uint32_t rowc[R] = {row_offset(j), row_offset(j + 1)};
+    const uint32_t lstride = (uint32_t)g.P;
     const bool inA = ia >= 0 && ia < nx, inB = ib >= 0 && ib < nx;
-    const size_t lstride = (size_t)g.P;
+    auto jin = [&](int jr) { return INT || (jr >= 0 && jr < ny); };
+    auto jint = [&](int jr) { return INT || (jr > 0 && jr < ny - 1); };
+    // the pair's columns that this tile stores (rows start on 16-byte
+    // boundaries and ia is even: the pair is 8-byte aligned)
+    const bool sta = (INT || inA) && X >= xlo && X < xhi, stb = (INT || inB) && X + 1 >= xlo && X + 1 < xhi;
+    float *const outs = p.out[s];
+    auto ldcol = [&](const float *src, uint32_t row, int lev) -> float2 {
+        return *reinterpret_cast<const float2 *>(src + (row + (uint32_t)lev * lstride));
+    };
 
-    // own-column values by plain loads, one level ahead
-    // (the fast variant carries dz*J*rho as its reciprocal: each value
-    // divides twice, in the donor pass and in the corrective pass)
-    float2 r_wm[RPW], n_wm[RPW], r_djr0[RPW], r_djrm[RPW], n_djr[RPW], n_dz[RPW];
-    auto djr_in = [](float2 v) -> float2 {
-        if constexpr (EXACT) return v;
-        else return rcp2(v);
-    };
-    // carried z state of the output cells, the donor pass's flux through
-    // the top of the level it formed last, and (fast variant) the
-    // reciprocal of J*rho that the donor pass formed for the level the
-    // corrective pass updates next (r_rg: level t, n_rg: level t+1)
-    float2 r_w2[RPW], r_bzi[RPW], r_bzo[RPW], r_fb[RPW], r_part[RPW], r_vt[RPW], r_rg[RPW], n_rg[RPW];
-    auto ldcol = [&](const float *src, int r, int lev) -> float2 {
-        return *reinterpret_cast<const float2 *>(src + rowc[r] + (size_t)lev * lstride);
-    };
+    // ---- P0: donor-cell pass at level L on two rows (at: the first one's
+    // position, jr its global row) into the q1 plane of L.  wtop = W_m(L), djr =
+    // dz*J*rho at L; v: on entry the flux through the bottom of L (the one
+    // through the top of L-1), on return the flux through its top.
+    auto donor = [&](int L, float *at, int jr, const float2 (&wtop)[R], const float2 (&djr)[R], float2 (&v)[R], float2 (&q1)[R]) {
+        const float *Q = atq(at, L), *Qn = atq(at, L + 1), *F = at4(at, L);
+        const float2 c[R + 2] = {ld2(Q, 0, -1), ld2(Q, 0), ld2(Q, 0, 1), ld2(Q, 0, 2)};
+        float2 south = flux<M>(c[0], c[1], split<M>(ld2(F, F_V)), nz2);
 #pragma unroll
-    for (int r = 0; r < RPW; r++) {
-        r_wm[r] = ldcol(p.Wm, r, 0);
-        r_djr0[r] = djr_in(ldcol(p.DJR, r, 0));
-        n_wm[r] = nz > 1 ? ldcol(p.Wm, r, 1) : splat2(0.0f);
-        n_djr[r] = nz > 1 ? ldcol(p.DJR, r, 1) : splat2(1.0f);
-        n_dz[r] = ldcol(p.dz, r, 0);
-        r_djrm[r] = splat2(1.0f);
-        r_w2[r] = r_bzi[r] = r_bzo[r] = r_fb[r] = r_part[r] = r_vt[r] = splat2(0.0f);
-    }
-
-    const float2 zero2 = splat2(0.0f);
-
-    // ---- P0: donor-cell pass at level L into the q1 plane of L ----------
-    // wtop = W_m(L), djr = dz*J*rho at L (its reciprocal in the fast
-    // variant), own pair.  Levels are formed in order, so the flux through
-    // the bottom of L is the one through the top of L-1, carried in r_vt.
-    auto donor = [&](int L, int r, float2 wtop, float2 djr) {
-        const int Y = rowY[r], j = rowj[r];
-        const bool need = Y >= 1 && Y <= PH - 2;     // warp-uniform
-        if (!need) return;
-        const float *Q = sq0(L);
-        const float2 c = ld2(Q, Y, X);
-        const float2 n = ld2(Q, Y + 1, X), sth = ld2(Q, Y - 1, X);
-        const float2 w = lft(c);
-        const float2 uw = ld2(sU(L), Y, X);
-        const float2 vs = ld2(sV(L), Y, X), vn = ld2(sV(L), Y + 1, X);
-        const float2 G = ld2(sG(L), Y, X);
-        // a cell's east face is the next cell's west face: same operands,
-        // same value, so it is formed once and passed along by a shuffle
-        const float2 fw = flux<EXACT>(w, c, uw), fe = rgt(fw);
-        const float2 f3 = flux<EXACT>(c, n, vn), f4 = flux<EXACT>(sth, c, vs);
-        const float2 hd = ad<EXACT>(sb<EXACT>(fe, fw), sb<EXACT>(f3, f4));
+        for (int r = 0; r < R; r++) {
+            const float2 cc = c[r + 1];
+            if constexpr (M == A_EXACT) worst_of(worst, cc);
+            // a cell's east face is the next cell's west face: same operands,
+            // same value, so it is formed once and passed along by a shuffle
+            const float2 fw = flux<M>(lft(cc), cc, split<M>(ld2(F, F_U, r)), nz2), fe = rgt(fw);
+            const Split vn = split<M>(ld2(F, F_V, r + 1));
+            const float2 hd = ad<M>(sb<M>(fe, fw), north_less<M>(cc, c[r + 2], vn, south, nz2));
+            if (r + 1 < R) south = flux<M>(cc, c[r + 2], vn, nz2);
+            const float2 G = ld2(F, F_G, r);
+            float2 vd;
+            if (L < nz - 1) {
+                const float2 vt = flux<M>(cc, ld2(Qn, 0, r), split<M>(wtop[r]), nz2);
+                vd = sb<M>(vt, v[r]);
+                v[r] = vt;
+            } else if constexpr (M == A_FAST) {   // the model top: q times the face's W_m
+                vd = fma2(cc, add2(wtop[r], wtop[r]), neg2(v[r]));
+            } else if constexpr (M == A_EXACT) {
+                vd = sub2(mul2_sep(cc, wtop[r], nz2), v[r]);
+            } else {
+                vd = sub2x(mul2x(cc, wtop[r]), v[r]);
+            }
+            float2 val;
+            if constexpr (M == A_IEEE) {
+                val = sub2x(sub2x(cc, div2x(hd, G)), div2x(vd, djr[r]));
+            } else if constexpr (M == A_EXACT) {
+                val = add2(cc, nquot(hd, exdiv(G, S48, R48), tie));
+                val = add2(val, nquot(vd, exdiv(djr[r], S48, R48), tie));
+            } else {
+                val = sub2(sub2(cc, mul2(hd, half_of(rcp2(G)))), mul2(vd, half_of(rcp2(djr[r]))));
+            }
+            if (!INT) {
+                const int jj = jr + r;
+                const bool rin = jj >= 0 && jj < ny, jring = jj == 0 || jj == ny - 1;
+                val.x = !(inA && rin) ? 0.0f : ((jring || ia == 0 || ia == nx - 1) ? cc.x : val.x);
+                val.y = !(inB && rin) ? 0.0f : ((jring || ib == 0 || ib == nx - 1) ? cc.y : val.y);
+            }
+            q1[r] = val;
+        }
+    };
+    // the flux through the top of level L on a row, for a march (or a row)
+    // that does not carry it
+    auto top_flux = [&](int L, float *at, uint32_t row) -> float2 {
+        return flux<M>(ld2(atq(at, L), 0), ld2(atq(at, L + 1), 0), split<M>(ldcol(p.Wm, row, L)), nz2);
+    };
+    // ---- P1: pseudo-velocities at level t ------------------------------------
+    // y face: v2 on the south faces of a row.  qc, qs: q1(t) of the row and of
+    // the one south of it; qu, qsu, qd, qsd: the same at t+1 and t-1; the wind
+    // and metric operands likewise.  The unlimited flux goes to its plane.
+    auto face_y = [&](auto st, int t, int jr, float2 qc, float2 qs, float2 qu, float2 qsu, float2 qd, float2 qsd, float2 Vt,
+                      float2 Gc, float2 Gst, float2 Ut, float2 Us, float2 Wt, float2 Wd, float2 Wts, float2 Wds,
+                      float2 &fv) -> float2 {
+        const bool kint = decltype(st)::value || (t > 0 && t < nz - 1);
+        const float2 Gs = ad<M>(Gc, Gst);
+        const bool xa = INT || (ia > 0 && ia < nx - 1), xb = INT || (ib > 0 && ib < nx - 1);
         float2 val;
-        const bool mid = L > 0 && L < nz - 1;
-        float2 vt = zero2;
-        const float2 vb = L > 0 ? r_vt[r] : zero2;
-        if (L < nz - 1) vt = flux<EXACT>(c, ld2(sq0(L + 1), Y, X), wtop);
-        r_vt[r] = vt;
-        if constexpr (EXACT) {
-            val = sub2x(c, div2x(hd, G));
-            if (mid) val = sub2x(val, div2x(sub2x(vt, vb), djr));
-            else if (L == 0) val = sub2x(val, div2x(vt, djr));
-            else val = sub2x(val, div2x(sub2x(mul2x(c, wtop), vb), djr));
+        if constexpr (M != A_FAST) {
+            ExDiv d{};
+            if constexpr (M == A_EXACT) d = exdiv(Gs, S51, R51);
+            val = base_o<M>(Vt, Gs, d, qc, qs);
+            {
+                const float2 qcl = lft(qc), qcr = rgt(qc), qsl = lft(qs), qsr = rgt(qs);
+                const float2 Utr = rgt(Ut), Usr = rgt(Us);
+                const float2 cp = make_float2(qc.y, qcr.y), sp = make_float2(qs.y, qsr.y);   // x+1
+                float2 ct = cross_term<M>(Vt, Gs, d, sum4<M>(make_float2(Ut.y, Utr.y), make_float2(Us.y, Usr.y), Ut, Us),
+                                          sp, qcl, cp, qsl, sum4<M>(cp, sp, qcl, qsl));
+                // no cross term on the domain's first and last columns
+                if (!xa) ct.x = 0.0f;
+                if (!xb) ct.y = 0.0f;
+                val = ad<M>(val, ct);
+            }
+            if (kint)
+                val = ad<M>(val, cross_term<M>(Vt, Gs, d, sum4<M>(Wt, Wd, Wts, Wds), qsu, qd, qu, qsd,
+                                               sum4<M>(qsu, qd, qu, qsd)));
+            if constexpr (M == A_EXACT) val = mul2_sep(val, splat2(0.5f), nz2);
+            else val = mul2x(val, splat2(0.5f));
         } else {
-            const float2 vdiv = mid ? sub2(vt, vb) : (L == 0 ? vt : sub2(mul2(c, wtop), vb));
-            const float2 rg = rcp2(G);
-            n_rg[r] = rg;
-            val = sub2(sub2(c, mul2(hd, rg)), mul2(vdiv, djr));
+            // the final 0.5 folded in: 0.5 |V| (1 - 2 |V| / Gs) = 0.5 |V| - V^2 / Gs, and each
+            // cross term 0.25 V / Gs times the 4-face average (1/4 of the face sum) times eq
+            const float2 rG = rcp2(Gs);
+            const float2 F0 = sub2(mul2(splat2(0.5f), abs2(Vt)), mul2(mul2(Vt, Vt), rG));
+            const float2 sq = add2(qc, qs);
+            val = mul2(mul2(F0, sub2(qc, qs)), rcp2(add2(sq, splat2(1e-10f))));
+            const float2 mc = mul2(splat2(-0.0625f), mul2(Vt, rG));
+            // x cross term: the two rows' pair sums at x+1 and x-1, and U_m on the
+            // cells' west and east faces in both rows, each formed from one shuffle
+            const float2 yp = rgt(sq), ym = lft(sq);
+            float2 eq = mul2(sub2(yp, ym), rcp2(add2(add2(yp, ym), splat2(1e-10f))));
+            const float2 su = add2(Ut, Us);
+            float2 ev = add2(su, rgt(su));
+            // no cross term on the domain's first and last columns (their
+            // shuffled neighbours may lie outside the plane)
+            if (!xa) ev.x = eq.x = 0.0f;
+            if (!xb) ev.y = eq.y = 0.0f;
+            val = fma2(mul2(mc, ev), eq, val);
+            if (kint) {
+                const float2 zp = add2(qu, qsu), zm = add2(qd, qsd);
+                const float2 eq2 = mul2(sub2(zp, zm), rcp2(add2(add2(zp, zm), splat2(1e-10f))));
+                val = fma2(mul2(mc, add2(add2(Wt, Wd), add2(Wts, Wds))), eq2, val);
+            }
         }
-        float2 q1 = val;
         if (!INT) {
-            const bool jin = j >= 0 && j < ny, jring = j == 0 || j == ny - 1;
-            q1.x = !(inA && jin) ? 0.0f : ((jring || ia == 0 || ia == nx - 1) ? c.x : val.x);
-            q1.y = !(inB && jin) ? 0.0f : ((jring || ib == 0 || ib == nx - 1) ? c.y : val.y);
+            const bool fin = jr >= 1 && jr <= ny - 1;
+            val.x = (fin && inA) ? val.x : 0.0f;
+            val.y = (fin && inB) ? val.y : 0.0f;
         }
-        st2(sQ1(L), Y, X, q1);
+        if constexpr (M == A_EXACT) worst_of(worst, val);
+        if constexpr (FCT) fv = lflux<M>(qs, qc, val, nz2);
+        return val;
+    };
+    // the same for a row of the halo warp
+    auto face_y_row = [&](auto st, int t, int yr, float2 &f) -> float2 {
+        float *at = sm + yr * PW + X;
+        const float *C = at4(at, t), *Up = at4(at, t + 1), *Dn = at4(at, t - 1);
+        return face_y(st, t, y0 + yr, ld2(C, F_Q1), ld2(C, F_Q1, -1), ld2(Up, F_Q1), ld2(Up, F_Q1, -1), ld2(Dn, F_Q1),
+                      ld2(Dn, F_Q1, -1), ld2(C, F_V), ld2(C, F_G), ld2(C, F_G, -1), ld2(C, F_U), ld2(C, F_U, -1),
+                      ld2(C, F_WP), ld2(Dn, F_WP), ld2(C, F_WP, -1), ld2(Dn, F_WP, -1), f);
+    };
+    // x faces ia, ib (west faces of the pair)
+    auto face_x = [&](auto st, int t, int jr, float2 qc, float2 qn, float2 qs, float2 qu, float2 qd, float2 Ut, float2 Gt,
+                      float2 Vt, float2 Vtn, float2 Wt, float2 Wd) -> float2 {
+        const bool kint = decltype(st)::value || (t > 0 && t < nz - 1);
+        const float2 qcl = lft(qc), Gs = ad<M>(Gt, lft(Gt));
+        float2 val;
+        if constexpr (M != A_FAST) {
+            ExDiv d{};
+            if constexpr (M == A_EXACT) d = exdiv(Gs, S51, R51);
+            val = base_o<M>(Ut, Gs, d, qc, qcl);
+            if (jint(jr)) {
+                const float2 qnl = lft(qn), qsl = lft(qs);
+                val = ad<M>(val, cross_term<M>(Ut, Gs, d, sum4<M>(Vt, Vtn, lft(Vt), lft(Vtn)), qn, qs, qnl, qsl,
+                                               sum4<M>(qn, qs, qnl, qsl)));
+            }
+            if (kint) {
+                const float2 qul = lft(qu), qdl = lft(qd);
+                val = ad<M>(val, cross_term<M>(Ut, Gs, d, sum4<M>(Wt, Wd, lft(Wt), lft(Wd)), qu, qd, qul, qdl,
+                                               sum4<M>(qu, qd, qul, qdl)));
+            }
+            if constexpr (M == A_EXACT) val = mul2_sep(val, splat2(0.5f), nz2);
+            else val = mul2x(val, splat2(0.5f));
+        } else {
+            const float2 rG = rcp2(Gs);
+            const float2 F0 = sub2(mul2(splat2(0.5f), abs2(Ut)), mul2(mul2(Ut, Ut), rG));
+            val = mul2(mul2(F0, sub2(qc, qcl)), rcp2(add2(add2(qc, qcl), splat2(1e-10f))));
+            const float2 mc = mul2(splat2(-0.0625f), mul2(Ut, rG));
+            if (jint(jr)) {
+                const float2 sv = add2(Vt, Vtn);
+                const float2 xp = add2(qn, lft(qn)), xm = add2(qs, lft(qs));
+                const float2 eq = mul2(sub2(xp, xm), rcp2(add2(add2(xp, xm), splat2(1e-10f))));
+                val = fma2(mul2(mc, add2(sv, lft(sv))), eq, val);
+            }
+            if (kint) {
+                const float2 sw = add2(Wt, Wd);
+                const float2 xp = add2(qu, lft(qu)), xm = add2(qd, lft(qd));
+                const float2 eq = mul2(sub2(xp, xm), rcp2(add2(add2(xp, xm), splat2(1e-10f))));
+                val = fma2(mul2(mc, add2(sw, lft(sw))), eq, val);
+            }
+        }
+        if (!INT) {
+            val.x = (jin(jr) && ia >= 1 && ia <= nx - 1) ? val.x : 0.0f;
+            val.y = (jin(jr) && ib >= 1 && ib <= nx - 1) ? val.y : 0.0f;
+        }
+        if constexpr (M == A_EXACT) worst_of(worst, val);
+        return val;
+    };
+    // z face at the top of a level below the last (columns inside the domain interior)
+    auto face_z = [&](int jr, float2 dz, float2 qc, float2 qu, float2 qn, float2 qs, float2 qnu, float2 qsu, float2 Wt,
+                      float2 Gt, float2 Gu, float2 Ut, float2 Uu, float2 Vt, float2 Vtn, float2 Vu, float2 Vun) -> float2 {
+        const float2 Gs = ad<M>(Gu, Gt);
+        float2 val;
+        if constexpr (M != A_FAST) {
+            ExDiv d{};
+            if constexpr (M == A_EXACT) d = exdiv(Gs, S51, R51);
+            val = base_o<M>(Wt, Gs, d, qu, qc);
+            {
+                const float2 qcl = lft(qc), qcr = rgt(qc), qul = lft(qu), qur = rgt(qu);
+                const float2 Utr = rgt(Ut), Uur = rgt(Uu);
+                const float2 cp = make_float2(qc.y, qcr.y), pp = make_float2(qu.y, qur.y);   // x+1
+                val = ad<M>(val, cross_term<M>(Wt, Gs, d,
+                                               sum4<M>(make_float2(Ut.y, Utr.y), make_float2(Uu.y, Uur.y), Ut, Uu), pp,
+                                               qcl, cp, qul, sum4<M>(cp, pp, qcl, qul)));
+            }
+            val = ad<M>(val, cross_term<M>(Wt, Gs, d, sum4<M>(Vt, Vu, Vtn, Vun), qnu, qs, qn, qsu,
+                                           sum4<M>(qn, qsu, qnu, qs)));
+            if constexpr (M == A_EXACT) val = mul2_sep(mul2(val, splat2(0.5f)), dz, nz2);
+            else val = mul2x(mul2x(val, splat2(0.5f)), dz);
+        } else {
+            const float2 rG = rcp2(Gs);
+            const float2 F0 = sub2(mul2(splat2(0.5f), abs2(Wt)), mul2(mul2(Wt, Wt), rG));
+            const float2 sq = add2(qc, qu);
+            val = mul2(mul2(F0, sub2(qu, qc)), rcp2(add2(sq, splat2(1e-10f))));
+            const float2 mc = mul2(splat2(-0.0625f), mul2(Wt, rG));
+            const float2 zp = rgt(sq), zm = lft(sq);
+            const float2 eq = mul2(sub2(zp, zm), rcp2(add2(add2(zp, zm), splat2(1e-10f))));
+            const float2 su = add2(Ut, Uu);
+            val = fma2(mul2(mc, add2(su, rgt(su))), eq, val);
+            const float2 np = add2(qn, qnu), sp = add2(qs, qsu);
+            const float2 eq2 = mul2(sub2(np, sp), rcp2(add2(add2(np, sp), splat2(1e-10f))));
+            const float2 sv = add2(add2(Vt, Vu), add2(Vtn, Vun));
+            val = fma2(mul2(mc, sv), eq2, val);
+            val = mul2(val, dz);
+        }
+        if (!INT) {
+            const bool jj = jr >= 1 && jr <= ny - 2;
+            val.x = (jj && ia >= 1 && ia <= nx - 2) ? val.x : 0.0f;
+            val.y = (jj && ib >= 1 && ib <= nx - 2) ? val.y : 0.0f;
+        }
+        if constexpr (M == A_EXACT) worst_of(worst, val);
+        return val;
+    };
+    // y-line betas of a row at level t (its unlimited south flux from the own
+    // value, its north one from the plane), stored for its neighbours too
+    auto betas_y = [&](int jr, float *at, float2 qc, float2 q0c, float2 qs, float2 q0s, float2 qn, float2 q0n, float2 fl,
+                       float2 &bi, float2 &bo) {
+        float2 fr = ld2(at, S_FV, 1);
+        float2 hs = max2(qs, q0s), ls = min2(qs, q0s), hn = max2(qn, q0n), ln = min2(qn, q0n);
+        float2 hc = max2(qc, q0c), lc = min2(qc, q0c);
+        if (!INT) {   // line ends (row-uniform), as in the x lines below
+            if (jr == 0) { hs = hc; ls = lc; }
+            if (jr == ny - 1) { hc = lc = hn = ln = qc; }
+            if (jr == 0 || jr == ny - 1) fl = fr = zero2;
+        }
+        betas<M>(max2(max2(hs, hc), hn), min2(min2(ls, lc), ln), qc, fl, fr, bi, bo);
     };
 
-    // ---- prologue: batch 0 landed -> q1 at level 0 ----------------------
-    ok = __syncthreads_and(wait_mine(0) ? 1 : 0) != 0;
-    if (!ok) goto drain;
+    // ---- prologue: batch 0 landed -> q1 at levels t0 and t0+1 --------------
+    // carried between iterations, per row: the donor pass's flux through the
+    // top of the level it formed last (vt); level t's pseudo-velocities,
+    // betas and vertical flux, and those of the level below that the z line
+    // needs; the limited flux through the bottom of level t-1; the own-column
+    // values loaded ahead
+    float2 vt[R], n_wm[R], n_djr[R], n_dz[R], djr_m[R];
+    float2 u2[R], v2[R], w2[R], w2b[R], fz[R], fzb[R], bxi[R], bxo[R], byi[R], byo[R], bzi[R], bzo[R], hx[R], fb[R], gm[R], fs = zero2;
 #pragma unroll
-    for (int r = 0; r < RPW; r++) donor(0, r, r_wm[r], r_djr0[r]);
-
-    // Three block barriers per level: after P0, after P1 (v2 plane), after
-    // P2 (y betas).  P0 of iteration t may overlap P3 of iteration t-1: it
-    // writes the q1 slot of level t+1, which the 5-level ring keeps apart
-    // from the levels t-3 .. t-1 that P3 reads, and reads only TMA planes.
-    for (int t = 0; t <= nz; t++) {
-        const bool landed = t == 0 || wait_mine(t);
-
-        const bool haveA = t < nz;
-        // own-column values for this iteration; prefetch the next level's
-        float2 c_wmn[RPW], c_djrn[RPW], c_dz[RPW];
+    for (int r = 0; r < R; r++) {
+        vt[r] = n_wm[r] = n_dz[r] = u2[r] = v2[r] = w2[r] = w2b[r] = fz[r] = fzb[r] = zero2;
+        bxi[r] = bxo[r] = byi[r] = byo[r] = bzi[r] = bzo[r] = hx[r] = fb[r] = zero2;
+        n_djr[r] = djr_m[r] = gm[r] = splat2(1.0f);
+    }
+    // The halo warp carries the donor pass's state for its two row pairs: the
+    // lower pair's in vt, n_wm and n_djr, the upper pair's in these (which its
+    // rows do not need otherwise).
+    float2(&vt_b)[R] = u2, (&wm_b)[R] = bxi, (&djr_b)[R] = bxo;
+    const uint32_t rowb[R] = {row_offset(y0 + YB), row_offset(y0 + YB + 1)};
+    if (__syncthreads_and(wait_mine(0) ? 1 : 0) == 0) return drain(0);
+    auto load_ahead = [&](int L) {
 #pragma unroll
-        for (int r = 0; r < RPW; r++) {
-            c_wmn[r] = n_wm[r];
-            c_djrn[r] = djr_in(n_djr[r]);
-            r_rg[r] = n_rg[r];
-            c_dz[r] = n_dz[r];
-            if (t + 2 < nz) {
-                n_wm[r] = ldcol(p.Wm, r, t + 2);
-                n_djr[r] = ldcol(p.DJR, r, t + 2);
+        for (int r = 0; r < R; r++) {
+            n_wm[r] = ldcol(p.Wm, rowc[r], L);
+            n_djr[r] = ldcol(p.DJR, rowc[r], L);
+        }
+    };
+    auto load_ahead_b = [&](int L) {
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            wm_b[r] = ldcol(p.Wm, rowb[r], L);
+            djr_b[r] = ldcol(p.DJR, rowb[r], L);
+        }
+    };
+    // (loops, with the two pairs' state swapped: the halo warp's code has to
+    // fit the instruction cache beside the row warps')
+    auto donor_halo = [&](int L) {
+#pragma unroll 1
+        for (int q = 0; q < 2; q++) {
+            float *at = q == 0 ? own : top;
+            float2 q1[R];
+            donor(L, at, q == 0 ? j : y0 + YB, n_wm, n_djr, vt, q1);
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                st2(at4(at, L), F_Q1, q1[r], r);
+                const float2 a = vt[r], b = n_wm[r], c = n_djr[r];
+                vt[r] = vt_b[r], n_wm[r] = wm_b[r], n_djr[r] = djr_b[r];
+                vt_b[r] = a, wm_b[r] = b, djr_b[r] = c;
             }
-            if (t + 1 < nz) n_dz[r] = ldcol(p.dz, r, t + 1);
+            if constexpr (M == A_EXACT) worst_of(worst, ld2(atq(at, L), 0, q == 0 ? -1 : 2));   // the plane's end rows
         }
-
-        // ---- P0: q1 at level t+1 ------------------------------------------
-        if (t + 1 < nz) {
+    };
+    for (int L = t0; L <= min(t0 + 1, l1); L++) {
+        load_ahead(L);
 #pragma unroll
-            for (int r = 0; r < RPW; r++) donor(t + 1, r, c_wmn[r], c_djrn[r]);
+        for (int r = 0; r < R; r++)
+            if (L == t0 && t0 > 0) vt[r] = top_flux(t0 - 1, own + r * PW, rowc[r]);
+        if (halo) {
+            load_ahead_b(L);
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                if (L == t0 && t0 > 0) vt_b[r] = top_flux(t0 - 1, top + r * PW, rowb[r]);
+            donor_halo(L);
+        } else {
+            float2 q1[R];
+            donor(L, own, j, n_wm, n_djr, vt, q1);
+#pragma unroll
+            for (int r = 0; r < R; r++) st2(at4(own, L), F_Q1, q1[r], r);
         }
-        // every thread is past iteration t-1 and the batch of iteration t
-        // landed (or the CTA stops): the planes that batch t+1 overwrites
-        // (q0 of t-2, U_m, V_m, J*rho of t-1, W_m/dz of t-2) are free.  The
-        // elected thread's warp has one row with nothing to do in P1, so
-        // the issue costs no time on the block's critical path.
-        ok = __syncthreads_and(landed ? 1 : 0) != 0;
-        if (!ok) goto drain;
-        if (threadIdx.x == 0) issue(&bars[(t + 1) & 1], t + 3, t + 2, t + 2, t + 1, t + 2);
-
-        float2 u2[RPW], v2[RPW], w2[RPW], fz[RPW];
-        float2 bxi[RPW], bxo[RPW], byi[RPW], byo[RPW], bzi[RPW], bzo[RPW];
-        if (haveA) {
-            const bool kint = t > 0 && t < nz - 1;
-            const bool top = t == nz - 1;
-            // ---- P1: pseudo-velocities at level t ---------------------------
-            // Each face block loads its own stencil (shared-memory loads are
-            // cheap; long live ranges across the three blocks are not).
-            const float *Qc = sQ1(t), *Qu = sQ1(t + 1), *Qd = sQ1(t - 1);
-            const float *Uc = sU(t), *Uup = sU(t + 1), *Vc = sV(t), *Vup = sV(t + 1);
-            const float *Wc = sW(t), *Wdn = sW(t - 1), *Gcp = sG(t), *Gup = sG(t + 1);
+    }
+    if (t0 + 2 <= l1) {
+        load_ahead(t0 + 2);
+        if (halo) load_ahead_b(t0 + 2);
+    }
 #pragma unroll
-            for (int r = 0; r < RPW; r++) {
-                u2[r] = v2[r] = w2[r] = fz[r] = zero2;
-                const int Y = rowY[r], j = rowj[r];
-                if (!(Y >= 2 && Y <= PH - 2)) continue;
-                const bool jin = INT || (j >= 0 && j < ny);
-                const bool jint = INT || (j > 0 && j < ny - 1);
-                // x faces ia, ib (west faces of the pair)
-                {
-                    const float2 qc = ld2(Qc, Y, X), Ut = ld2(Uc, Y, X), Gt = ld2(Gcp, Y, X);
-                    const float2 qcl = lft(qc), Gs = ad<EXACT>(Gt, lft(Gt));
-                    float2 val;
-                    if constexpr (EXACT) {
-                        val = base_x(Ut, Gs, qc, qcl);
-                        if (jint) {
-                            const float2 qn = ld2(Qc, Y + 1, X), qs = ld2(Qc, Y - 1, X);
-                            const float2 Vt = ld2(Vc, Y, X), Vtn = ld2(Vc, Y + 1, X);
-                            const float2 qnl = lft(qn), qsl = lft(qs);
-                            val = cross_x(val, Ut, avg4(Vt, Vtn, lft(Vt), lft(Vtn)),
-                                          div2x(xnum(qn, qs, qnl, qsl), xden(qn, qs, qnl, qsl)), Gs);
-                        }
-                        if (kint) {
-                            const float2 qu = ld2(Qu, Y, X), qd = ld2(Qd, Y, X);
-                            const float2 Wt = ld2(Wc, Y, X), Wd = ld2(Wdn, Y, X);
-                            const float2 qul = lft(qu), qdl = lft(qd);
-                            val = cross_x(val, Ut, avg4(Wt, Wd, lft(Wt), lft(Wd)),
-                                          div2x(xnum(qu, qd, qul, qdl), xden(qu, qd, qul, qdl)), Gs);
-                        }
-                        val = mul2x(val, splat2(0.5f));
-                    } else {
-                        // the final 0.5 folded in: 0.5 |U| (1 - 2 |U| / Gs) = 0.5 |U| - U^2 / Gs, and each
-                        // cross term 0.25 U / Gs times the 4-face average (1/4 of the face sum) times eq
-                        const float2 rG = rcp2(Gs);
-                        const float2 F0 = sub2(mul2(splat2(0.5f), abs2(Ut)), mul2(mul2(Ut, Ut), rG));
-                        val = mul2(mul2(F0, sub2(qc, qcl)), rcp2(add2(add2(qc, qcl), splat2(1e-10f))));
-                        const float2 mc = mul2(splat2(-0.0625f), mul2(Ut, rG));
-                        if (jint) {
-                            const float2 qn = ld2(Qc, Y + 1, X), qs = ld2(Qc, Y - 1, X);
-                            const float2 sv = add2(ld2(Vc, Y, X), ld2(Vc, Y + 1, X));
-                            const float2 xp = add2(qn, lft(qn)), xm = add2(qs, lft(qs));
-                            const float2 eq = mul2(sub2(xp, xm), rcp2(add2(add2(xp, xm), splat2(1e-10f))));
-                            val = fma2(mul2(mc, add2(sv, lft(sv))), eq, val);
-                        }
-                        if (kint) {
-                            const float2 qu = ld2(Qu, Y, X), qd = ld2(Qd, Y, X);
-                            const float2 sw = add2(ld2(Wc, Y, X), ld2(Wdn, Y, X));
-                            const float2 xp = add2(qu, lft(qu)), xm = add2(qd, lft(qd));
-                            const float2 eq = mul2(sub2(xp, xm), rcp2(add2(add2(xp, xm), splat2(1e-10f))));
-                            val = fma2(mul2(mc, add2(sw, lft(sw))), eq, val);
-                        }
-                    }
-                    u2[r] = val;
-                    if (!INT) {
-                        u2[r].x = (jin && ia >= 1 && ia <= nx - 1) ? val.x : 0.0f;
-                        u2[r].y = (jin && ib >= 1 && ib <= nx - 1) ? val.y : 0.0f;
-                    }
+    for (int r = 0; r < R; r++) n_dz[r] = ldcol(p.dz, rowc[r], t0);
+    __syncthreads();   // q1 of t0 and t0+1 complete
+
+    // ST: an iteration in the middle of a march, where every condition on the
+    // level holds; it compiles to few large blocks, which the scheduler can
+    // interleave.
+    auto level = [&](auto st, const int t) -> bool {
+        constexpr bool ST = decltype(st)::value;
+        const int n = t - t0;
+        const bool hor = ST || (t >= ka && t < kb);          // level t's horizontal terms are needed
+        bool landed;
+        if (!halo) {
+            float2 vs = zero2;
+            float *C = at4(own, t), *Up = at4(own, t + 1), *Dn = at4(own, t - 1);
+            // ---- P3: limited west and south faces of level t-1 -----------------
+            if (ST || t - 1 >= ka) {
+                const float2 q[R + 1] = {ld2(Dn, F_Q1, -1), ld2(Dn, F_Q1), ld2(Dn, F_Q1, 1)};
+                [[maybe_unused]] float2 bs = zero2, os = zero2;
+                if constexpr (FCT) {
+                    bs = ld2(own, S_BYI, -1);
+                    os = ld2(own, S_BYO, -1);
                 }
-                // y face j (south faces of the pair)
-                {
-                    const float2 qc = ld2(Qc, Y, X), qs = ld2(Qc, Y - 1, X);
-                    const float2 Vt = ld2(Vc, Y, X), Gs = ad<EXACT>(ld2(Gcp, Y, X), ld2(Gcp, Y - 1, X));
-                    const float2 Ut = ld2(Uc, Y, X), Us = ld2(Uc, Y - 1, X);
-                    const bool xa = INT || (ia > 0 && ia < nx - 1), xb = INT || (ib > 0 && ib < nx - 1);
-                    float2 val;
-                    if constexpr (EXACT) {
-                        const float2 qcl = lft(qc), qcr = rgt(qc), qsl = lft(qs), qsr = rgt(qs);
-                        const float2 Utr = rgt(Ut), Usr = rgt(Us);
-                        val = base_x(Vt, Gs, qc, qs);
-                        float2 eq = div2x(xnum(make_float2(qs.y, qsr.y), qcl, make_float2(qc.y, qcr.y), qsl),
-                                          xden(make_float2(qc.y, qcr.y), make_float2(qs.y, qsr.y), qcl, qsl));
-                        float2 ev = avg4(make_float2(Ut.y, Utr.y), make_float2(Us.y, Usr.y), Ut, Us);
-                        if (!xa) eq.x = ev.x = 0.0f;
-                        if (!xb) eq.y = ev.y = 0.0f;
-                        val = cross_x(val, Vt, ev, eq, Gs);
-                        if (kint) {
-                            const float2 qu = ld2(Qu, Y, X), qd = ld2(Qd, Y, X);
-                            const float2 qsu = ld2(Qu, Y - 1, X), qsd = ld2(Qd, Y - 1, X);
-                            const float2 Wt = ld2(Wc, Y, X), Wd = ld2(Wdn, Y, X);
-                            const float2 Wts = ld2(Wc, Y - 1, X), Wds = ld2(Wdn, Y - 1, X);
-                            val = cross_x(val, Vt, avg4(Wt, Wd, Wts, Wds), div2x(xnum(qsu, qd, qu, qsd),
-                                                                                xden(qsu, qd, qu, qsd)), Gs);
-                        }
-                        val = mul2x(val, splat2(0.5f));
+                float2 below = zero2;   // the first row's south flux
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    const float2 qc = q[r + 1], qcl = lft(qc);
+                    Split u, v;
+                    if constexpr (FCT) {
+                        u = limit<M>(u2[r], bxi[r], lft(bxo[r]), lft(bxi[r]), bxo[r]);
+                        v = limit<M>(v2[r], byi[r], os, bs, byo[r]);
+                        bs = byi[r];
+                        os = byo[r];
                     } else {
-                        const float2 rG = rcp2(Gs);
-                        const float2 F0 = sub2(mul2(splat2(0.5f), abs2(Vt)), mul2(mul2(Vt, Vt), rG));
-                        val = mul2(mul2(F0, sub2(qc, qs)), rcp2(add2(add2(qc, qs), splat2(1e-10f))));
-                        const float2 mc = mul2(splat2(-0.0625f), mul2(Vt, rG));
-                        // x cross term: the two rows' pair sums at x+1 and x-1, and U_m on the
-                        // cells' west and east faces in both rows, each formed from one shuffle
-                        const float2 sq = add2(qc, qs), yp = rgt(sq), ym = lft(sq);
-                        float2 eq = mul2(sub2(yp, ym), rcp2(add2(add2(yp, ym), splat2(1e-10f))));
-                        const float2 su = add2(Ut, Us);
-                        float2 ev = add2(su, rgt(su));
-                        // no cross term on the domain's first and last columns (their
-                        // shuffled neighbours may lie outside the plane)
-                        if (!xa) ev.x = eq.x = 0.0f;
-                        if (!xb) ev.y = eq.y = 0.0f;
-                        val = fma2(mul2(mc, ev), eq, val);
-                        if (kint) {
-                            const float2 zp = add2(ld2(Qu, Y, X), ld2(Qu, Y - 1, X));
-                            const float2 zm = add2(ld2(Qd, Y, X), ld2(Qd, Y - 1, X));
-                            const float2 eq2 = mul2(sub2(zp, zm), rcp2(add2(add2(zp, zm), splat2(1e-10f))));
-                            const float2 sw = add2(add2(ld2(Wc, Y, X), ld2(Wdn, Y, X)),
-                                                   add2(ld2(Wc, Y - 1, X), ld2(Wdn, Y - 1, X)));
-                            val = fma2(mul2(mc, sw), eq2, val);
-                        }
+                        u = split<M>(u2[r]);
+                        v = split<M>(v2[r]);
                     }
-                    v2[r] = val;
-                    if (!INT) {
-                        const bool fin = j >= 1 && j <= ny - 1;
-                        v2[r].x = (fin && inA) ? val.x : 0.0f;
-                        v2[r].y = (fin && inB) ? val.y : 0.0f;
+                    // east faces as the next cell's limited west faces
+                    const float2 fw = flux<M>(qcl, qc, u, nz2), fn = flux<M>(q[r], qc, v, nz2);
+                    hx[r] = sb<M>(rgt(fw), fw);
+                    gm[r] = ld2(Dn, F_G, r);   // its plane is refilled after the next barrier
+                    if (r == 0) {
+                        below = fn;
+                        vs = join<M>(v);
+                    } else {   // the first row's divergence is complete
+                        hx[0] = ad<M>(hx[0], north_less<M>(q[r], qc, v, below, nz2));
+                        fs = fn;
                     }
-                    st2(P(S_V2), Y, X, v2[r]);
-                }
-                // z face at the top of level t (columns inside the domain interior)
-                if (!top) {
-                    const float2 qc = ld2(Qc, Y, X), qu = ld2(Qu, Y, X);
-                    const float2 Wt = ld2(Wc, Y, X), Gs = ad<EXACT>(ld2(Gup, Y, X), ld2(Gcp, Y, X));
-                    const float2 Ut = ld2(Uc, Y, X), Uu = ld2(Uup, Y, X);
-                    const float2 qn = ld2(Qc, Y + 1, X), qs = ld2(Qc, Y - 1, X);
-                    const float2 qnu = ld2(Qu, Y + 1, X), qsu = ld2(Qu, Y - 1, X);
-                    const float2 Vt = ld2(Vc, Y, X), Vtn = ld2(Vc, Y + 1, X);
-                    const float2 Vu = ld2(Vup, Y, X), Vun = ld2(Vup, Y + 1, X);
-                    float2 val;
-                    if constexpr (EXACT) {
-                        const float2 qcl = lft(qc), qcr = rgt(qc), qul = lft(qu), qur = rgt(qu);
-                        const float2 Utr = rgt(Ut), Uur = rgt(Uu);
-                        val = base_x(Wt, Gs, qu, qc);
-                        val = cross_x(val, Wt, avg4(make_float2(Ut.y, Utr.y), make_float2(Uu.y, Uur.y), Ut, Uu),
-                                      div2x(xnum(make_float2(qu.y, qur.y), qcl, make_float2(qc.y, qcr.y), qul),
-                                            xden(make_float2(qc.y, qcr.y), make_float2(qu.y, qur.y), qcl, qul)),
-                                      Gs);
-                        val = cross_x(val, Wt, avg4(Vt, Vu, Vtn, Vun), div2x(xnum(qnu, qs, qn, qsu), xden(qn, qsu, qnu, qs)),
-                                      Gs);
-                        val = mul2x(mul2x(val, splat2(0.5f)), c_dz[r]);
-                    } else {
-                        const float2 rG = rcp2(Gs);
-                        const float2 F0 = sub2(mul2(splat2(0.5f), abs2(Wt)), mul2(mul2(Wt, Wt), rG));
-                        val = mul2(mul2(F0, sub2(qu, qc)), rcp2(add2(add2(qu, qc), splat2(1e-10f))));
-                        const float2 mc = mul2(splat2(-0.0625f), mul2(Wt, rG));
-                        const float2 sq = add2(qc, qu), zp = rgt(sq), zm = lft(sq);
-                        const float2 eq = mul2(sub2(zp, zm), rcp2(add2(add2(zp, zm), splat2(1e-10f))));
-                        const float2 su = add2(Ut, Uu);
-                        val = fma2(mul2(mc, add2(su, rgt(su))), eq, val);
-                        const float2 np = add2(qn, qnu), sp = add2(qs, qsu);
-                        const float2 eq2 = mul2(sub2(np, sp), rcp2(add2(add2(np, sp), splat2(1e-10f))));
-                        const float2 sv = add2(add2(Vt, Vu), add2(Vtn, Vun));
-                        val = fma2(mul2(mc, sv), eq2, val);
-                        val = mul2(val, c_dz[r]);
-                    }
-                    w2[r] = val;
-                    if (!INT) {
-                        const bool jj = j >= 1 && j <= ny - 2;
-                        w2[r].x = (jj && ia >= 1 && ia <= nx - 2) ? val.x : 0.0f;
-                        w2[r].y = (jj && ib >= 1 && ib <= nx - 2) ? val.y : 0.0f;
-                    }
-                    fz[r] = flux<EXACT>(qc, qu, w2[r]);
                 }
             }
-            __syncthreads();   // v2 plane complete
+            landed = wait_mine(n);
+            // ---- P0: q1 at level t+2 ----------------------------------------
+            float2 q1n[R], fv[R];
+            if (ST || t + 2 <= l1) donor(t + 2, own, j, n_wm, n_djr, vt, q1n);
+            // ---- P1: pseudo-velocities at level t -----------------------------
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                w2b[r] = w2[r];
+                fzb[r] = fz[r];
+            }
+            if (ST || t <= tl) {
+                const float2 qc[R + 2] = {ld2(C, F_Q1, -1), ld2(C, F_Q1), ld2(C, F_Q1, 1), ld2(C, F_Q1, 2)};
+                const float2 qu[R + 2] = {ld2(Up, F_Q1, -1), ld2(Up, F_Q1), ld2(Up, F_Q1, 1), ld2(Up, F_Q1, 2)};
+                const float2 U[R + 1] = {ld2(C, F_U, -1), ld2(C, F_U), ld2(C, F_U, 1)};
+                const float2 V[R + 1] = {ld2(C, F_V), ld2(C, F_V, 1), ld2(C, F_V, 2)};
+                const float2 W[R + 1] = {ld2(C, F_WP, -1), ld2(C, F_WP), ld2(C, F_WP, 1)};
+                const float2 G[R + 1] = {ld2(C, F_G, -1), ld2(C, F_G), ld2(C, F_G, 1)};
+                if (hor) {
+                    const float2 qd[R + 1] = {ld2(Dn, F_Q1, -1), ld2(Dn, F_Q1), ld2(Dn, F_Q1, 1)};
+                    const float2 Wd[R + 1] = {ld2(Dn, F_WP, -1), ld2(Dn, F_WP), ld2(Dn, F_WP, 1)};
+#pragma unroll
+                    for (int r = 0; r < R; r++) {
+                        v2[r] = face_y(st, t, j + r, qc[r + 1], qc[r], qu[r + 1], qu[r], qd[r + 1], qd[r], V[r], G[r + 1], G[r],
+                                       U[r + 1], U[r], W[r + 1], Wd[r + 1], W[r], Wd[r], fv[r]);
+                        u2[r] = face_x(st, t, j + r, qc[r + 1], qc[r + 2], qc[r], qu[r + 1], qd[r + 1], U[r + 1], G[r + 1], V[r],
+                                       V[r + 1], W[r + 1], Wd[r + 1]);
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < R; r++) w2[r] = fz[r] = zero2;
+                if (ST || t < nz - 1) {
+                    const float2 Vu[R + 1] = {ld2(Up, F_V), ld2(Up, F_V, 1), ld2(Up, F_V, 2)};
+#pragma unroll
+                    for (int r = 0; r < R; r++) {
+                        w2[r] = face_z(j + r, n_dz[r], qc[r + 1], qu[r + 1], qc[r + 2], qc[r], qu[r + 2], qu[r], W[r + 1],
+                                       G[r + 1], ld2(Up, F_G, r), U[r + 1], ld2(Up, F_U, r), V[r], V[r + 1], Vu[r],
+                                       Vu[r + 1]);
+                        if constexpr (FCT) fz[r] = lflux<M>(qc[r + 1], qu[r + 1], w2[r], nz2);
+                    }
+                }
+            }
+            if (ST || t + 2 <= l1) {
+#pragma unroll
+                for (int r = 0; r < R; r++) st2(at4(own, t + 2), F_Q1, q1n[r], r);
+            }
+            if (FCT && hor) {
+#pragma unroll
+                for (int r = 0; r < R; r++) st2(own, S_FV, fv[r], r);
+            }
+            if (ST || t - 1 >= ka) st2(own, S_FY, vs);   // for the row south of the first: its north faces
+        } else {
+            // the halo warp: south faces of row 25 (limited, for row 24's north
+            // faces), P0 of its four rows, south faces of rows 2, 25 and 26
+            if (ST || t - 1 >= ka) {
+                Split v;
+                if constexpr (FCT)
+                    v = limit<M>(v2[0], ld2(top, S_BYI), ld2(top, S_BYO, -1), ld2(top, S_BYI, -1), ld2(top, S_BYO));
+                else v = split<M>(v2[0]);
+                st2(top, S_FY, join<M>(v));
+            }
+            landed = wait_mine(n);
+            if (ST || t + 2 <= l1) donor_halo(t + 2);
+            if (hor) {
+#pragma unroll 1
+                for (int q = 0; q < 3; q++) {
+                    const int yr = q == 0 ? 2 : YB - 1 + q;
+                    float2 f;
+                    const float2 v = face_y_row(st, t, yr, f);
+                    if (q == 1) v2[0] = v;
+                    if constexpr (FCT) st2(sm + yr * PW + X, S_FV, f);
+                }
+            }
+        }
+        // every thread is past I1 of t and the batch of iteration n has
+        // landed (or the CTA stops): the planes that batch n+1 overwrites (q0
+        // of t-4, the others of t-1) are free
+        if (__syncthreads_and(landed ? 1 : 0) == 0) return drain(n);
+        if (threadIdx.x == 0 && (ST || t < kb)) issue(t + 1);
 
+        // own-column values for the next iteration and this one's store
+        if (ST || t + 3 <= l1) {
+            load_ahead(t + 3);
+            if (halo) load_ahead_b(t + 3);
+        }
+        if (halo) {
+            if (FCT && hor) {
+#pragma unroll 1
+                for (int q = 0; q < 2; q++) {
+                    const int yr = q == 0 ? 2 : PH - 3;
+                    float *at = sm + yr * PW + X;
+                    const float *Q1 = at4(at, t), *Q0 = atq(at, t);
+                    float2 bi, bo;
+                    betas_y(y0 + yr, at, ld2(Q1, F_Q1), ld2(Q0, 0), ld2(Q1, F_Q1, -1), ld2(Q0, 0, -1), ld2(Q1, F_Q1, 1),
+                            ld2(Q0, 0, 1), ld2(at, S_FV), bi, bo);
+                    st2(at, S_BYI, bi);
+                    st2(at, S_BYO, bo);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                if (ST || t + 1 <= tl) n_dz[r] = ldcol(p.dz, rowc[r], t + 1);
+                if (ST || t - 1 >= ka) djr_m[r] = ldcol(p.DJR, rowc[r], t - 1);
+            }
+            const float *C = at4(own, t), *Up = at4(own, t + 1), *Dn = at4(own, t - 1);
+            float2 pbi[R], pbo[R];   // the z betas of t-1
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                pbi[r] = bzi[r];
+                pbo[r] = bzo[r];
+            }
             // ---- P2: limiter betas at level t --------------------------------
+            if (FCT && (ST || (t <= tl && t >= ka - 1))) {
+                const float *Q0 = atq(own, t);
+                const float2 qc[R + 2] = {ld2(C, F_Q1, -1), ld2(C, F_Q1), ld2(C, F_Q1, 1), ld2(C, F_Q1, 2)};
+                const float2 q0[R + 2] = {ld2(Q0, 0, -1), ld2(Q0, 0), ld2(Q0, 0, 1), ld2(Q0, 0, 2)};
 #pragma unroll
-            for (int r = 0; r < RPW; r++) {
-                bxi[r] = bxo[r] = byi[r] = byo[r] = bzi[r] = bzo[r] = splat2(0.0f);
-                const int Y = rowY[r], j = rowj[r];
-                if (!FCT || !(Y >= 2 && Y <= PH - 3)) continue;
-                const float2 qc = ld2(sQ1(t), Y, X), q0c = ld2(sq0(t), Y, X);
-                const float2 qcl = lft(qc), qcr = rgt(qc), q0l = lft(q0c), q0r = rgt(q0c);
-                // x lines: faces ia, ib, ib+1
-                {
-                    const float2 fl = flux<EXACT>(qcl, qc, u2[r]), fr = rgt(fl);
-                    if constexpr (INT && !EXACT) {
-                        fct_pair_fast(qcl, qc, qcr, q0l, q0c, q0r, fl, fr, bxi[r], bxo[r]);
-                    } else if constexpr (!EXACT) {
-                        float2 a1m = qcl, a1p = qcr, a0m = q0l, a0c = q0c, a0p = q0r, afl = fl, afr = fr;
-                        fct_edge_sub(ia == 0, ia == nx - 1, a1m.x, qc.x, a1p.x, a0m.x, a0c.x, a0p.x, afl.x, afr.x);
-                        fct_edge_sub(ib == 0, ib == nx - 1, a1m.y, qc.y, a1p.y, a0m.y, a0c.y, a0p.y, afl.y, afr.y);
-                        fct_pair_fast(a1m, qc, a1p, a0m, a0c, a0p, afl, afr, bxi[r], bxo[r]);
-                    } else {
-                        const int pa = INT ? 0 : (ia == 0 ? 1 : (ia == nx - 1 ? 2 : 0));
-                        const int pb = INT ? 0 : (ib == 0 ? 1 : (ib == nx - 1 ? 2 : 0));
-                        fct_cell<EXACT>(qcl.x, qc.x, qcr.x, q0l.x, q0c.x, q0r.x, fl.x, fr.x, pa, false, bxi[r].x,
-                                        bxo[r].x);
-                        fct_cell<EXACT>(qcl.y, qc.y, qcr.y, q0l.y, q0c.y, q0r.y, fl.y, fr.y, pb, false, bxi[r].y,
-                                        bxo[r].y);
-                    }
-                }
-                // y lines: faces j and j+1
-                {
-                    const float2 qn = ld2(sQ1(t), Y + 1, X), qs = ld2(sQ1(t), Y - 1, X);
-                    const float2 q0n = ld2(sq0(t), Y + 1, X), q0s = ld2(sq0(t), Y - 1, X);
-                    const float2 vn = ld2(P(S_V2), Y + 1, X);
-                    const float2 fl = flux<EXACT>(qs, qc, v2[r]), fr = flux<EXACT>(qc, qn, vn);
-                    if constexpr (INT && !EXACT) {
-                        fct_pair_fast(qs, qc, qn, q0s, q0c, q0n, fl, fr, byi[r], byo[r]);
-                    } else if constexpr (!EXACT) {
-                        float2 a1m = qs, a1p = qn, a0m = q0s, a0c = q0c, a0p = q0n, afl = fl, afr = fr;
-                        if (j == 0 || j == ny - 1) {   // row-uniform
-                            fct_edge_sub(j == 0, j == ny - 1, a1m.x, qc.x, a1p.x, a0m.x, a0c.x, a0p.x, afl.x, afr.x);
-                            fct_edge_sub(j == 0, j == ny - 1, a1m.y, qc.y, a1p.y, a0m.y, a0c.y, a0p.y, afl.y, afr.y);
+                for (int r = 0; r < R; r++) {
+                    const float2 q = qc[r + 1], hi = max2(q, q0[r + 1]), lo = min2(q, q0[r + 1]);
+                    if (hor) {
+                        // x lines: faces ia, ib, ib+1
+                        {
+                            const float2 fl = lflux<M>(lft(q), q, u2[r], nz2), fr = rgt(fl);
+                            float2 hl = lft(hi), hr = rgt(hi), ll = lft(lo), lr = rgt(lo), hc = hi, lc = lo;
+                            float2 afl = fl, afr = fr;
+                            if (!INT) {
+                                // line ends: the first cell's bounds omit the cell before it;
+                                // the last cell's omit the cell after it and its own old
+                                // value; both have no flux sums
+                                if (ia == 0) { hl.x = hi.x; ll.x = lo.x; }
+                                if (ib == 0) { hl.y = hi.y; ll.y = lo.y; }
+                                if (ia == nx - 1) { hc.x = lc.x = hr.x = lr.x = q.x; }
+                                if (ib == nx - 1) { hc.y = lc.y = hr.y = lr.y = q.y; }
+                                if (ia == 0 || ia == nx - 1) afl.x = afr.x = 0.0f;
+                                if (ib == 0 || ib == nx - 1) afl.y = afr.y = 0.0f;
+                            }
+                            betas<M>(max2(max2(hl, hc), hr), min2(min2(ll, lc), lr), q, afl, afr, bxi[r], bxo[r]);
                         }
-                        fct_pair_fast(a1m, qc, a1p, a0m, a0c, a0p, afl, afr, byi[r], byo[r]);
-                    } else {
-                        const int pj = INT ? 0 : (j == 0 ? 1 : (j == ny - 1 ? 2 : 0));
-                        fct_cell<EXACT>(qs.x, qc.x, qn.x, q0s.x, q0c.x, q0n.x, fl.x, fr.x, pj, false, byi[r].x,
-                                        byo[r].x);
-                        fct_cell<EXACT>(qs.y, qc.y, qn.y, q0s.y, q0c.y, q0n.y, fl.y, fr.y, pj, false, byi[r].y,
-                                        byo[r].y);
+                        // y lines: faces j and j+1
+                        betas_y(j + r, own + r * PW, q, q0[r + 1], qc[r], q0[r], qc[r + 2], q0[r + 2],
+                                lflux<M>(qc[r], q, v2[r], nz2), byi[r], byo[r]);
                     }
-                    st2(P(S_BYI), Y, X, byi[r]);
-                    st2(P(S_BYO), Y, X, byo[r]);
-                }
-                // z line of the own column (fz of the faces below and above)
-                {
-                    const float2 qu = t < nz - 1 ? ld2(sQ1(t + 1), Y, X) : zero2;
-                    const float2 qd = t > 0 ? ld2(sQ1(t - 1), Y, X) : zero2;
-                    const float2 q0u = t < nz - 1 ? ld2(sq0(t + 1), Y, X) : zero2;
-                    const float2 q0d = t > 0 ? ld2(sq0(t - 1), Y, X) : zero2;
-                    // flux through the top of level t-1, as P1 formed it one level ago
-                    const float2 fzd = flux<EXACT>(qd, qc, r_w2[r]);
-                    const int pz = t == 0 ? 1 : (t == nz - 1 ? 2 : 0);
-                    if (!EXACT && pz == 0) {
-                        fct_pair_fast(qd, qc, qu, q0d, q0c, q0u, fzd, fz[r], bzi[r], bzo[r]);
-                    } else {
-                        fct_cell<EXACT>(qd.x, qc.x, qu.x, q0d.x, q0c.x, q0u.x, fzd.x, fz[r].x, pz, true, bzi[r].x,
-                                        bzo[r].x);
-                        fct_cell<EXACT>(qd.y, qc.y, qu.y, q0d.y, q0c.y, q0u.y, fzd.y, fz[r].y, pz, true, bzi[r].y,
-                                        bzo[r].y);
+                    // z line of the own column (its ends keep their fluxes)
+                    {
+                        float2 hd = hi, ld = lo, hu = hi, lu = lo, hc = hi, lc = lo, fr = fz[r];
+                        if (ST || t > 0) {
+                            const float2 qd = ld2(Dn, F_Q1, r), q0d = ld2(atq(own, t - 1), 0, r);
+                            hd = max2(qd, q0d);
+                            ld = min2(qd, q0d);
+                        }
+                        if (ST || t < nz - 1) {
+                            const float2 qu = ld2(Up, F_Q1, r), q0u = ld2(atq(own, t + 1), 0, r);
+                            hu = max2(qu, q0u);
+                            lu = min2(qu, q0u);
+                        } else {
+                            hc = lc = hu = lu = q;
+                            fr = fzb[r];
+                        }
+                        betas<M>(max2(max2(hd, hc), hu), min2(min2(ld, lc), lu), q, fzb[r], fr, bzi[r], bzo[r]);
                     }
                 }
             }
-            __syncthreads();   // y betas complete
-        }
-
-        // ---- P3: limited faces, corrective pass; output level t-1 ----------
+            // ---- level t-1: the limited flux through its top, the update ---------
+            if (ST || t >= ka) {
 #pragma unroll
-        for (int r = 0; r < RPW; r++) {
-            const int Y = rowY[r], j = rowj[r];
-            const bool outrow = Y >= 3 && Y <= PH - 4;      // warp-uniform
-            // n_ft: the limited flux through the top of level t-1, formed with
-            // the level-t betas and carried to the next level as its bottom flux
-            float2 n_part = zero2, n_ft = zero2;
-            if (haveA && outrow) {
-                const float2 qc = ld2(sQ1(t), Y, X), qn = ld2(sQ1(t), Y + 1, X), qs = ld2(sQ1(t), Y - 1, X);
-                const float2 qcl = lft(qc);
-                const float2 vn0 = ld2(P(S_V2), Y + 1, X);
-                float2 fw, f3, f4;
-                if constexpr (EXACT) {
-                    float2 uw = u2[r], vs = v2[r], vn = vn0;
-                    if (FCT) {
-                        const float2 bil = lft(bxi[r]), bol = lft(bxo[r]);
-                        uw.x = limit<EXACT>(uw.x, bxi[r].x, bol.x, bil.x, bxo[r].x);
-                        uw.y = limit<EXACT>(uw.y, bxi[r].y, bxo[r].x, bxi[r].x, bxo[r].y);
-                        const float2 bis = ld2(P(S_BYI), Y - 1, X), bos = ld2(P(S_BYO), Y - 1, X);
-                        const float2 bin = ld2(P(S_BYI), Y + 1, X), bon = ld2(P(S_BYO), Y + 1, X);
-                        vs.x = limit<EXACT>(vs.x, byi[r].x, bos.x, bis.x, byo[r].x);
-                        vs.y = limit<EXACT>(vs.y, byi[r].y, bos.y, bis.y, byo[r].y);
-                        vn.x = limit<EXACT>(vn.x, bin.x, byo[r].x, byi[r].x, bon.x);
-                        vn.y = limit<EXACT>(vn.y, bin.y, byo[r].y, byi[r].y, bon.y);
+                for (int r = 0; r < R; r++) {
+                    float2 ft = zero2;
+                    const float2 qd = ld2(Dn, F_Q1, r);   // q1 of t-1
+                    if (ST || (t >= 1 && t < nz)) {
+                        const float2 qc = ld2(C, F_Q1, r);
+                        if constexpr (FCT) ft = flux<M>(qd, qc, limit<M>(w2b[r], bzi[r], pbo[r], pbi[r], bzo[r]), nz2);
+                        else ft = flux<M>(qd, qc, split<M>(w2b[r]), nz2);
+                    } else if (M == A_IEEE && t >= 1) {
+                        ft = mul2x(qd, zero2);   // the model top: q times a face velocity of zero
                     }
-                    fw = flux_x(qcl, qc, uw);
-                    f3 = flux_x(qc, qn, vn);
-                    f4 = flux_x(qs, qc, vs);
-                } else if (FCT) {
-                    const float2 bis = ld2(P(S_BYI), Y - 1, X), bos = ld2(P(S_BYO), Y - 1, X);
-                    const float2 bin = ld2(P(S_BYI), Y + 1, X), bon = ld2(P(S_BYO), Y + 1, X);
-                    fw = lim_flux2(u2[r], qcl, qc, bxi[r], lft(bxo[r]), lft(bxi[r]), bxo[r]);
-                    f4 = lim_flux2(v2[r], qs, qc, byi[r], bos, bis, byo[r]);
-                    f3 = lim_flux2(vn0, qc, qn, bin, byo[r], byi[r], bon);
-                } else {
-                    fw = flux_f(qcl, qc, u2[r]);
-                    f3 = flux_f(qc, qn, vn0);
-                    f4 = flux_f(qs, qc, v2[r]);
-                }
-                // east faces as the next cell's limited west faces
-                const float2 fe = rgt(fw);
-                const float2 hd = ad<EXACT>(sb<EXACT>(fe, fw), sb<EXACT>(f3, f4));
-                const float2 G = ld2(sG(t), Y, X);
-                if constexpr (EXACT) n_part = sub2x(qc, div2x(hd, G));
-                else n_part = sub2(qc, mul2(hd, r_rg[r]));
-                if (t >= 1) {
-                    const float2 qd = ld2(sQ1(t - 1), Y, X);
-                    if constexpr (EXACT) {
-                        float2 w = r_w2[r];
-                        if (FCT) {
-                            w.x = limit<EXACT>(w.x, bzi[r].x, r_bzo[r].x, r_bzi[r].x, bzo[r].x);
-                            w.y = limit<EXACT>(w.y, bzi[r].y, r_bzo[r].y, r_bzi[r].y, bzo[r].y);
+                    if (ST || t - 1 >= ka) {
+                        const int L = t - 1, jr = j + r;
+                        float2 hd = hx[r];
+                        if (r + 1 == R)
+                            hd = ad<M>(hd, north_less<M>(qd, ld2(Dn, F_Q1, R), unjoin<M>(ld2(own, S_FY, R)), fs, nz2));
+                        const float2 vd = sb<M>(ft, fb[r]);
+                        const float2 G = gm[r];
+                        float2 val;
+                        if constexpr (M == A_IEEE) {
+                            val = sub2x(sub2x(qd, div2x(hd, G)), div2x(vd, djr_m[r]));
+                        } else if constexpr (M == A_EXACT) {
+                            val = add2(qd, nquot(hd, exdiv(G, S48, R48), tie));
+                            val = add2(val, nquot(vd, exdiv(djr_m[r], S48, R48), tie));
+                        } else {
+                            val = sub2(sub2(qd, mul2(hd, half_of(rcp2(G)))), mul2(vd, half_of(rcp2(djr_m[r]))));
                         }
-                        n_ft = flux_x(qd, qc, w);
-                    } else if (FCT) {
-                        n_ft = lim_flux2(r_w2[r], qd, qc, bzi[r], r_bzo[r], r_bzi[r], bzo[r]);
-                    } else {
-                        n_ft = flux_f(qd, qc, r_w2[r]);
+                        const bool oa = sta && jin(jr), ob = stb && jin(jr);
+                        if (!INT) {
+                            const bool jring = jr == 0 || jr == ny - 1;
+                            const float2 q0L = ld2(atq(own, L), 0, r);
+                            if (jring || ia == 0 || ia == nx - 1) val.x = q0L.x;
+                            if (jring || ib == 0 || ib == nx - 1) val.y = q0L.y;
+                        }
+                        if constexpr (M == A_EXACT) worst_of(worst, make_float2(oa ? val.x : 0.0f, ob ? val.y : 0.0f));
+                        if (oa || ob) {
+                            float *dst = outs + (rowc[r] + (uint32_t)L * lstride);
+                            if (oa && ob) *reinterpret_cast<float2 *>(dst) = val;
+                            else if (oa) dst[0] = val.x;
+                            else dst[1] = val.y;
+                        }
                     }
+                    fb[r] = ft;
                 }
             }
-            // vertical part of level L = t-1 and the store
-            if (t >= 1 && outrow) {
-                const int L = t - 1;
-                float2 val = r_part[r];
-                const float2 djr = r_djrm[r];
-                if constexpr (EXACT) {
-                    if (L > 0 && L < nz - 1) {
-                        val = sub2x(val, div2x(sub2x(n_ft, r_fb[r]), djr));
-                    } else if (L == 0) {
-                        val = sub2x(val, div2x(n_ft, djr));
-                    } else {
-                        // the model top: q times the (zero) face velocity there
-                        const float2 qc = ld2(sQ1(L), Y, X);
-                        val = sub2x(val, div2x(sub2x(mul2x(qc, zero2), r_fb[r]), djr));
-                    }
-                } else {
-                    float2 vd;
-                    if (L > 0 && L < nz - 1) vd = sub2(n_ft, r_fb[r]);
-                    else if (L == 0) vd = n_ft;
-                    else vd = make_float2(-r_fb[r].x, -r_fb[r].y);   // nothing leaves through the model top
-                    val = sub2(val, mul2(vd, djr));
-                }
-                const bool jin = INT || (j >= 0 && j < ny);
-                const bool jring = !INT && (j == 0 || j == ny - 1);
-                const bool oa = jin && (INT || inA) && X >= xlo && X < xhi;
-                const bool ob = jin && (INT || inB) && X + 1 >= xlo && X + 1 < xhi;
-                float va = val.x, vb = val.y;
-                if (!INT) {
-                    const float2 q0L = ld2(sq0(L), Y, X);
-                    va = (jring || ia == 0 || ia == nx - 1) ? q0L.x : val.x;
-                    vb = (jring || ib == 0 || ib == nx - 1) ? q0L.y : val.y;
-                }
-                if (oa || ob) {
-                    // ia is even and rows start on 16-byte boundaries: the pair is 8-byte aligned
-                    float *dst = outg + ix(g, 0, L, j);
-                    if (oa && ob) *reinterpret_cast<float2 *>(dst + ia) = make_float2(va, vb);
-                    else if (oa) dst[ia] = va;
-                    else dst[ib] = vb;
-                }
-            }
-            // rotate the carried state
-            if (haveA) {
-                r_fb[r] = n_ft;
-                r_part[r] = n_part;
-                r_w2[r] = w2[r];
-                r_bzi[r] = bzi[r];
-                r_bzo[r] = bzo[r];
-            }
-            r_djrm[r] = r_djr0[r];
-            r_djr0[r] = c_djrn[r];
         }
+        if (FCT && hor && !halo) {
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                st2(own, S_BYI, byi[r], r);
+                st2(own, S_BYO, byo[r], r);
+            }
+        }
+        if (ST || t < kb) __syncthreads();   // y betas complete; level t-1 is done with
+        return true;
+    };
+#pragma unroll 1
+    for (int t = t0; t <= kb; t++) {
+        const bool mid = M != A_IEEE && t > ka && t <= l1 - 3 && t < kb;
+        if (mid ? !level(std::bool_constant<M != A_IEEE>{}, t) : !level(std::false_type{}, t)) return false;
     }
     return true;
-
-drain:
-    // a wait gave up: wait (bounded) for both barriers' latest batches so
-    // no copy is left in flight into this CTA's shared memory, then stop
-    mbar_wait_bounded(&bars[0], (ph[0] - 1) & 1u, WAIT_NS);
-    mbar_wait_bounded(&bars[1], (ph[1] - 1) & 1u, WAIT_NS);
-    return false;
 }
 
-// Barrier set-up, once per CTA.
-__device__ __forceinline__ void onepass_init_bars(uint64_t *bars, uint32_t *ph)
+// Barrier set-up (threads of the CTA are synchronised by it).
+__device__ __forceinline__ void onepass_init_bars(uint64_t *bars)
 {
     if (threadIdx.x == 0) {
         mbar_init(&bars[0], 1);
         mbar_init(&bars[1], 1);
         mbar_fence_init();
     }
-    ph[0] = ph[1] = 0;
     __syncthreads();
 }
 
@@ -962,18 +1176,62 @@ __device__ __forceinline__ bool onepass_interior(const Geo &g, int x0, int j0)
     return x0 >= 1 && x0 + op::PW - 1 <= g.nx - 2 && j0 - 3 >= 1 && j0 - 3 + op::PH - 1 <= g.ny - 2;
 }
 
-// Tile (tx, j0) of a domain: plane origin and output columns, then the march.
-template <bool EXACT, bool FCT>
-__device__ __forceinline__ bool onepass_run(float *sm, uint64_t *bars, uint32_t *ph, const OnePassParams &p, int s,
-                                            int tx, int j0)
+// Tile (tx, j0) of a domain, output levels [ka, kb): plane origin and output
+// columns, then the march.
+template <int M, bool FCT>
+__device__ __forceinline__ bool onepass_run(float *sm, uint64_t *bars, const OnePassParams &p, int s, int tx, int j0,
+                                            int ka, int kb, bool tie, float &worst)
 {
     int x0, xlo, xhi;
     op::xtile(p.g.nx, tx, p.tiles_x, x0, xlo, xhi);
-    if (onepass_interior(p.g, x0, j0)) return onepass_tile<EXACT, FCT, true>(sm, bars, ph, p, s, x0, xlo, xhi, j0);
-    return onepass_tile<EXACT, FCT, false>(sm, bars, ph, p, s, x0, xlo, xhi, j0);
+    if (onepass_interior(p.g, x0, j0))
+        return onepass_tile<M, FCT, true>(sm, bars, p, s, x0, xlo, xhi, j0, ka, kb, tie, worst);
+    return onepass_tile<M, FCT, false>(sm, bars, p, s, x0, xlo, xhi, j0, ka, kb, tie, worst);
 }
 
-template <bool EXACT, bool FCT>
+// The march with IEEE division, out of line, so that it costs the others no
+// registers.
+template <bool FCT>
+__device__ __noinline__ void onepass_redo(float *sm, uint64_t *bars, const OnePassParams &p, int s, int tx, int j0, int ka,
+                                          int kb)
+{
+    if (threadIdx.x == 0) {
+        mbar_inval(&bars[0]);
+        mbar_inval(&bars[1]);
+    }
+    __syncthreads();
+    onepass_init_bars(bars);
+    float worst = 0.0f;
+    int x0, xlo, xhi;
+    op::xtile(p.g.nx, tx, p.tiles_x, x0, xlo, xhi);
+    onepass_tile<opx::A_IEEE, FCT, false>(sm, bars, p, s, x0, xlo, xhi, j0, ka, kb, false, worst);
+}
+
+// One work item of either form.  A_EXACT: a tile whose fields or values lie
+// outside what its quotients are proven for (the prep kernel's FLAG_IEEE, or
+// `worst` at the end of the march) is marched with IEEE division; the tile's
+// stores are then overwritten, which no other tile reads.
+template <int M, bool FCT>
+__device__ __forceinline__ void onepass_item(float *sm, uint64_t *bars, const OnePassParams &p, int s, int tx, int j0,
+                                             int ka, int kb)
+{
+    float worst = 0.0f;
+    if constexpr (M == opx::A_EXACT) {
+        const bool tie = p.flags[FLAG_TIE] == p.epoch;
+        bool redo = p.flags[FLAG_IEEE] == p.epoch;
+        if (!redo) {
+            if (!onepass_run<M, FCT>(sm, bars, p, s, tx, j0, ka, kb, tie, worst)) return;
+            redo = __syncthreads_or(worst < opx::EXACT_MAX ? 0 : 1) != 0;
+        }
+        if (redo) onepass_redo<FCT>(sm, bars, p, s, tx, j0, ka, kb);
+    } else {
+        onepass_run<M, FCT>(sm, bars, p, s, tx, j0, ka, kb, false, worst);
+    }
+}
+
+// Grid: species fastest, so the CTAs of a tile run together and share its
+// wind and metric planes through L2.
+template <int M, bool FCT>
 __global__ void __launch_bounds__(op::NT, 1) k_mpdata_onepass(const __grid_constant__ OnePassParams p)
 {
     using namespace op;
@@ -982,26 +1240,25 @@ __global__ void __launch_bounds__(op::NT, 1) k_mpdata_onepass(const __grid_const
     float *sm = reinterpret_cast<float *>(smem4) + ((128u - (smem_u32(smem4) & 127u)) & 127u) / sizeof(float);
     __shared__ __align__(8) uint64_t bars[2];
     const int s = blockIdx.x % p.nspecies;
-    const int tile = blockIdx.x / p.nspecies;
-    const int tx = tile % p.tiles_x, j0 = (tile / p.tiles_x) * TY;
+    int rest = blockIdx.x / p.nspecies;
+    const int parts = (p.g.nz + p.klen - 1) / p.klen;
+    const int ka = (rest % parts) * p.klen, kb = min(ka + p.klen, p.g.nz);
+    rest /= parts;
+    const int tx = rest % p.tiles_x, j0 = (rest / p.tiles_x) * TY;
     __shared__ int stop;
     if (threadIdx.x == 0) stop = *reinterpret_cast<volatile const int *>(p.err);
     __syncthreads();
     if (stop) return;   // an earlier tile of this launch gave up on a TMA wait: stop (the whole CTA)
-    uint32_t ph[2];
-    onepass_init_bars(bars, ph);
-    onepass_run<EXACT, FCT>(sm, bars, ph, p, s, tx, j0);
+    onepass_init_bars(bars);
+    onepass_item<M, FCT>(sm, bars, p, s, tx, j0, ka, kb);
 }
 
-// Batched form: one launch over the work list of (member, species, column
-// tile tx, first row j0) items, one CTA per item; params[member] holds that
-// member's descriptors, pointers and geometry for the current buffer
-// parity.  The hardware block scheduler hands out the items in list order
-// as SMs free up.  (A persistent form, CTAs pulling items with an atomic
-// counter, carried its barrier phases and item bookkeeping through the
-// march, spilled some 400 bytes per thread to local memory and ran the
-// 64-member ensemble 1.5x slower.)
-template <bool EXACT, bool FCT>
+// Batched form: one launch over the work list of (member, species and level
+// part, column tile tx, first row j0) items, one CTA per item; params[member]
+// holds that member's descriptors, pointers and geometry for the current
+// buffer parity.  The hardware block scheduler hands out the items in list
+// order as SMs free up.
+template <int M, bool FCT>
 __global__ void __launch_bounds__(op::NT, 1)
     k_batch_onepass_items(const OnePassParams *__restrict__ params, const int4 *__restrict__ items)
 {
@@ -1018,9 +1275,9 @@ __global__ void __launch_bounds__(op::NT, 1)
     if (threadIdx.x == 0) stop = *reinterpret_cast<volatile const int *>(params[0].err);
     __syncthreads();
     if (stop) return;
-    uint32_t ph[2];
-    onepass_init_bars(bars, ph);
-    onepass_run<EXACT, FCT>(sm, bars, ph, sp, w.y, w.z, w.w);
+    onepass_init_bars(bars);
+    const int ka = (w.y / op::MAXS) * sp.klen, kb = min(ka + sp.klen, sp.g.nz);
+    onepass_item<M, FCT>(sm, bars, sp, w.y % op::MAXS, w.z, w.w, ka, kb);
 }
 
 }  // namespace icar

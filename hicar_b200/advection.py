@@ -311,9 +311,9 @@ class Domain:
         return int(b.value)
 
     def set_launch_shape(self, tile_shape: int | None = None, species_group: int | None = None) -> None:
-        """Tile shape of the fused correction kernel (0..3 = 8/15/24/31 rows
-        per tile) and species per thread of its donor-cell pass (0 = all);
-        see hicar_b200.autotune.  Results do not depend on either."""
+        """Launch-shape knobs of earlier kernels: checked and accepted, but the
+        single-pass kernel chooses its own launch.  Results never depended on
+        either."""
         lib = L.load()
         if tile_shape is not None:
             L.check(lib.icar_adv_set_tile_shape(self.handle, int(tile_shape)), self.handle)
@@ -326,7 +326,8 @@ class Domain:
     def use_single_pass(self, fast: bool = False) -> None:
         """MPDATA order 2 through the single-pass kernel (donor-cell pass,
         pseudo-velocities, limiter and corrective pass in one launch): bit-exact
-        arithmetic, or fast=True for the fast-arithmetic variant."""
+        arithmetic (also the default), or fast=True for the fast-arithmetic
+        variant."""
         L.check(L.load().icar_adv_set_path(self.handle, 3 if fast else 2), self.handle)
 
     def set_path(self, path: int) -> None:

@@ -8,7 +8,7 @@
     b.sync(); d.fetch("qv")
 
 The members keep their own device fields (the C-ABI handles); the batch owns
-the member tables, the (member, species, tile) work list and the two CUDA
+the member tables, the (member, species, tile, levels) work list and the two CUDA
 graphs (one per buffer parity).  See icar_adv_batch_* in include/icar_adv.h.
 """
 from __future__ import annotations
@@ -52,8 +52,7 @@ class Batch:
         self._check(self._lib.icar_adv_batch_set_tile_shape(self._b, int(shape)), self._b)
 
     def set_path(self, path: int) -> None:
-        """0: donor-cell kernel + fused correction (default); 2: single-pass
-        kernel, bit-exact; 3: single-pass kernel, fast arithmetic."""
+        """0 (default) or 2: bit-exact arithmetic; 3: fast arithmetic."""
         self._check(self._lib.icar_adv_batch_set_path(self._b, int(path)), self._b)
 
     def set_species_group(self, group: int) -> None:

@@ -73,7 +73,7 @@ struct icar_adv_domain {
     // per-step Courant fluxes and staged-path scratch
     DevBuf Um, Vm, Wm;
     DevBuf q1, u2, v2, w2, u2l, v2l, w2l;      // MPDATA staged scratch
-    DevBuf Gc, DJR, Wp;                        // fused path: J*rho, dz*J*rho, W_m/dz
+    DevBuf Gc, DJR, Wp;                        // per-step fields: J*rho, dz*J*rho, W_m/dz
     DevBuf dtbuf;                              // compute_dt: 4 maxima then dz_levels (nz)
     // simple microphysics: its extra resident fields, the real64 rain and
     // snow accumulations (nx*ny each) and the device stop flag
@@ -84,13 +84,12 @@ struct icar_adv_domain {
     double *acc_precip = nullptr;             // rain [0, nx*ny), snow [nx*ny, 2*nx*ny)
     int *mp_stop = nullptr;
     bool mp_ran = false;
-    std::vector<DevBuf> qn, q1s;               // fused path: next state and pass-1 result per species
-    bool fused_ready = false;
+    std::vector<DevBuf> qn, q1s;               // next state per species; the standard scheme's stage result
     bool std_ready = false;      // fused standard-scheme buffers and kernel attributes
     bool std_staged_ready = false;
     DevBuf fx, fy, fz, ufx, ufy, ufz, dq, sin_, sout, temp;  // STD scratch
-    // 0 = fused kernels (MPDATA order 2, every standard-scheme setting), 1 = staged kernels,
-    // 2 = single-pass MPDATA kernel (exact), 3 = single-pass MPDATA kernel (fast arithmetic)
+    // 0 and 2 = fused kernels (the single-pass MPDATA kernel for order 2, every standard-scheme setting),
+    // 1 = staged kernels, 3 = the single-pass MPDATA kernel in fast arithmetic
     int path = 0;
     // single-pass kernel: TMA descriptors by device address (host cache),
     // two device tables of descriptors (the species buffers alternate between
@@ -104,8 +103,6 @@ struct icar_adv_domain {
     int op_epoch = 0;
     bool op_ready = false;
     int nsm = 148;     // SMs of the device
-    int mp_shape = 1;  // tile shape of the fused correction kernel (icar::mp_shape_ty)
-    int sp_group = 0;  // species per thread of the fused upwind pass (0 = all)
     // diagnostics: launch counter and optional event timing of the species kernels
     int64_t launches = 0;
     int64_t timed_launches = 0;
@@ -209,7 +206,7 @@ int64_t footprint_bytes(const icar_adv_desc &d, const icar_adv_opts &o)
     total += f * (int64_t)nc * (d.n_species + 1);                      // species + spare
     total += f * (int64_t)(nu + nv + nc);                              // Um Vm Wm
     if (o.advection == ICAR_ADV_MPDATA && !o.rk3 && icar::fused_eligible(o.mpdata_order, o.mpdata_fct))
-        total += f * (int64_t)nc * (2 * d.n_species + 3);              // fused: next + pass-1 per species, G, DJR, W'
+        total += f * (int64_t)nc * (d.n_species + 3);                  // single pass: next state per species, G, DJR, W'
     else if (o.advection == ICAR_ADV_MPDATA)
         total += f * (int64_t)(nc + 2 * (nu + nv + nc));               // staged scratch
     else
@@ -685,26 +682,6 @@ int std_advect3d(icar_adv_t *h, const float *qf, const float *qold, float *qout,
     return check_launch(h, "std kernels", flux_corr == 1 ? 8 : 2);
 }
 
-// Fused MPDATA (order 2): prep -> pass 1 for all species -> fused
-// pseudo-velocity/FCT/corrective pass for all species, then swap buffers.
-int ensure_fused(icar_adv_t *h)
-{
-    const int S = h->desc.n_species;
-    int e;
-    if (!h->fused_ready) {
-        h->qn.resize(S);
-        h->q1s.resize(S);
-        if ((e = alloc(h, h->Gc, h->n_cell)) || (e = alloc(h, h->DJR, h->n_cell)) || (e = alloc(h, h->Wp, h->n_cell)))
-            return e;
-        for (int s = 0; s < S; s++)
-            if ((e = alloc(h, h->qn[s], h->n_cell)) || (e = alloc(h, h->q1s[s], h->n_cell))) return e;
-        cudaError_t ce = icar::mp_corr_setup();
-        if (ce != cudaSuccess) return fail(h, ICAR_ADV_CUDA_ERROR, "cudaFuncSetAttribute: %s", cudaGetErrorString(ce));
-        h->fused_ready = true;
-    }
-    return ICAR_ADV_OK;
-}
-
 // ---------------------------------------------------------------------------
 // Single-pass MPDATA kernel (mpdata_onepass.cuh): per-step fields from
 // k_mp_prep, then one launch for every species.  It needs no pass-1
@@ -882,7 +859,7 @@ int mpdata_onepass_group(icar_adv_t *h, int s0, int s1)
 int mpdata_prep(icar_adv_t *h, float dt)
 {
     const Geo &g = h->g;
-    int e = h->path >= 2 ? ensure_onepass(h) : ensure_fused(h);
+    int e = ensure_onepass(h);
     if (e) return e;
     const size_t nf = (size_t)(g.nx + 1) * g.nz * (g.ny + 1);
     icar::k_mp_prep<<<blocks_for(nf, 256), 256, 0, h->stream>>>(
@@ -895,44 +872,12 @@ int mpdata_prep(icar_adv_t *h, float dt)
     return check_launch(h, "fused MPDATA prep", 1);
 }
 
-// Donor-cell pass and fused correction for species [s0, s1); results in qn.
-int mpdata_group(icar_adv_t *h, int s0, int s1)
-{
-    const Geo &g = h->g;
-    const int S = s1 - s0;
-    if (S <= 0) return ICAR_ADV_OK;
-    icar::SpeciesPtrs sp{};
-    for (int s = 0; s < S; s++) {
-        sp.q0[s] = h->q[s0 + s].p;
-        sp.q1[s] = h->q1s[s0 + s].p;
-        sp.out[s] = h->qn[s0 + s].p;
-    }
-    const int sg = std::min(icar::upwind_group(S, h->sp_group), icar::upf::SGMAX);
-    const dim3 gu((unsigned)((g.nx + icar::upf::BX - 1) / icar::upf::BX),
-                  (unsigned)((g.ny + icar::upf::BY - 1) / icar::upf::BY), (unsigned)((S + sg - 1) / sg));
-    icar::k_mp_upwind_cols<<<gu, icar::upf::NT, icar::upf::SMEM, h->stream>>>(g, sp, S, sg, h->Um.p, h->Vm.p, h->Wm.p,
-                                                                            h->Gc.p, h->DJR.p);
-    cudaEvent_t c0 = nullptr, c1 = nullptr;
-    if (h->profiling) {
-        cudaEventCreate(&c0);
-        cudaEventCreate(&c1);
-        cudaEventRecord(c0, h->stream);
-    }
-    icar::mp_corr_launch(h->stream, h->mp_shape, g, sp, S, h->opts.mpdata_fct, h->Um.p, h->Vm.p, h->Wp.p, h->Gc.p,
-                         h->DJR.p, h->dz.p);
-    if (h->profiling) {
-        cudaEventRecord(c1, h->stream);
-        h->corr_events.emplace_back(c0, c1);
-    }
-    return check_launch(h, "fused MPDATA kernels", 2);
-}
-
 int mpdata_fused_step(icar_adv_t *h, float dt)
 {
     const int S = h->desc.n_species;
     int e = mpdata_prep(h, dt);
     if (e) return e;
-    if ((e = h->path >= 2 ? mpdata_onepass_group(h, 0, S) : mpdata_group(h, 0, S))) return e;
+    if ((e = mpdata_onepass_group(h, 0, S))) return e;
     for (int s = 0; s < S; s++) std::swap(h->q[s], h->qn[s]);
     return ICAR_ADV_OK;
 }
@@ -1038,7 +983,7 @@ int advect_impl(icar_adv_t *h, float dt)
     if (!(dt >= 0.0f) || !std::isfinite(dt)) return fail(h, ICAR_ADV_BAD_ARG, "dt must be finite and >= 0");
     const bool mp = h->opts.advection == ICAR_ADV_MPDATA;
     const bool fused_mp = mp && !h->opts.rk3 && icar::fused_eligible(h->opts.mpdata_order, h->opts.mpdata_fct);
-    if ((h->path == 0 && (fused_mp || !mp)) || (h->path >= 2 && (fused_mp || !mp))) {
+    if (h->path != 1 && (fused_mp || !mp)) {
         cudaEvent_t ev0 = nullptr, ev1 = nullptr;
         int64_t before = h->launches;
         if (h->profiling) {
@@ -1193,7 +1138,7 @@ int icar_adv_create(const icar_adv_desc *desc, const icar_adv_opts *opts, icar_a
         return bail(e);
     for (int s = 0; s < S; s++)
         if ((e = alloc(h, h->q[s], nc))) return bail(e);
-    // the scratch of either scheme is allocated on first use (ensure_fused,
+    // the scratch of either scheme is allocated on first use (ensure_onepass,
     // ensure_std_fused, mpdata_staged, std_advect3d)
     relax_filter(desc->nx, desc->ny, h->hs, desc->north_boundary, desc->south_boundary, desc->east_boundary,
                  desc->west_boundary, h->filter_host);
@@ -1611,9 +1556,7 @@ int icar_adv_step_host(icar_adv_t *h, double dt_seconds, int32_t enforce_limits,
             CUDA_TRY(h, cudaEventRecord(ev_in, h->io_in));
             CUDA_TRY(h, cudaStreamWaitEvent(h->stream, ev_in, 0));
             if ((e = forcing_range(h, dt_seconds, s0, s1))) return e;
-            if ((e = mp ? (h->path >= 2 ? mpdata_onepass_group(h, s0, s1) : mpdata_group(h, s0, s1))
-                    : std_group(h, s0, s1)))
-            return e;
+            if ((e = mp ? mpdata_onepass_group(h, s0, s1) : std_group(h, s0, s1))) return e;
             if (enforce_limits) {
                 for (int s = s0; s < s1; s++)
                     icar::k_enforce_limits<<<blocks_for(h->n_cell, 256), 256, 0, h->stream>>>(h->g, result(s).p);
@@ -1800,7 +1743,6 @@ int icar_adv_set_tile_shape(icar_adv_t *h, int32_t shape)
 {
     if (!h) return fail(nullptr, ICAR_ADV_BAD_ARG, "handle is NULL");
     if (shape < 0 || shape >= icar::MP_NSHAPES) return fail(h, ICAR_ADV_BAD_ARG, "tile shape %d out of range", shape);
-    h->mp_shape = shape;
     return ICAR_ADV_OK;
 }
 
@@ -1808,7 +1750,6 @@ int icar_adv_set_species_group(icar_adv_t *h, int32_t group)
 {
     if (!h) return fail(nullptr, ICAR_ADV_BAD_ARG, "handle is NULL");
     if (group < 0 || group > ICAR_ADV_MAX_SPECIES) return fail(h, ICAR_ADV_BAD_ARG, "species group %d out of range", group);
-    h->sp_group = group;
     return ICAR_ADV_OK;
 }
 
@@ -1841,23 +1782,20 @@ struct icar_adv_batch {
     int nsm = 0;
     std::vector<icar_adv_t *> members;
     std::vector<double> dts;
-    int shape = 1;
-    int sp_group = 0;  // species per thread of the upwind pass (0 = all)
     int fct = -1;
     bool tables_dirty = true, graph_dirty = true;
     int parity = 0;
     // device tables and work lists
     icar::BatchMember *d_mem[2] = {nullptr, nullptr};
     size_t mem_cap = 0;
-    int *d_ints = nullptr;   // prep prefix | upwind prefix | forcing prefix | counter
+    int *d_ints = nullptr;   // prep prefix | forcing prefix
     size_t ints_cap = 0;
     int2 *d_pairs = nullptr;
     size_t pairs_cap = 0;
     int4 *d_items = nullptr;
     size_t items_cap = 0;
-    int n_prep = 0, n_up = 0, n_force = 0, n_pairs = 0, n_items = 0, ctas = 0;
-    // single-pass kernel (path 2 exact, 3 fast; 0 = the two-pass kernels):
-    // per-member kernel parameters for both buffer parities, their TMA
+    int n_prep = 0, n_force = 0, n_pairs = 0, n_items = 0;
+    // arithmetic of the single-pass kernel (3: fast, otherwise exact): per-member kernel parameters for both buffer parities, their TMA
     // descriptor tables, and one timeout flag for the whole batch
     int path = 0;
     icar::OnePassParams *d_opp[2] = {nullptr, nullptr};
@@ -1865,7 +1803,7 @@ struct icar_adv_batch {
     CUtensorMap *d_bmaps = nullptr;
     size_t bmaps_cap = 0;
     int *d_operr = nullptr;
-    size_t off_up = 0, off_f = 0, off_counter = 0;
+    size_t off_f = 0;
     cudaGraph_t graph[2] = {nullptr, nullptr};
     cudaGraphExec_t exec[2] = {nullptr, nullptr};
     int stable_steps = 0;  // steps since the last table rebuild; graphs are captured once it reaches 2
@@ -1952,7 +1890,6 @@ void fill_member(icar::BatchMember &m, icar_adv_t *h, double dt, int parity)
         float *nxt = parity == 0 ? h->qn[s].p : h->q[s].p;
         m.q0[s] = cur;
         m.out[s] = nxt;
-        m.q1[s] = s < (int)h->q1s.size() ? h->q1s[s].p : nullptr;
         m.forcing[s] = h->forcing[s].p;
         m.dqdt[s] = h->dqdt[s].p;
     }
@@ -1965,51 +1902,42 @@ int build_tables(icar_adv_batch_t *b)
     std::vector<icar::BatchMember> mem[2];
     mem[0].resize(std::max(M, 1));
     mem[1].resize(std::max(M, 1));
-    std::vector<int> prep(M + 1, 0), up(M + 1, 0), fpre(1, 0);
+    std::vector<int> prep(M + 1, 0), fpre(1, 0);
     std::vector<int2> pairs;
     std::vector<int4> items;
-    const int ty = icar::mp_shape_ty(b->shape);
-    const bool onepass = b->path >= 2;
     std::vector<icar::OnePassParams> opp[2];
     std::vector<CUtensorMap> maps;
     std::vector<size_t> map_base[2];
     std::vector<int> klen(M, 0);   // levels per single-pass item of each member
-    if (onepass) {
-        long tiles = 0;
-        for (icar_adv_t *h : b->members)
-            tiles += (long)onepass_tiles_x(h->g) * onepass_tiles_y(h->g) * h->desc.n_species;
-        for (int m = 0; m < M; m++) klen[m] = icar::op::levels_per_cta(tiles, b->members[m]->g.nz, b->nsm);
-        opp[0].resize(std::max(M, 1));
-        opp[1].resize(std::max(M, 1));
-        map_base[0].resize(M);
-        map_base[1].resize(M);
-        if (!b->d_operr) {
-            BCUDA(b, cudaMalloc(&b->d_operr, sizeof(int)));
-            BCUDA(b, cudaMemsetAsync(b->d_operr, 0, sizeof(int), b->stream));
-        }
+    long tiles = 0;
+    for (icar_adv_t *h : b->members)
+        tiles += (long)onepass_tiles_x(h->g) * onepass_tiles_y(h->g) * h->desc.n_species;
+    for (int m = 0; m < M; m++) klen[m] = icar::op::levels_per_cta(tiles, b->members[m]->g.nz, b->nsm);
+    opp[0].resize(std::max(M, 1));
+    opp[1].resize(std::max(M, 1));
+    map_base[0].resize(M);
+    map_base[1].resize(M);
+    if (!b->d_operr) {
+        BCUDA(b, cudaMalloc(&b->d_operr, sizeof(int)));
+        BCUDA(b, cudaMemsetAsync(b->d_operr, 0, sizeof(int), b->stream));
     }
     for (int m = 0; m < M; m++) {
         icar_adv_t *h = b->members[m];
-        if (onepass) {
-            int r = ensure_onepass(h);
-            if (r) return bfail(b, r, "member scratch: %s", h->err.c_str());
-            h->op_epoch++;   // one epoch for every step these tables serve
-            // descriptors of both parities: species inputs, then U_m, V_m, W_m/dz, J*rho
-            for (int pp = 0; pp < 2; pp++) {
-                map_base[pp][m] = maps.size();
-                const int S = h->desc.n_species;
-                for (int f = 0; f < S + 4; f++) {
-                    const float *base = f < S ? (pp == 0 ? h->q[f].p : h->qn[f].p)
-                                              : (f == S ? h->Um.p : f == S + 1 ? h->Vm.p : f == S + 2 ? h->Wp.p : h->Gc.p);
-                    const CUtensorMap *mp;
-                    if ((r = plane_map(h, base, f == S + 1 ? h->g.ny + 1 : h->g.ny, &mp)))
-                        return bfail(b, r, "%s", h->err.c_str());
-                    maps.push_back(*mp);
-                }
+        int r = ensure_onepass(h);
+        if (r) return bfail(b, r, "member scratch: %s", h->err.c_str());
+        h->op_epoch++;   // one epoch for every step these tables serve
+        // descriptors of both parities: species inputs, then U_m, V_m, W_m/dz, J*rho
+        for (int pp = 0; pp < 2; pp++) {
+            map_base[pp][m] = maps.size();
+            const int S = h->desc.n_species;
+            for (int f = 0; f < S + 4; f++) {
+                const float *base = f < S ? (pp == 0 ? h->q[f].p : h->qn[f].p)
+                                          : (f == S ? h->Um.p : f == S + 1 ? h->Vm.p : f == S + 2 ? h->Wp.p : h->Gc.p);
+                const CUtensorMap *mp;
+                if ((r = plane_map(h, base, f == S + 1 ? h->g.ny + 1 : h->g.ny, &mp)))
+                    return bfail(b, r, "%s", h->err.c_str());
+                maps.push_back(*mp);
             }
-        } else {
-            int r = ensure_fused(h);
-            if (r) return bfail(b, r, "member scratch: %s", h->err.c_str());
         }
         // members' buffers hold "current" in q at the batch's parity 0
         fill_member(mem[0][m], h, b->dts[m], b->parity == 0 ? 0 : 1);
@@ -2017,29 +1945,20 @@ int build_tables(icar_adv_batch_t *b)
         const Geo &g = h->g;
         const size_t nf = (size_t)(g.nx + 1) * g.nz * (g.ny + 1);
         prep[m + 1] = prep[m] + (int)((nf + 255) / 256);
-        up[m + 1] = up[m] + icar::upwind_cols_blocks(h->g, h->desc.n_species, b->sp_group);
         for (int s = 0; s < h->desc.n_species; s++) {
             if (h->forcing[s].p && h->nzone > 0) {
                 pairs.push_back(make_int2(m, s));
                 fpre.push_back(fpre.back() + (int)(((size_t)h->nzone * g.nz + 255) / 256));
             }
         }
-        if (onepass) {
-            const int tx = onepass_tiles_x(g), tyn = onepass_tiles_y(g), parts = (g.nz + klen[m] - 1) / klen[m];
-            for (int s = 0; s < h->desc.n_species; s++)
-                for (int a = 0; a < tyn; a++)
-                    for (int c = 0; c < tx; c++)
-                        for (int k = 0; k < parts; k++)
-                            items.push_back(make_int4(m, s + icar::op::MAXS * k, c, a * icar::op::TY));
-        } else {
-            const int tx = icar::mp_tiles_x(g), tyn = icar::mp_tiles_y(g, ty);
-            for (int s = 0; s < h->desc.n_species; s++)
-                for (int a = 0; a < tyn; a++)
-                    for (int c = 0; c < tx; c++)
-                        items.push_back(make_int4(m, s, c * icar::mpf::TX - 2, 1 + a * ty));
-        }
+        const int tx = onepass_tiles_x(g), tyn = onepass_tiles_y(g), parts = (g.nz + klen[m] - 1) / klen[m];
+        for (int s = 0; s < h->desc.n_species; s++)
+            for (int a = 0; a < tyn; a++)
+                for (int c = 0; c < tx; c++)
+                    for (int k = 0; k < parts; k++)
+                        items.push_back(make_int4(m, s + icar::op::MAXS * k, c, a * icar::op::TY));
     }
-    if (onepass && !maps.empty() && (maps.size() > b->bmaps_cap || !b->d_bmaps)) {
+    if (!maps.empty() && (maps.size() > b->bmaps_cap || !b->d_bmaps)) {
         if (b->d_bmaps) cudaFree(b->d_bmaps);  // synchronises: queued launches may read it
         b->d_bmaps = nullptr;
         b->bmaps_cap = 0;
@@ -2047,47 +1966,42 @@ int build_tables(icar_adv_batch_t *b)
         BCUDA(b, cudaMalloc(&b->d_bmaps, cap * sizeof(CUtensorMap)));
         b->bmaps_cap = cap;
     }
-    if (onepass) {
-        for (int pp = 0; pp < 2; pp++)
-            for (int m = 0; m < M; m++) {
-                icar_adv_t *h = b->members[m];
-                icar::OnePassParams &q = opp[pp][m];
-                memset(&q, 0, sizeof(q));
-                const int S = h->desc.n_species;
-                q.q0maps = b->d_bmaps + map_base[pp][m];
-                q.fmaps = q.q0maps + S;
-                for (int s2 = 0; s2 < S; s2++) q.out[s2] = pp == 0 ? h->qn[s2].p : h->q[s2].p;
-                q.Wm = h->Wm.p;
-                q.DJR = h->DJR.p;
-                q.dz = h->dz.p;
-                q.err = b->d_operr;
-                q.flags = h->op_flags;
-                q.epoch = h->op_epoch;
-                q.nzero = -0.0f;
-                q.g = h->g;
-                q.nspecies = S;
-                q.tiles_x = onepass_tiles_x(h->g);
-                q.klen = klen[m];
-            }
-        if ((size_t)std::max(M, 1) > b->opp_cap || !b->d_opp[0]) {
-            for (int pp = 0; pp < 2; pp++) {
-                if (b->d_opp[pp]) cudaFree(b->d_opp[pp]);
-                b->d_opp[pp] = nullptr;
-            }
-            b->opp_cap = 0;
-            const size_t cap = std::max<size_t>(M, 16);
-            for (int pp = 0; pp < 2; pp++) BCUDA(b, cudaMalloc(&b->d_opp[pp], cap * sizeof(icar::OnePassParams)));
-            b->opp_cap = cap;
+    for (int pp = 0; pp < 2; pp++)
+        for (int m = 0; m < M; m++) {
+            icar_adv_t *h = b->members[m];
+            icar::OnePassParams &q = opp[pp][m];
+            memset(&q, 0, sizeof(q));
+            const int S = h->desc.n_species;
+            q.q0maps = b->d_bmaps + map_base[pp][m];
+            q.fmaps = q.q0maps + S;
+            for (int s2 = 0; s2 < S; s2++) q.out[s2] = pp == 0 ? h->qn[s2].p : h->q[s2].p;
+            q.Wm = h->Wm.p;
+            q.DJR = h->DJR.p;
+            q.dz = h->dz.p;
+            q.err = b->d_operr;
+            q.flags = h->op_flags;
+            q.epoch = h->op_epoch;
+            q.nzero = -0.0f;
+            q.g = h->g;
+            q.nspecies = S;
+            q.tiles_x = onepass_tiles_x(h->g);
+            q.klen = klen[m];
         }
+    if ((size_t)std::max(M, 1) > b->opp_cap || !b->d_opp[0]) {
+        for (int pp = 0; pp < 2; pp++) {
+            if (b->d_opp[pp]) cudaFree(b->d_opp[pp]);
+            b->d_opp[pp] = nullptr;
+        }
+        b->opp_cap = 0;
+        const size_t cap = std::max<size_t>(M, 16);
+        for (int pp = 0; pp < 2; pp++) BCUDA(b, cudaMalloc(&b->d_opp[pp], cap * sizeof(icar::OnePassParams)));
+        b->opp_cap = cap;
     }
     // longest columns first (cost ~ levels per item), so the tail of the
     // launch is made of short items
-    std::stable_sort(items.begin(), items.end(), [&](const int4 &x, const int4 &y) {
-        if (onepass) return klen[x.x] > klen[y.x];
-        return b->members[x.x]->g.nz > b->members[y.x]->g.nz;
-    });
+    std::stable_sort(items.begin(), items.end(),
+                     [&](const int4 &x, const int4 &y) { return klen[x.x] > klen[y.x]; });
     b->n_prep = prep[M];
-    b->n_up = up[M];
     b->n_pairs = (int)pairs.size();
     b->n_force = fpre.back();
     b->n_items = (int)items.size();
@@ -2102,12 +2016,9 @@ int build_tables(icar_adv_batch_t *b)
         for (int p = 0; p < 2; p++) BCUDA(b, cudaMalloc(&b->d_mem[p], cap * sizeof(icar::BatchMember)));
         b->mem_cap = cap;
     }
-    b->off_up = M + 1;
-    b->off_f = b->off_up + M + 1;
-    b->off_counter = b->off_f + fpre.size();
-    std::vector<int> ints(b->off_counter + 1, 0);
+    b->off_f = M + 1;
+    std::vector<int> ints(b->off_f + fpre.size(), 0);
     std::copy(prep.begin(), prep.end(), ints.begin());
-    std::copy(up.begin(), up.end(), ints.begin() + b->off_up);
     std::copy(fpre.begin(), fpre.end(), ints.begin() + b->off_f);
     if ((e = grow(b, b->d_ints, b->ints_cap, ints.size()))) return e;
     if ((e = grow(b, b->d_pairs, b->pairs_cap, std::max<size_t>(pairs.size(), 1)))) return e;
@@ -2117,7 +2028,7 @@ int build_tables(icar_adv_batch_t *b)
     // staging sets alternate; a set is reused only after its previous upload
     // has been consumed.
     const size_t bm = sizeof(icar::BatchMember) * std::max(M, 1);
-    const size_t po = onepass ? sizeof(icar::OnePassParams) * std::max(M, 1) : 0;
+    const size_t po = sizeof(icar::OnePassParams) * std::max(M, 1);
     const size_t seg[8] = {bm, bm, sizeof(int) * ints.size(), sizeof(int2) * pairs.size(),
                            sizeof(int4) * items.size(), po, po, sizeof(CUtensorMap) * maps.size()};
     size_t off[8], total = 0;
@@ -2154,10 +2065,6 @@ int build_tables(icar_adv_batch_t *b)
     if (seg[7]) BCUDA(b, cudaMemcpyAsync(b->d_bmaps, st + off[7], seg[7], cudaMemcpyHostToDevice, b->stream));
     BCUDA(b, cudaEventRecord(b->stage_done[t], b->stream));
     b->stage_turn ^= 1;
-    // the single-pass launch has one CTA per item; the two-pass correction
-    // kernel is persistent
-    b->ctas = onepass ? b->n_items
-                      : std::min(std::max(b->n_items, 1), icar::batch_corr_max_ctas(b->shape, b->fct, b->nsm));
     b->tables_dirty = false;
     return ICAR_ADV_OK;
 }
@@ -2170,26 +2077,18 @@ void enqueue_step(icar_adv_batch_t *b, int p, cudaStream_t st)
     if (b->n_force > 0)
         icar::k_batch_forcing<<<b->n_force, 256, 0, st>>>(mem, b->d_ints + b->off_f, b->d_pairs, b->n_pairs);
     if (b->n_prep > 0) icar::k_batch_prep<<<b->n_prep, 256, 0, st>>>(mem, b->d_ints, M);
-    if (b->path >= 2) {
-        if (b->n_items > 0) {
-            const icar::OnePassParams *opp = b->d_opp[p];
-            const int n = b->n_items;
-            const size_t sm = icar::op::SMEM;
-            const int4 *it = b->d_items;
-            if (b->path == 2 && b->fct) icar::k_batch_onepass_items<icar::opx::A_EXACT, true><<<n, icar::op::NT, sm, st>>>(opp, it);
-            else if (b->path == 2) icar::k_batch_onepass_items<icar::opx::A_EXACT, false><<<n, icar::op::NT, sm, st>>>(opp, it);
-            else if (b->fct) icar::k_batch_onepass_items<icar::opx::A_FAST, true><<<n, icar::op::NT, sm, st>>>(opp, it);
-            else icar::k_batch_onepass_items<icar::opx::A_FAST, false><<<n, icar::op::NT, sm, st>>>(opp, it);
-        }
-        return;
+    if (b->n_items > 0) {
+        const icar::OnePassParams *opp = b->d_opp[p];
+        const int n = b->n_items;
+        const size_t sm = icar::op::SMEM;
+        const int4 *it = b->d_items;
+        using icar::opx::A_EXACT;
+        using icar::opx::A_FAST;
+        if (b->path != 3 && b->fct) icar::k_batch_onepass_items<A_EXACT, true><<<n, icar::op::NT, sm, st>>>(opp, it);
+        else if (b->path != 3) icar::k_batch_onepass_items<A_EXACT, false><<<n, icar::op::NT, sm, st>>>(opp, it);
+        else if (b->fct) icar::k_batch_onepass_items<A_FAST, true><<<n, icar::op::NT, sm, st>>>(opp, it);
+        else icar::k_batch_onepass_items<A_FAST, false><<<n, icar::op::NT, sm, st>>>(opp, it);
     }
-    if (b->n_up > 0)
-        icar::k_batch_upwind<<<b->n_up, icar::upf::NT, icar::upf::SMEM, st>>>(mem, b->d_ints + b->off_up, M,
-                                                                           b->sp_group);
-    cudaMemsetAsync(b->d_ints + b->off_counter, 0, sizeof(int), st);
-    if (b->n_items > 0)
-        icar::batch_corr_launch(st, b->shape, b->ctas, b->fct, mem, b->d_items, b->n_items,
-                                b->d_ints + b->off_counter);
 }
 
 cudaError_t batch_onepass_setup()
@@ -2236,8 +2135,6 @@ int icar_adv_batch_create(int32_t device, icar_adv_batch_t **out)
     b->device = device;
     cudaDeviceGetAttribute(&b->nsm, cudaDevAttrMultiProcessorCount, device);
     cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = icar::mp_corr_setup();
-    if (e == cudaSuccess) e = icar::batch_setup();
     if (e == cudaSuccess) e = batch_onepass_setup();
     if (e != cudaSuccess) {
         int code = bfail(nullptr, ICAR_ADV_CUDA_ERROR, "batch setup failed: %s", cudaGetErrorString(e));
@@ -2263,7 +2160,7 @@ int icar_adv_batch_add(icar_adv_batch_t *b, icar_adv_t *h, double dt_seconds)
     cudaSetDevice(b->device);
     int e = ensure_ready(h);
     if (e) return bfail(b, e, "member not ready: %s", h->err.c_str());
-    e = b->path >= 2 ? ensure_onepass(h) : ensure_fused(h);
+    e = ensure_onepass(h);
     if (e) return bfail(b, e, "member scratch: %s", h->err.c_str());
     // order the member's pending work before the batch's, then share the stream
     cudaStreamSynchronize(h->stream);
@@ -2319,10 +2216,6 @@ int icar_adv_batch_set_tile_shape(icar_adv_batch_t *b, int32_t shape)
 {
     if (!b) return bfail(nullptr, ICAR_ADV_BAD_ARG, "batch is NULL");
     if (shape < 0 || shape >= icar::MP_NSHAPES) return bfail(b, ICAR_ADV_BAD_ARG, "tile shape out of range");
-    if (shape != b->shape) {
-        b->shape = shape;
-        b->tables_dirty = b->graph_dirty = true;
-    }
     return ICAR_ADV_OK;
 }
 
@@ -2330,10 +2223,6 @@ int icar_adv_batch_set_species_group(icar_adv_batch_t *b, int32_t group)
 {
     if (!b) return bfail(nullptr, ICAR_ADV_BAD_ARG, "batch is NULL");
     if (group < 0 || group > ICAR_ADV_MAX_SPECIES) return bfail(b, ICAR_ADV_BAD_ARG, "species group out of range");
-    if (group != b->sp_group) {
-        b->sp_group = group;
-        b->tables_dirty = b->graph_dirty = true;
-    }
     return ICAR_ADV_OK;
 }
 
@@ -2463,7 +2352,7 @@ int icar_adv_batch_profile_read(icar_adv_batch_t *b, double *step_ms, int64_t *s
     if (step_ms) *step_ms = ms;
     if (steps) *steps = (int64_t)b->events.size();
     if (kernels_per_step)
-        *kernels_per_step = (b->n_force > 0) + (b->n_prep > 0) + (b->n_up > 0) + (b->n_items > 0);
+        *kernels_per_step = (b->n_force > 0) + (b->n_prep > 0) + (b->n_items > 0);
     if (cell_species_per_step) {
         int64_t cs = 0;
         for (icar_adv_t *h : b->members) cs += (int64_t)h->g.nx * h->g.ny * h->g.nz * h->desc.n_species;
@@ -2638,7 +2527,7 @@ extern "C" int icar_adv_advect_noalloc(const icar_adv_noalloc_args *a)
         sp.q1[0] = q1;
         sp.out[0] = a->q_out[s];
         icar::k_mp_upwind_cols<<<gu, icar::upf::NT, icar::upf::SMEM, st>>>(g, sp, 1, 1, Um, Vm, Wm, Gc, DJR);
-        icar::mp_corr_launch(st, 1, g, sp, 1, a->mpdata_fct ? 1 : 0, Um, Vm, Wp, Gc, DJR, a->advection_dz);
+        icar::mp_corr_launch(st, g, sp, 1, a->mpdata_fct ? 1 : 0, Um, Vm, Wp, Gc, DJR, a->advection_dz);
     }
     ce = cudaGetLastError();
     if (ce != cudaSuccess) return fail(nullptr, ICAR_ADV_CUDA_ERROR, "launch failed: %s", cudaGetErrorString(ce));

@@ -1,5 +1,6 @@
-// Fused MPDATA step for the configuration ICAR runs (mpdata_order 2, with or
-// without the FCT limiter).  Two kernels per step:
+// Two-pass MPDATA step (mpdata_order 2, with or without the FCT limiter) for
+// callers that own all device memory (icar_adv_advect_noalloc), and the
+// per-step fields every MPDATA kernel reads:
 //
 //   k_mp_prep     species-independent per-step fields: the Courant fluxes
 //                 U_m, V_m, W_m (mpdata_compute_wind) plus G = J*rho,
@@ -120,9 +121,6 @@ struct SpeciesPtrs {
     float *q1[32];
     float *out[32];
 };
-
-// Species per group of the donor-cell pass for the knob sg (0 = all species).
-__host__ __device__ inline int upwind_group(int S, int sg) { return sg <= 0 || sg > S ? S : sg; }
 
 namespace mpf {
 constexpr int TX = 28;            // output columns per tile
@@ -804,12 +802,10 @@ inline int check_courant(cudaStream_t st, const Geo &g, const float *Um, const f
 
 namespace icar {
 
-// Tile shapes of the fused correction kernel (selected per grid shape by
-// the autotuner): output rows per tile and warps per CTA.
-using MpShape8 = mpf::Shape<8, 4>;
-using MpShape16 = mpf::Shape<15, 16>;
-using MpShape24 = mpf::Shape<24, 8>;
-using MpShape32 = mpf::Shape<31, 32>;
+// Tile shape of the fused correction kernel: output rows and warps per CTA.
+// (The launch-shape knobs of the C ABI still name the rows of the shapes it
+// once had; the single-pass kernel that replaced it there has one.)
+using MpShape = mpf::Shape<15, 16>;
 constexpr int MP_NSHAPES = 4;
 inline int mp_shape_ty(int shape)
 {
@@ -817,51 +813,29 @@ inline int mp_shape_ty(int shape)
     return ty[shape < 0 || shape >= MP_NSHAPES ? 1 : shape];
 }
 
-template <class SH>
-inline cudaError_t mp_corr_attr()
-{
-    cudaError_t e = cudaFuncSetAttribute(k_mp_corr<true, SH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)mpf::smem_bytes<SH>());
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_mp_corr<false, SH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)mpf::smem_bytes<SH>());
-    return e;
-}
-
-// Allow every instantiation its dynamic shared memory (once per device).
+// Allow the kernels their dynamic shared memory (once per device).
 inline cudaError_t mp_corr_setup()
 {
     cudaError_t e = cudaFuncSetAttribute(k_mp_upwind_cols, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)upf::SMEM);
-    if (e == cudaSuccess) e = mp_corr_attr<MpShape8>();
-    if (e == cudaSuccess) e = mp_corr_attr<MpShape16>();
-    if (e == cudaSuccess) e = mp_corr_attr<MpShape24>();
-    if (e == cudaSuccess) e = mp_corr_attr<MpShape32>();
+    const int sm = (int)mpf::smem_bytes<MpShape>();
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_mp_corr<true, MpShape>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_mp_corr<false, MpShape>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     return e;
 }
 
-template <class SH>
-inline void mp_corr_launch_t(cudaStream_t st, const Geo &g, const SpeciesPtrs &sp, int S, int fct, const float *Um,
-                             const float *Vm, const float *Wp, const float *Gc, const float *DJR, const float *dz)
+inline void mp_corr_launch(cudaStream_t st, const Geo &g, const SpeciesPtrs &sp, int S, int fct, const float *Um,
+                           const float *Vm, const float *Wp, const float *Gc, const float *DJR, const float *dz)
 {
+    using SH = MpShape;
     const int tx = mp_tiles_x(g), ty = mp_tiles_y(g, SH::TY);
     const unsigned nblk = (unsigned)(tx * ty * S);
     if (fct)
         k_mp_corr<true, SH><<<nblk, SH::NT, mpf::smem_bytes<SH>(), st>>>(g, sp, S, tx, Um, Vm, Wp, Gc, DJR, dz);
     else
         k_mp_corr<false, SH><<<nblk, SH::NT, mpf::smem_bytes<SH>(), st>>>(g, sp, S, tx, Um, Vm, Wp, Gc, DJR, dz);
-}
-
-inline void mp_corr_launch(cudaStream_t st, int shape, const Geo &g, const SpeciesPtrs &sp, int S, int fct,
-                           const float *Um, const float *Vm, const float *Wp, const float *Gc, const float *DJR,
-                           const float *dz)
-{
-    switch (shape) {
-    case 0: mp_corr_launch_t<MpShape8>(st, g, sp, S, fct, Um, Vm, Wp, Gc, DJR, dz); break;
-    case 2: mp_corr_launch_t<MpShape24>(st, g, sp, S, fct, Um, Vm, Wp, Gc, DJR, dz); break;
-    case 3: mp_corr_launch_t<MpShape32>(st, g, sp, S, fct, Um, Vm, Wp, Gc, DJR, dz); break;
-    default: mp_corr_launch_t<MpShape16>(st, g, sp, S, fct, Um, Vm, Wp, Gc, DJR, dz); break;
-    }
 }
 
 }  // namespace icar

@@ -87,8 +87,8 @@ class InjectedFault(RuntimeError):
 
 
 class Server:
-    """path: MPDATA kernels of the batched step (0 two-pass, 2 single-pass
-    bit-exact, 3 single-pass fast; see icar_adv_set_path).  fault_hook(req,
+    """path: arithmetic of the batched step (0 or 2 bit-exact, 3 fast; see
+    icar_adv_set_path).  fault_hook(req,
     stage, steps_done), if given, is called on the host when a request is set
     up (stage "setup") and after each of its steps (stage "step"); an
     exception it raises fails that request alone: the request leaves the

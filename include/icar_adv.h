@@ -285,11 +285,9 @@ int icar_adv_profile_read_correction(icar_adv_t *h, double *ms, int64_t *launche
  * Batched form (no reference counterpart: the reference advances one domain
  * per process).  Many independent domains -- ensemble members or served
  * requests of uneven nx x ny x nz -- advance together: one step is a single
- * CUDA-graph launch holding the boundary update, the per-step wind fields,
- * the donor-cell pass and one correction kernel over a (member, species,
- * tile) work list (two-pass kernels, persistent CTAs), or one single-pass
- * launch over that work list with one CTA per item (icar_adv_batch_set_path
- * 2 or 3).  Each member keeps its own device
+ * CUDA-graph launch holding the boundary update, the per-step wind fields and
+ * one single-pass launch over a (member, species, tile, level range) work
+ * list with one CTA per item.  Each member keeps its own device
  * fields; while it is a member its work runs on the batch's stream, it
  * cannot be stepped on its own, and set/get_field stay available.  All
  * members must use MPDATA order 2 without RK3 and share MPDATA_FCT.
@@ -308,12 +306,10 @@ int icar_adv_batch_sync(icar_adv_batch_t *b);
 /* Bounded wait for the batch's steps; ICAR_ADV_TIMEOUT after timeout_s. */
 int icar_adv_batch_sync_timeout(icar_adv_batch_t *b, double timeout_s);
 int icar_adv_batch_set_stream(icar_adv_batch_t *b, void *cuda_stream);
-/* MPDATA kernels of the batch's step (no reference counterpart): 0 = the
- * donor-cell kernel then the fused correction (default), 2 = the single-pass
- * kernel with the reference's FP32 arithmetic (bit-identical results), 3 =
- * the single-pass kernel with fast arithmetic (hardware reciprocal
- * approximation and fused multiply-adds; results within the tolerance
- * stated with icar_adv_set_path). */
+/* Arithmetic of the batch's step (no reference counterpart): 0 or 2 = the
+ * reference's FP32 arithmetic (default; bit-identical results), 3 = fast
+ * arithmetic (hardware reciprocal approximation and fused multiply-adds;
+ * results within the tolerance stated with icar_adv_set_path). */
 int icar_adv_batch_set_path(icar_adv_batch_t *b, int32_t path);
 /* Event timing of every step launched while enabled; reading synchronises. */
 int icar_adv_batch_profile(icar_adv_batch_t *b, int32_t enable);
@@ -374,24 +370,22 @@ typedef struct {
 
 int icar_adv_advect_noalloc(const icar_adv_noalloc_args *args);
 
-/* Launch shape of the fused MPDATA kernels (no reference counterpart; chosen
- * per grid shape by the autotuner, hicar_b200/autotune.py).  The tile shape
- * selects the output rows per tile of the correction kernel;
- * icar_adv_tile_shapes reports how many shapes exist and the rows of each
- * (rows may be NULL).  The species group is the number of species one thread
- * of the donor-cell pass takes (0 = all, the default; 1..32).  Neither
- * changes any result. */
+/* Launch shape (no reference counterpart).  The single-pass kernel that runs
+ * the handle and batched MPDATA steps has one tile shape and chooses its level
+ * ranges itself, so these are accepted and checked but choose nothing; they
+ * never changed a result.  icar_adv_tile_shapes reports how many shapes may be
+ * named and the rows each stood for (rows may be NULL). */
 int icar_adv_set_tile_shape(icar_adv_t *h, int32_t shape);
 int icar_adv_set_species_group(icar_adv_t *h, int32_t group);
 int icar_adv_tile_shapes(int32_t *n_shapes, int32_t *rows);
 
 /* Kernel selection (no reference counterpart).  MPDATA order 2 without
  * RK3 runs as:
- *   0  the donor-cell kernel then the fused correction kernel (default;
- *      the reference's FP32 arithmetic, bit-identical results);
+ *   0  the single-pass kernel (donor-cell pass, pseudo-velocities, limiter
+ *      and corrective pass in one launch for every species) with the
+ *      reference's FP32 arithmetic (default; bit-identical results);
  *   1  one kernel per reference stage (any mpdata_order; bit-identical);
- *   2  the single-pass kernel (donor-cell pass, pseudo-velocities, limiter
- *      and corrective pass in one launch for every species; bit-identical);
+ *   2  the same as 0;
  *   3  the single-pass kernel with fast arithmetic: hardware reciprocal
  *      approximation, fused multiply-adds and reassociated pair sums.  Not
  *      bit-identical; tolerance as tested: max relative error (floor

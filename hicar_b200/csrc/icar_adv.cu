@@ -23,6 +23,7 @@
 #include "../../include/icar_adv.h"
 #include "boundary_kernels.cuh"
 #include "common.cuh"
+#include "field_copy.cuh"
 #include "mpdata_fused.cuh"
 #include "mpdata_kernels.cuh"
 #include "std_kernels.cuh"
@@ -701,6 +702,36 @@ PFN_cuTensorMapEncodeTiled_v12000 tma_encoder()
     return fn;
 }
 
+// Whether [p, p + bytes) is ordinary memory of one allocation on device dev
+// that a kernel there may touch.  A copy call checks the pointer it is given
+// and takes host, managed and other devices' memory too; a kernel does
+// neither, so what does not pass here stays with the copy call.
+bool plain_device_range(const void *p, size_t bytes, int dev)
+{
+    static PFN_cuPointerGetAttributes_v7000 fn = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &f, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            fn = reinterpret_cast<PFN_cuPointerGetAttributes_v7000>(f);
+    });
+    if (!fn || (uintptr_t)p % 4 != 0) return false;
+    unsigned type = 0, managed = 1, flags = 0;
+    int ordinal = -1;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    CUpointer_attribute at[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE,      CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,   CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                CU_POINTER_ATTRIBUTE_RANGE_SIZE,       CU_POINTER_ATTRIBUTE_ACCESS_FLAGS};
+    void *out[] = {&type, &managed, &ordinal, &start, &size, &flags};
+    if (fn(6, at, out, (CUdeviceptr)p) != CUDA_SUCCESS) return false;
+    return type == CU_MEMORYTYPE_DEVICE && !managed && ordinal == dev &&
+           flags == CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE && (CUdeviceptr)p >= start &&
+           bytes <= size && (CUdeviceptr)p - start <= size - bytes;
+}
+
 // Descriptor of one pitched 3-D field (rows = ny or ny+1) for 64 x 1 x 28
 // plane boxes; cached per device address.
 int plane_map(icar_adv_t *h, const float *base, int rows, const CUtensorMap **out)
@@ -1272,15 +1303,19 @@ static int device_copy(icar_adv_t *h, int32_t field, float *dev, bool to_handle)
     int e = resolve(h, field, r);
     if (e) return e;
     if (r.is_filter) return fail(h, ICAR_ADV_BAD_ARG, "the relaxation filter is set from host memory");
-    const size_t P = (size_t)h->g.P;
-    cudaError_t ce;
-    if (to_handle)
-        ce = cudaMemcpy2DAsync(r.buf->p, P * 4, dev, (size_t)r.ex * 4, (size_t)r.ex * 4, (size_t)r.ez * r.ey,
-                               cudaMemcpyDeviceToDevice, h->stream);
-    else
-        ce = cudaMemcpy2DAsync(dev, (size_t)r.ex * 4, r.buf->p, P * 4, (size_t)r.ex * 4, (size_t)r.ez * r.ey,
-                               cudaMemcpyDeviceToDevice, h->stream);
-    if (ce != cudaSuccess) return fail(h, ICAR_ADV_CUDA_ERROR, "cudaMemcpy2DAsync: %s", cudaGetErrorString(ce));
+    const size_t P = (size_t)h->g.P, ex = (size_t)r.ex, rows = (size_t)r.ez * r.ey;
+    if (plain_device_range(dev, ex * rows * 4, h->desc.device)) {
+        if (to_handle)
+            icar::repack(dev, ex, r.buf->p, P, ex, rows, h->stream);
+        else
+            icar::repack(r.buf->p, P, dev, ex, ex, rows, h->stream);
+        if ((e = check_launch(h, "field copy"))) return e;
+    } else {
+        const cudaError_t ce =
+            to_handle ? cudaMemcpy2DAsync(r.buf->p, P * 4, dev, ex * 4, ex * 4, rows, cudaMemcpyDeviceToDevice, h->stream)
+                      : cudaMemcpy2DAsync(dev, ex * 4, r.buf->p, P * 4, ex * 4, rows, cudaMemcpyDeviceToDevice, h->stream);
+        if (ce != cudaSuccess) return fail(h, ICAR_ADV_CUDA_ERROR, "cudaMemcpy2DAsync: %s", cudaGetErrorString(ce));
+    }
     if (to_handle) {
         if (r.flag) *r.flag = true;
         if (r.species >= 0 && !r.is_forcing && !r.is_dqdt) h->have_q[r.species] = true;

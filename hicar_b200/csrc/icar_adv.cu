@@ -56,6 +56,7 @@ struct icar_adv_domain {
     // icar_adv_step_host: copy streams and per-group events, created on first use
     cudaStream_t io_in = nullptr, io_out = nullptr;
     std::vector<cudaEvent_t> io_events;
+    DevBuf io_stage;                          // 2 * IO_SLOTS contiguous species, see icar_adv_step_host
     size_t n_cell = 0, n_u = 0, n_v = 0, n_zf = 0;
     size_t bytes = 0;
     // resident inputs
@@ -1217,6 +1218,7 @@ int icar_adv_destroy(icar_adv_t *h)
                       &h->DJR, &h->Wp, &h->dtbuf, &h->pressure, &h->exner, &h->dz_mass, &h->dz_interface})
         release(*b, st);
     dev_free(h->acc_precip, st);
+    release(h->io_stage, st);
     dev_free(h->mp_stop, st);
     dev_free(h->op_err, st);
     dev_free(h->op_flags, st);
@@ -1522,12 +1524,84 @@ namespace {
 // time; 4 groups left 20 % more exposed).
 constexpr int IO_GROUPS = 12;
 
-int copy_species_async(icar_adv_t *h, float *dev, float *host, bool to_device, cudaStream_t st)
+// Floats of one staging buffer: a contiguous species, rounded to 16 bytes.
+size_t io_slot_floats(const icar_adv_t *h)
+{
+    return ((size_t)h->g.nx * h->g.nz * h->g.ny + 3) / 4 * 4;
+}
+
+// Contiguous species buffers on the device per direction.  A 2-D copy across
+// the host link goes row by row, about 100 ns each: 7200 rows of 800 bytes
+// moved at 8 GB/s, and 12 species of 200x180x40 took 9.0-9.6 ms a step.  A
+// plain copy of the whole species runs at the link's rate, and k_repack lays
+// it out in rows at the device's: 1.79 ms a step, 39 GB/s each way with both
+// directions busy.  Two buffers let the next species' copy run while the last
+// one is repacked.
+constexpr int IO_SLOTS = 2;
+
+// Events of icar_adv_step_host: per group (in, done), the start, and per slot
+// and direction (buffer free).
+constexpr int EV_START = 2 * IO_GROUPS, EV_FREE_IN = EV_START + 1, EV_FREE_OUT = EV_FREE_IN + IO_SLOTS,
+              N_IO_EVENTS = EV_FREE_OUT + IO_SLOTS;
+
+// The staging buffers; without room for them (io_stage.p stays null) the
+// copies go row by row.
+void ensure_io_stage(icar_adv_t *h)
+{
+    if (h->io_stage.p) return;
+    const size_t n = 2 * IO_SLOTS * io_slot_floats(h);
+    if (dev_alloc(h, (void **)&h->io_stage.p, n * sizeof(float)) != cudaSuccess) {
+        cudaGetLastError();
+        h->io_stage.p = nullptr;
+        return;
+    }
+    h->io_stage.n = n;
+    h->bytes += n * sizeof(float);
+}
+
+// Species s from the host: on the copy stream into its slot, then into rows
+// on the handle's stream, which waits for it.
+int species_in(icar_adv_t *h, int s, const float *host, cudaEvent_t arrived)
 {
     const size_t P = (size_t)h->g.P, ex = (size_t)h->g.nx, rows = (size_t)h->g.nz * h->g.ny;
-    cudaError_t ce = to_device ? cudaMemcpy2DAsync(dev, P * 4, host, ex * 4, ex * 4, rows, cudaMemcpyHostToDevice, st)
-                               : cudaMemcpy2DAsync(host, ex * 4, dev, P * 4, ex * 4, rows, cudaMemcpyDeviceToHost, st);
-    if (ce != cudaSuccess) return fail(h, ICAR_ADV_CUDA_ERROR, "cudaMemcpy2DAsync: %s", cudaGetErrorString(ce));
+    if (!h->io_stage.p) {
+        CUDA_TRY(h, cudaMemcpy2DAsync(h->q[s].p, P * 4, host, ex * 4, ex * 4, rows, cudaMemcpyHostToDevice, h->io_in));
+        CUDA_TRY(h, cudaEventRecord(arrived, h->io_in));
+        CUDA_TRY(h, cudaStreamWaitEvent(h->stream, arrived, 0));
+        return ICAR_ADV_OK;
+    }
+    float *slot = h->io_stage.p + (s % IO_SLOTS) * io_slot_floats(h);
+    cudaEvent_t free_in = h->io_events[EV_FREE_IN + s % IO_SLOTS];
+    CUDA_TRY(h, cudaStreamWaitEvent(h->io_in, free_in, 0));
+    CUDA_TRY(h, cudaMemcpyAsync(slot, host, ex * rows * 4, cudaMemcpyHostToDevice, h->io_in));
+    CUDA_TRY(h, cudaEventRecord(arrived, h->io_in));
+    CUDA_TRY(h, cudaStreamWaitEvent(h->stream, arrived, 0));
+    icar::repack(slot, ex, h->q[s].p, P, ex, rows, h->stream);
+    CUDA_TRY(h, cudaEventRecord(free_in, h->stream));
+    return check_launch(h, "species copy");
+}
+
+// Species s to the host from dev: out of its rows into a slot on the handle's
+// stream, then on the other copy stream.
+int species_out(icar_adv_t *h, int s, const float *dev, float *host, cudaEvent_t done)
+{
+    const size_t P = (size_t)h->g.P, ex = (size_t)h->g.nx, rows = (size_t)h->g.nz * h->g.ny;
+    if (!h->io_stage.p) {
+        CUDA_TRY(h, cudaEventRecord(done, h->stream));
+        CUDA_TRY(h, cudaStreamWaitEvent(h->io_out, done, 0));
+        CUDA_TRY(h, cudaMemcpy2DAsync(host, ex * 4, dev, P * 4, ex * 4, rows, cudaMemcpyDeviceToHost, h->io_out));
+        return ICAR_ADV_OK;
+    }
+    float *slot = h->io_stage.p + (IO_SLOTS + s % IO_SLOTS) * io_slot_floats(h);
+    cudaEvent_t free_out = h->io_events[EV_FREE_OUT + s % IO_SLOTS];
+    CUDA_TRY(h, cudaStreamWaitEvent(h->stream, free_out, 0));
+    icar::repack(dev, P, slot, ex, ex, rows, h->stream);
+    int e = check_launch(h, "species copy");
+    if (e) return e;
+    CUDA_TRY(h, cudaEventRecord(done, h->stream));
+    CUDA_TRY(h, cudaStreamWaitEvent(h->io_out, done, 0));
+    CUDA_TRY(h, cudaMemcpyAsync(host, slot, ex * rows * 4, cudaMemcpyDeviceToHost, h->io_out));
+    CUDA_TRY(h, cudaEventRecord(free_out, h->io_out));
     return ICAR_ADV_OK;
 }
 
@@ -1560,14 +1634,15 @@ int icar_adv_step_host(icar_adv_t *h, double dt_seconds, int32_t enforce_limits,
     if (!h->io_in) {
         CUDA_TRY(h, cudaStreamCreateWithFlags(&h->io_in, cudaStreamNonBlocking));
         CUDA_TRY(h, cudaStreamCreateWithFlags(&h->io_out, cudaStreamNonBlocking));
-        h->io_events.assign(2 * IO_GROUPS + 1, nullptr);
+        h->io_events.assign(N_IO_EVENTS, nullptr);
         for (auto &ev : h->io_events) CUDA_TRY(h, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     }
+    ensure_io_stage(h);
     // Every return after the first enqueue goes through `pipeline`, so that
     // on an error the copies already queued into or out of the caller's host
     // arrays are drained before the call returns.
     auto pipeline = [&]() -> int {
-        cudaEvent_t ev_start = h->io_events[2 * IO_GROUPS];
+        cudaEvent_t ev_start = h->io_events[EV_START];
         // uploads start once the work already queued on the handle's stream is done
         CUDA_TRY(h, cudaEventRecord(ev_start, h->stream));
         CUDA_TRY(h, cudaStreamWaitEvent(h->io_in, ev_start, 0));
@@ -1587,9 +1662,7 @@ int icar_adv_step_host(icar_adv_t *h, double dt_seconds, int32_t enforce_limits,
             const int s0 = S * gi / ngroups, s1 = S * (gi + 1) / ngroups;
             cudaEvent_t ev_in = h->io_events[gi], ev_done = h->io_events[IO_GROUPS + gi];
             for (int s = s0; s < s1; s++)
-                if ((e = copy_species_async(h, h->q[s].p, const_cast<float *>(q_in[s]), true, h->io_in))) return e;
-            CUDA_TRY(h, cudaEventRecord(ev_in, h->io_in));
-            CUDA_TRY(h, cudaStreamWaitEvent(h->stream, ev_in, 0));
+                if ((e = species_in(h, s, q_in[s], ev_in))) return e;
             if ((e = forcing_range(h, dt_seconds, s0, s1))) return e;
             if ((e = mp ? mpdata_onepass_group(h, s0, s1) : std_group(h, s0, s1))) return e;
             if (enforce_limits) {
@@ -1597,10 +1670,8 @@ int icar_adv_step_host(icar_adv_t *h, double dt_seconds, int32_t enforce_limits,
                     icar::k_enforce_limits<<<blocks_for(h->n_cell, 256), 256, 0, h->stream>>>(h->g, result(s).p);
                 if ((e = check_launch(h, "enforce_limits", s1 - s0))) return e;
             }
-            CUDA_TRY(h, cudaEventRecord(ev_done, h->stream));
-            CUDA_TRY(h, cudaStreamWaitEvent(h->io_out, ev_done, 0));
             for (int s = s0; s < s1; s++)
-                if ((e = copy_species_async(h, result(s).p, q_out[s], false, h->io_out))) return e;
+                if ((e = species_out(h, s, result(s).p, q_out[s], ev_done))) return e;
         }
         if (h->profiling) {
             cudaEventRecord(ev1, h->stream);

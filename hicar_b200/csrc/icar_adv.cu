@@ -1378,9 +1378,12 @@ int icar_adv_enforce_limits(icar_adv_t *h)
 {
     if (!h) return fail(nullptr, ICAR_ADV_BAD_ARG, "handle is NULL");
     cudaSetDevice(h->desc.device);
-    for (int s = 0; s < h->desc.n_species; s++)
-        icar::k_enforce_limits<<<blocks_for(h->n_cell, 256), 256, 0, h->stream>>>(h->g, h->q[s].p);
-    return check_launch(h, "enforce_limits", h->desc.n_species);
+    float *q[ICAR_ADV_MAX_SPECIES];
+    const int S = h->desc.n_species;
+    if (S == 0) return ICAR_ADV_OK;
+    for (int s = 0; s < S; s++) q[s] = h->q[s].p;
+    icar::enforce_limits(h->g, q, S, h->stream);
+    return check_launch(h, "enforce_limits");
 }
 
 int icar_adv_balance_uvw(icar_adv_t *h)
@@ -1666,9 +1669,10 @@ int icar_adv_step_host(icar_adv_t *h, double dt_seconds, int32_t enforce_limits,
             if ((e = forcing_range(h, dt_seconds, s0, s1))) return e;
             if ((e = mp ? mpdata_onepass_group(h, s0, s1) : std_group(h, s0, s1))) return e;
             if (enforce_limits) {
-                for (int s = s0; s < s1; s++)
-                    icar::k_enforce_limits<<<blocks_for(h->n_cell, 256), 256, 0, h->stream>>>(h->g, result(s).p);
-                if ((e = check_launch(h, "enforce_limits", s1 - s0))) return e;
+                float *q[ICAR_ADV_MAX_SPECIES];
+                for (int s = s0; s < s1; s++) q[s - s0] = result(s).p;
+                icar::enforce_limits(h->g, q, s1 - s0, h->stream);
+                if ((e = check_launch(h, "enforce_limits"))) return e;
             }
             for (int s = s0; s < s1; s++)
                 if ((e = species_out(h, s, result(s).p, q_out[s], ev_done))) return e;

@@ -1425,9 +1425,7 @@ int icar_adv_compute_dt(icar_adv_t *h, const float *dz_levels, float cfl, int32_
     float *d_dz = h->dtbuf.p + 4;
     CUDA_TRY(h, cudaMemcpyAsync(d_dz, dz_levels, sizeof(float) * g.nz, cudaMemcpyHostToDevice, h->stream));
     CUDA_TRY(h, cudaMemsetAsync(d_out, 0, 4 * sizeof(unsigned), h->stream));
-    const size_t total = (size_t)(g.nx + 1) * g.nz * (g.ny + 1);
-    const unsigned blocks = (unsigned)std::min<size_t>(blocks_for(total, 256), 148 * 8);
-    icar::k_dt_maxima<<<blocks, 256, 0, h->stream>>>(g, h->hs, h->desc.dx, h->u.p, h->v.p, h->w.p, d_dz, d_out);
+    icar::k_dt_maxima<<<blocks_for((size_t)g.nz * (g.ny + 1), icar::dtm::WARPS), icar::dtm::NT, 0, h->stream>>>(g, h->hs, h->desc.dx, h->u.p, h->v.p, h->w.p, d_dz, d_out);
     e = check_launch(h, "compute_dt");
     if (e) return e;
     unsigned bits[4];

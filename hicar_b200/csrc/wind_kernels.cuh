@@ -173,40 +173,94 @@ __global__ void __launch_bounds__(balf::NT)
 // out[0..2] = bits of max |u|, |v|, |w| over the arrays; out[3] = bits of
 // the largest per-cell rate over the tile (i, j in [hs, n-1-hs], every k).
 // out must be zero on entry.  dzl is dz_levels (nz).
-__global__ void k_dt_maxima(Geo g, int hs, float dx, const float *__restrict__ u, const float *__restrict__ v,
-                            const float *__restrict__ w, const float *__restrict__ dzl, unsigned *__restrict__ out)
+//
+// Bound by reading the three fields.  Rounded division by a positive number
+// is monotone, so the largest rate is the largest speed divided: of u over
+// the tile's x faces [hs, nx-hs] and of v over its y faces by dx, once per
+// block, and of w over a row of level k by the thickness of level k and (its
+// top face being the bottom face of the next cell) of level k+1, once per
+// thread and row.  So no value is read twice or divided by itself, and a warp
+// reads its row of u, v and w in 16-byte pieces.  With one value per thread,
+// three divisions each and indices from 64-bit divisions the call took 176 us
+// at 512x512x40; it takes 66 now, of which reading 126 MB has to take 19 and
+// the small copies and the wait for the result are most of the rest.
+namespace dtm {
+constexpr int NT = 256, WARPS = NT / 32, U = 2;
+}
+
+// mx: maximum so far over the whole row; tx: over x in [a, b]; both over x < n
+__device__ __forceinline__ void dt_take(float4 v, int i, int n, int a, int b, bool tile, float &mx, float &tx)
 {
-    const int nx = g.nx, ny = g.ny, nz = g.nz;
-    float mu = 0.0f, mv = 0.0f, mw = 0.0f, m3 = 0.0f;
-    const size_t total = (size_t)(nx + 1) * nz * (ny + 1);  // covers u (nx+1 wide) and v (ny+1 rows)
-    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-        const int i = (int)(t % (size_t)(nx + 1));
-        const size_t rest = t / (size_t)(nx + 1);
-        const int k = (int)(rest % (size_t)nz);
-        const int j = (int)(rest / (size_t)nz);
-        const size_t c = ix(g, i, k, j);
-        if (j < ny) mu = fmax_(mu, fabsf(u[c]));
-        if (i < nx) mv = fmax_(mv, fabsf(v[c]));
-        if (i < nx && j < ny) mw = fmax_(mw, fabsf(w[c]));
-        if (i >= hs && i <= nx - 1 - hs && j >= hs && j <= ny - 1 - hs) {
-            const size_t cb = k == 0 ? c : c - (size_t)g.P;
-            const float cu = fmax_(fabsf(u[c]), fabsf(u[c + 1])) / dx;
-            const float cv = fmax_(fabsf(v[c]), fabsf(v[c + (size_t)g.P * nz])) / dx;
-            const float cw = fmax_(fabsf(w[c]), fabsf(w[cb])) / dzl[k];
-            m3 = fmax_(m3, fmax_(fmax_(cu, cv), cw));
+    const float f[4] = {fabsf(v.x), fabsf(v.y), fabsf(v.z), fabsf(v.w)};
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+        const float x = i + m < n ? f[m] : 0.0f;
+        mx = fmax_(x, mx);
+        if (tile && i + m >= a && i + m <= b) tx = fmax_(x, tx);
+    }
+}
+
+__global__ void __launch_bounds__(dtm::NT)
+    k_dt_maxima(Geo g, int hs, float dx, const float *__restrict__ u, const float *__restrict__ v,
+                const float *__restrict__ w, const float *__restrict__ dzl, unsigned *__restrict__ out)
+{
+    using namespace dtm;
+    __shared__ float part[4][WARPS];
+    const int nx = g.nx, ny = g.ny, nz = g.nz, nq = g.P / 4;
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const unsigned row = blockIdx.x * WARPS + warp;  // k + nz*j, j <= ny (v has ny+1 rows)
+    const int j = (int)(row / (unsigned)nz), k = (int)(row - (unsigned)j * nz);
+    float mu = 0.0f, mv = 0.0f, mw = 0.0f, tu = 0.0f, tv = 0.0f, tw = 0.0f;
+    if (j <= ny) {
+        const bool cells = j < ny, tile = j >= hs && j <= ny - 1 - hs, vtile = j >= hs && j <= ny - hs;
+        const float4 *pu = reinterpret_cast<const float4 *>(u + (size_t)row * g.P);
+        const float4 *pv = reinterpret_cast<const float4 *>(v + (size_t)row * g.P);
+        const float4 *pw = reinterpret_cast<const float4 *>(w + (size_t)row * g.P);
+        const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int q0 = lane; q0 < nq; q0 += 32 * U) {
+            float4 a[U], b[U], c[U];
+#pragma unroll
+            for (int m = 0; m < U; m++) {
+                const int q = q0 + 32 * m;
+                const bool in = q < nq;
+                a[m] = in && cells ? pu[q] : zero;
+                b[m] = in ? pv[q] : zero;
+                c[m] = in && cells ? pw[q] : zero;
+            }
+#pragma unroll
+            for (int m = 0; m < U; m++) {
+                const int i = 4 * (q0 + 32 * m);
+                dt_take(a[m], i, nx + 1, hs, nx - hs, tile && hs <= nx - 1 - hs, mu, tu);
+                dt_take(b[m], i, nx, hs, nx - 1 - hs, vtile && hs <= ny - 1 - hs, mv, tv);
+                dt_take(c[m], i, nx, hs, nx - 1 - hs, tile, mw, tw);
+            }
         }
     }
+    float m3 = 0.0f;
+    if (tw > 0.0f) {
+        m3 = fmax_(tw / dzl[k], m3);
+        if (k + 1 < nz) m3 = fmax_(tw / dzl[k + 1], m3);
+    }
+    m3 = fmax_(fmax_(tu, tv) / dx, m3);
     for (int o = 16; o > 0; o >>= 1) {
         mu = fmax_(mu, __shfl_xor_sync(0xffffffffu, mu, o));
         mv = fmax_(mv, __shfl_xor_sync(0xffffffffu, mv, o));
         mw = fmax_(mw, __shfl_xor_sync(0xffffffffu, mw, o));
         m3 = fmax_(m3, __shfl_xor_sync(0xffffffffu, m3, o));
     }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMax(&out[0], __float_as_uint(mu));
-        atomicMax(&out[1], __float_as_uint(mv));
-        atomicMax(&out[2], __float_as_uint(mw));
-        atomicMax(&out[3], __float_as_uint(m3));
+    if (lane == 0) {
+        part[0][warp] = mu;
+        part[1][warp] = mv;
+        part[2][warp] = mw;
+        part[3][warp] = m3;
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        float m = 0.0f;
+        for (int o = 0; o < WARPS; o++) m = fmax_(part[threadIdx.x][o], m);
+        // the values there only grow: no atomic where it could not change them
+        const unsigned bits = __float_as_uint(m);
+        if (bits > *reinterpret_cast<volatile unsigned *>(&out[threadIdx.x])) atomicMax(&out[threadIdx.x], bits);
     }
 }
 

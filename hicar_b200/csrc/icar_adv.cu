@@ -1359,9 +1359,8 @@ int forcing_range(icar_adv_t *h, double dt_seconds, int s0, int s1)
         ns++;
     }
     if (ns == 0) return ICAR_ADV_OK;
-    const size_t n = (size_t)h->nzone * h->g.nz * ns;
-    icar::k_apply_forcing<<<blocks_for(n, 256), 256, 0, h->stream>>>(h->g, h->nzone, h->zone_dev, h->filter_dev,
-                                                                      dt_seconds, fp, ns);
+    const dim3 grid(blocks_for(h->nzone, 256), blocks_for(h->g.nz, icar::FORCE_LEVELS), (unsigned)ns);
+    icar::k_apply_forcing<<<grid, 256, 0, h->stream>>>(h->g, h->nzone, h->zone_dev, h->filter_dev, dt_seconds, fp);
     return check_launch(h, "apply_forcing");
 }
 

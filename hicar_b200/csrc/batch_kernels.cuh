@@ -72,64 +72,15 @@ __global__ void k_batch_forcing(const BatchMember *__restrict__ mem, const int *
         q[c] = (float)((double)q[c] + ((double)flt * m.dtd / 3600.0) * (double)(fnew - q[c]));
 }
 
-// prefix over members of ceil((nx+1)*nz*(ny+1)/256) blocks
-__global__ void k_batch_prep(const BatchMember *__restrict__ mem, const int *__restrict__ prefix, int nmem)
+// prefix over members of ceil(prep_quads/256) blocks
+__global__ void __launch_bounds__(256)
+    k_batch_prep(const BatchMember *__restrict__ mem, const int *__restrict__ prefix, int nmem)
 {
     const int mi = find_owner(prefix, nmem, blockIdx.x);
     const BatchMember &m = mem[mi];
-    const Geo g = m.g;
-    const size_t t = (size_t)(blockIdx.x - prefix[mi]) * blockDim.x + threadIdx.x;
-    const int ni = g.nx + 1, nk = g.nz, nj = g.ny + 1;
-    const int i = (int)(t % (size_t)ni);
-    const size_t rest = t / (size_t)ni;
-    const int k = (int)(rest % (size_t)nk);
-    const int j = (int)(rest / (size_t)nk);
-    if (j >= nj) return;
-    const int adv_den = m.adv_den;
-    const float dt = m.dt, dx = m.dx;
+    const PrepFields f{m.u, m.v, m.w, m.rho, m.jac, m.ju, m.jv, m.jw, m.dz, m.Um, m.Vm, m.Wm, m.Gc, m.DJR, m.Wp};
     bool bad = false, tie = false;
-    if (j < g.ny) {
-        size_t c = ix(g, i, k, j);
-        if (i >= 1 && i <= g.nx - 1) {
-            float rr = adv_den ? m.rho[c] : 1.0f;
-            float rl = adv_den ? m.rho[c - 1] : 1.0f;
-            const float um = m.u[c] * dt * (rr + rl) * 0.5f * m.ju[c] / dx;
-            m.Um[c] = um;
-            bad |= !exact_wind(um);
-        } else {
-            m.Um[c] = 0.0f;
-        }
-        if (i < g.nx) {
-            float r0 = adv_den ? m.rho[c] : 1.0f;
-            float wm;
-            if (k < g.nz - 1) {
-                float r1 = adv_den ? m.rho[ix(g, i, k + 1, j)] : 1.0f;
-                wm = m.w[c] * dt * m.jw[c] * (r1 + r0) * 0.5f;
-            } else {
-                wm = m.w[c] * dt * m.jw[c] * r0;
-            }
-            m.Wm[c] = wm;
-            const float d = m.dz[c], jj = m.jac[c], rh = m.rho[c];
-            const float G = jj * rh, D = d * jj * rh, wp = wm / d;
-            m.Gc[c] = G;
-            m.DJR[c] = D;
-            m.Wp[c] = wp;
-            bad |= !exact_wind(wp) || !(fabsf(wm) < 0x1p20f) || !exact_metric(G) || !exact_metric(D) || !exact_metric(d);
-            tie |= tie_divisor(G) || tie_divisor(D);
-        }
-    }
-    if (i < g.nx) {
-        size_t c = ix(g, i, k, j);
-        if (j >= 1 && j <= g.ny - 1) {
-            float rr = adv_den ? m.rho[c] : 1.0f;
-            float rl = adv_den ? m.rho[ix(g, i, k, j - 1)] : 1.0f;
-            const float vm = m.v[c] * dt * (rr + rl) * 0.5f * m.jv[c] / dx;
-            m.Vm[c] = vm;
-            bad |= !exact_wind(vm);
-        } else {
-            m.Vm[c] = 0.0f;
-        }
-    }
+    prep_quad(m.g, m.dx, m.dt, m.adv_den, f, (blockIdx.x - prefix[mi]) * blockDim.x + threadIdx.x, bad, tie);
     if (bad && m.flags) m.flags[FLAG_IEEE] = m.epoch;
     if (tie && m.flags) m.flags[FLAG_TIE] = m.epoch;
 }

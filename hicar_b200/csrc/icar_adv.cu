@@ -893,11 +893,10 @@ int mpdata_prep(icar_adv_t *h, float dt)
     const Geo &g = h->g;
     int e = ensure_onepass(h);
     if (e) return e;
-    const size_t nf = (size_t)(g.nx + 1) * g.nz * (g.ny + 1);
-    icar::k_mp_prep<<<blocks_for(nf, 256), 256, 0, h->stream>>>(
-        g, h->desc.dx, dt, h->opts.advect_density, h->u.p, h->v.p, h->w.p, h->rho.p, h->jac.p, h->jac_u.p,
-        h->jac_v.p, h->jac_w.p, h->dz.p, h->Um.p, h->Vm.p, h->Wm.p, h->Gc.p, h->DJR.p, h->Wp.p, h->op_flags,
-        ++h->op_epoch);
+    const icar::PrepFields f{h->u.p,     h->v.p,  h->w.p,  h->rho.p, h->jac.p, h->jac_u.p, h->jac_v.p, h->jac_w.p,
+                             h->dz.p,    h->Um.p, h->Vm.p, h->Wm.p,  h->Gc.p,  h->DJR.p,   h->Wp.p};
+    icar::k_mp_prep<<<blocks_for(icar::prep_quads(g), 256), 256, 0, h->stream>>>(
+        g, h->desc.dx, dt, h->opts.advect_density, f, h->op_flags, ++h->op_epoch);
     if (h->opts.debug &&
         icar::check_courant(h->stream, h->g, h->Um.p, h->Vm.p, h->Wm.p, h->dz.p, h->jac.p, h->rho.p, 1))
         return fail(h, ICAR_ADV_CFL_VIOLATION, "a Courant number >= 1 was found (debug check)");
@@ -2050,8 +2049,7 @@ int build_tables(icar_adv_batch_t *b)
         fill_member(mem[0][m], h, b->dts[m], b->parity == 0 ? 0 : 1);
         fill_member(mem[1][m], h, b->dts[m], b->parity == 0 ? 1 : 0);
         const Geo &g = h->g;
-        const size_t nf = (size_t)(g.nx + 1) * g.nz * (g.ny + 1);
-        prep[m + 1] = prep[m] + (int)((nf + 255) / 256);
+        prep[m + 1] = prep[m] + (int)((icar::prep_quads(g) + 255) / 256);
         for (int s = 0; s < h->desc.n_species; s++) {
             if (h->forcing[s].p && h->nzone > 0) {
                 pairs.push_back(make_int2(m, s));
@@ -2620,11 +2618,11 @@ extern "C" int icar_adv_advect_noalloc(const icar_adv_noalloc_args *a)
     // tile loads read must start at zero, so clear the part this call uses
     ce = cudaMemsetAsync(base, 0, need * sizeof(float), st);
     if (ce != cudaSuccess) return fail(nullptr, ICAR_ADV_CUDA_ERROR, "cudaMemsetAsync: %s", cudaGetErrorString(ce));
-    const size_t nf = (size_t)(g.nx + 1) * g.nz * (g.ny + 1);
-    icar::k_mp_prep<<<blocks_for(nf, 256), 256, 0, st>>>(g, a->dx, a->dt, a->advect_density, a->u, a->v, a->w,
-                                                       a->density, a->jacobian, a->jacobian_u, a->jacobian_v,
-                                                       a->jacobian_w, a->advection_dz, Um, Vm, Wm, Gc, DJR, Wp, nullptr, 0);
-    // the column-march donor-cell pass of the handle path, one species at a
+    const icar::PrepFields f{a->u,          a->v,            a->w,  a->density, a->jacobian, a->jacobian_u, a->jacobian_v,
+                             a->jacobian_w, a->advection_dz, Um, Vm, Wm,         Gc,          DJR,           Wp};
+    icar::k_mp_prep<<<blocks_for(icar::prep_quads(g), 256), 256, 0, st>>>(g, a->dx, a->dt, a->advect_density, f, nullptr,
+                                                                        0);
+    // the column-march donor-cell pass, one species at a
     // time through the one pass-1 field of the scratch
     const dim3 gu((unsigned)((g.nx + icar::upf::BX - 1) / icar::upf::BX),
                   (unsigned)((g.ny + icar::upf::BY - 1) / icar::upf::BY), 1u);

@@ -54,63 +54,103 @@ __device__ __forceinline__ bool tie_divisor(float x)
     return x >= 4.0f && rintf(0.5f * x) * 2.0f == x && (__float_as_int(x) & 0x7fffff) != 0;
 }
 
-__global__ void k_mp_prep(Geo g, float dx, float dt, int adv_den, const float *__restrict__ u,
-                          const float *__restrict__ v, const float *__restrict__ w, const float *__restrict__ rho,
-                          const float *__restrict__ jac, const float *__restrict__ ju, const float *__restrict__ jv,
-                          const float *__restrict__ jw, const float *__restrict__ dz, float *__restrict__ Um,
-                          float *__restrict__ Vm, float *__restrict__ Wm, float *__restrict__ Gc,
-                          float *__restrict__ DJR, float *__restrict__ Wp, int *flags, int epoch)
+// Bound by memory: nine fields read, six written, 630 MB at 512x512x40 (96 us
+// at the measured copy rate).  A thread takes four cells of a row with
+// 16-byte loads and stores and 32-bit index arithmetic; one cell per thread
+// with 64-bit divisions for its indices took 157 us,
+// this takes about 90.  The pad
+// columns of the results are written as the zeros they hold.
+struct PrepFields {
+    const float *u, *v, *w, *rho, *jac, *ju, *jv, *jw, *dz;
+    float *Um, *Vm, *Wm, *Gc, *DJR, *Wp;
+};
+
+// four-cell groups of the prep of one domain: every row of the y faces
+__host__ __device__ inline size_t prep_quads(const Geo &g) { return (size_t)(g.P / 4) * g.nz * (g.ny + 1); }
+
+__device__ __forceinline__ void load4(float (&r)[4], const float *p)
 {
-    size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int ni = g.nx + 1, nk = g.nz, nj = g.ny + 1;
-    const int i = (int)(t % (size_t)ni);
-    size_t rest = t / (size_t)ni;
-    const int k = (int)(rest % (size_t)nk);
-    const int j = (int)(rest / (size_t)nk);
-    if (j >= nj) return;
-    bool bad = false, tie = false;
-    if (j < g.ny) {
-        size_t c = ix(g, i, k, j);
-        if (i >= 1 && i <= g.nx - 1) {
-            float rr = adv_den ? rho[c] : 1.0f;
-            float rl = adv_den ? rho[c - 1] : 1.0f;
-            const float um = u[c] * dt * (rr + rl) * 0.5f * ju[c] / dx;
-            Um[c] = um;
-            bad |= !exact_wind(um);
-        } else {
-            Um[c] = 0.0f;
-        }
-        if (i < g.nx) {
-            float r0 = adv_den ? rho[c] : 1.0f;
-            float wm;
-            if (k < g.nz - 1) {
-                float r1 = adv_den ? rho[ix(g, i, k + 1, j)] : 1.0f;
-                wm = w[c] * dt * jw[c] * (r1 + r0) * 0.5f;
-            } else {
-                wm = w[c] * dt * jw[c] * r0;
+    const float4 v = *reinterpret_cast<const float4 *>(p);
+    r[0] = v.x; r[1] = v.y; r[2] = v.z; r[3] = v.w;
+}
+__device__ __forceinline__ void store4(float *p, const float (&r)[4])
+{
+    *reinterpret_cast<float4 *>(p) = make_float4(r[0], r[1], r[2], r[3]);
+}
+
+__device__ __forceinline__ void prep_quad(const Geo &g, float dx, float dt, int adv_den, const PrepFields &f, unsigned t,
+                                          bool &bad, bool &tie)
+{
+    const unsigned nq = (unsigned)g.P / 4u, row = t / nq;
+    const int i = 4 * (int)(t - row * nq), nx = g.nx, nz = g.nz;
+    const int j = (int)(row / (unsigned)nz), k = (int)(row - (unsigned)j * (unsigned)nz);
+    if (j > g.ny) return;
+    const size_t c = (size_t)row * g.P + i;
+    const bool cells = j < g.ny, yface = j >= 1 && j < g.ny;
+    float rh[4] = {1.0f, 1.0f, 1.0f, 1.0f}, r0[4] = {1.0f, 1.0f, 1.0f, 1.0f};
+    if (cells) {
+        load4(rh, f.rho + c);
+        if (adv_den)
+#pragma unroll
+            for (int m = 0; m < 4; m++) r0[m] = rh[m];
+    }
+    if (cells) {
+        const bool mid = k < nz - 1;
+        const float left = adv_den && i > 0 ? f.rho[c - 1] : 1.0f;
+        float r1[4] = {1.0f, 1.0f, 1.0f, 1.0f}, u[4], ju[4], w[4], jw[4], d[4], jj[4];
+        if (adv_den && mid) load4(r1, f.rho + c + g.P);
+        load4(u, f.u + c);
+        load4(ju, f.ju + c);
+        load4(w, f.w + c);
+        load4(jw, f.jw + c);
+        load4(d, f.dz + c);
+        load4(jj, f.jac + c);
+        float um[4], wm[4], G[4], D[4], wp[4];
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            const int x = i + m;
+            um[m] = wm[m] = G[m] = D[m] = wp[m] = 0.0f;
+            if (x >= 1 && x < nx) {
+                um[m] = u[m] * dt * (r0[m] + (m ? r0[m ? m - 1 : 0] : left)) * 0.5f * ju[m] / dx;
+                bad |= !exact_wind(um[m]);
             }
-            Wm[c] = wm;
-            const float d = dz[c], jj = jac[c], rh = rho[c];
-            const float G = jj * rh, D = d * jj * rh, wp = wm / d;
-            Gc[c] = G;
-            DJR[c] = D;
-            Wp[c] = wp;
-            bad |= !exact_wind(wp) || !(fabsf(wm) < 0x1p20f) || !exact_metric(G) || !exact_metric(D) || !exact_metric(d);
-            tie |= tie_divisor(G) || tie_divisor(D);
+            if (x < nx) {
+                wm[m] = mid ? w[m] * dt * jw[m] * (r1[m] + r0[m]) * 0.5f : w[m] * dt * jw[m] * r0[m];
+                G[m] = jj[m] * rh[m];
+                D[m] = d[m] * jj[m] * rh[m];
+                wp[m] = wm[m] / d[m];
+                bad |= !exact_wind(wp[m]) || !(fabsf(wm[m]) < 0x1p20f) || !exact_metric(G[m]) || !exact_metric(D[m]) ||
+                       !exact_metric(d[m]);
+                tie |= tie_divisor(G[m]) || tie_divisor(D[m]);
+            }
         }
+        store4(f.Um + c, um);
+        store4(f.Wm + c, wm);
+        store4(f.Gc + c, G);
+        store4(f.DJR + c, D);
+        store4(f.Wp + c, wp);
     }
-    if (i < g.nx) {
-        size_t c = ix(g, i, k, j);
-        if (j >= 1 && j <= g.ny - 1) {
-            float rr = adv_den ? rho[c] : 1.0f;
-            float rl = adv_den ? rho[ix(g, i, k, j - 1)] : 1.0f;
-            const float vm = v[c] * dt * (rr + rl) * 0.5f * jv[c] / dx;
-            Vm[c] = vm;
-            bad |= !exact_wind(vm);
-        } else {
-            Vm[c] = 0.0f;
-        }
+    float vm[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (yface) {
+        float rl[4] = {1.0f, 1.0f, 1.0f, 1.0f}, v[4], jv[4];
+        if (adv_den) load4(rl, f.rho + c - (size_t)g.P * nz);
+        load4(v, f.v + c);
+        load4(jv, f.jv + c);
+#pragma unroll
+        for (int m = 0; m < 4; m++)
+            if (i + m < nx) {
+                vm[m] = v[m] * dt * (r0[m] + rl[m]) * 0.5f * jv[m] / dx;
+                bad |= !exact_wind(vm[m]);
+            }
     }
+    store4(f.Vm + c, vm);
+}
+
+__global__ void __launch_bounds__(256)
+    k_mp_prep(Geo g, float dx, float dt, int adv_den, const __grid_constant__ PrepFields f, int *flags, int epoch)
+{
+    bool bad = false, tie = false;
+    prep_quad(g, dx, dt, adv_den, f, blockIdx.x * blockDim.x + threadIdx.x, bad, tie);
     if (bad && flags) flags[FLAG_IEEE] = epoch;
     if (tie && flags) flags[FLAG_TIE] = epoch;
 }

@@ -57,9 +57,8 @@ __device__ __forceinline__ bool tie_divisor(float x)
 // Bound by memory: nine fields read, six written, 630 MB at 512x512x40 (96 us
 // at the measured copy rate).  A thread takes four cells of a row with
 // 16-byte loads and stores and 32-bit index arithmetic; one cell per thread
-// with 64-bit divisions for its indices took 157 us,
-// this takes about 90.  The pad
-// columns of the results are written as the zeros they hold.
+// with 64-bit divisions for its indices took 157 us, this takes about 90.  The
+// pad columns of the results are written as the zeros they hold.
 struct PrepFields {
     const float *u, *v, *w, *rho, *jac, *ju, *jv, *jw, *dz;
     float *Um, *Vm, *Wm, *Gc, *DJR, *Wp;

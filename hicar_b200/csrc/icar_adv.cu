@@ -926,6 +926,10 @@ int ensure_std_fused(icar_adv_t *h)
         if ((e = alloc(h, h->Gc, h->n_cell)) || (e = alloc(h, h->DJR, h->n_cell))) return e;
         for (int s = 0; s < S; s++)
             if ((e = alloc(h, h->qn[s], h->n_cell)) || (e = alloc(h, h->q1s[s], h->n_cell))) return e;
+        if (!h->op_flags) {
+            CUDA_TRY(h, dev_alloc(h, (void **)&h->op_flags, icar::N_FLAGS * sizeof(int)));
+            CUDA_TRY(h, cudaMemsetAsync(h->op_flags, 0, icar::N_FLAGS * sizeof(int), h->stream));
+        }
         cudaError_t ce = icar::std_fused_setup();
         if (ce != cudaSuccess) return fail(h, ICAR_ADV_CUDA_ERROR, "cudaFuncSetAttribute: %s", cudaGetErrorString(ce));
         h->std_ready = true;
@@ -944,7 +948,7 @@ int std_prep(icar_adv_t *h, float dt)
     const float *rho = h->have_rho ? h->rho.p : h->jac.p;  // only read when advect_density
     icar::k_std_prep<<<blocks_for(nf, 256), 256, 0, h->stream>>>(
         g, h->desc.dx, dt, h->opts.advect_density, h->u.p, h->v.p, h->w.p, rho, h->jac.p, h->jac_u.p, h->jac_v.p,
-        h->jac_w.p, h->dz.p, h->Um.p, h->Vm.p, h->Wm.p, h->Gc.p, h->DJR.p);
+        h->jac_w.p, h->dz.p, h->Um.p, h->Vm.p, h->Wm.p, h->Gc.p, h->DJR.p, h->op_flags, ++h->op_epoch);
     if (h->opts.debug &&
         icar::check_courant(h->stream, h->g, h->Um.p, h->Vm.p, h->Wm.p, h->dz.p, h->jac.p, h->rho.p,
                             h->opts.advect_density))
@@ -969,7 +973,7 @@ int std_group(icar_adv_t *h, int s0, int s1)
             sp.out[s] = (*out)[s0 + s].p;
         }
         return icar::std_fused_launch(h->stream, c, ho, vo, g, hs, tf, sp, S, h->Um.p, h->Vm.p, h->Wm.p, h->Gc.p,
-                                      h->DJR.p);
+                                      h->DJR.p, h->op_flags, h->op_epoch);
     };
     cudaEvent_t c0 = nullptr, c1 = nullptr;
     if (h->profiling) {

@@ -64,7 +64,8 @@ namespace icar {
 // Measured at 256x256x40 with five species, orders 5/3: the corrected stage
 // 756 -> 572 us (38 -> 33 warp-instructions per cell-species; a third of the
 // gain from each thread forming the faces of its own cell, whose values it
-// holds, instead of faces dealt out by index), the plain stage 206 -> 203.
+// holds, instead of faces dealt out by index), the plain stage 206 -> 203, and
+// 166 with its faces on the owning threads too.
 constexpr float STD_WIND_MAX = 0x1p20f;
 constexpr float STD_VALUE_MAX = 0x1p120f;
 
@@ -331,6 +332,7 @@ __device__ __forceinline__ float std_stage_tile(const StdArith ar, float *sm, co
     using namespace stdf;
     constexpr int PW = SH::PW, PLANE = SH::PLANE, RPW = SH::RPW, TX = SH::TX, TY = SH::TY;
     const int nz = g.nz;
+    static_assert(TX == 32 && TY <= 32 && SH::NW >= 2, "the last faces go to two warps");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ox = floor4(i0 - SH::HX), oy = j0 - SH::HX;
     const size_t P = (size_t)g.P;
@@ -388,29 +390,34 @@ __device__ __forceinline__ float std_stage_tile(const StdArith ar, float *sm, co
         const float *V = PL(P_V + (b & 1));
         float *FX = PL(P_FX);
         float *FY = PL(P_FY);
-        // x faces i0..i0+TX of the tile rows, then y faces j0..j0+TY of the
-        // tile columns, as one index range: the leftover faces of both sets
-        // share one last partial round instead of one round each.
-        constexpr int NFX = (TX + 1) * TY, NF = NFX + TX * (TY + 1);
-        for (int e = threadIdx.x; e < NF; e += SH::NT) {
-            if (e < NFX) {
-                const int fx = e % (TX + 1), ry = e / (TX + 1);
-                const int p = (j0 + ry - oy) * PW + (i0 + fx - ox);
-                FX[p] = hflux(HORD, QF + p, 1, U[p] * tf);
-            } else {
-                const int cx = (e - NFX) % TX, fy = (e - NFX) / TX;
-                const int p = (j0 + fy - oy) * PW + (i0 + cx - ox);
-                FY[p] = hflux(HORD, QF + p, PW, V[p] * tf);
-            }
+        // Each thread forms the west and south faces of its own cells and keeps
+        // them; the east face comes from the lane beside it and the north face
+        // from the thread's next row or, through the planes, the next warp.
+        // The tile's last x and y faces go to the first two warps.
+        float fw[RPW], fs[RPW];
+#pragma unroll
+        for (int rr = 0; rr < RPW; rr++) {
+            const int p = (yr[rr] - oy) * PW + (x - ox);
+            fw[rr] = hflux(HORD, QF + p, 1, U[p] * tf);
+            fs[rr] = hflux(HORD, QF + p, PW, V[p] * tf);
+            FX[p] = fw[rr];
+            if (rr == 0) FY[p] = fs[0];
+        }
+        if (warp == 0) {
+            const int p = (j0 + TY - oy) * PW + (x - ox);
+            FY[p] = hflux(HORD, QF + p, PW, V[p] * tf);
+        } else if (warp == 1 && lane < TY) {
+            const int p = (j0 + lane - oy) * PW + (i0 + TX - ox);
+            FX[p] = hflux(HORD, QF + p, 1, U[p] * tf);
         }
         __syncthreads();
 #pragma unroll
         for (int rr = 0; rr < RPW; rr++) {
-            const int px = x - ox, py = yr[rr] - oy;
-            const int p = py * PW + px;
+            const int p = (yr[rr] - oy) * PW + (x - ox);
+            const float fn = rr + 1 < RPW ? fs[rr + 1 < RPW ? rr + 1 : 0] : FY[p + PW];
             const float fzt = std_zflux<VORD>(b + 1, nz, qfz[rr], wz[rr] * tf);
             if (act[rr]) {
-                const float tq = qo[rr] - std_quot<EX>((FX[p + 1] - FX[p]) + (FY[p + PW] - FY[p]), gz[rr],
+                const float tq = qo[rr] - std_quot<EX>((FX[p + 1] - fw[rr]) + (fn - fs[rr]), gz[rr],
                                                        std_nrcp<EX>(gz[rr]), ar);
                 const float o = tq - std_quot<EX>(fzt - fzb[rr], djr[rr], std_nrcp<EX>(djr[rr]), ar);
                 out[c0[rr] + (size_t)b * P] = o;
@@ -743,7 +750,7 @@ __device__ __noinline__ void std_redo(float *sm, const Geo &g, int its, int ite,
                                       const float *qf, const float *qold, float *out, int i0, int j0, const float *Um,
                                       const float *Vm, const float *Wm, const float *Gc, const float *DJR)
 {
-    if (SH::CORR)
+    if constexpr (SH::CORR)
         std_corr_tile<HORD, VORD, SH, false>({false}, sm, g, its, ite, jts, jte, tf, qf, qold, out, i0, j0, Um, Vm, Wm,
                                              Gc, DJR);
     else
@@ -770,7 +777,7 @@ __global__ void __launch_bounds__(SH::NT, SH::CORR ? 1 : 3)
     if (!redo) {
         const StdArith ar{flags[FLAG_TIE] == epoch};
         float worst;
-        if (SH::CORR)
+        if constexpr (SH::CORR)
             worst = std_corr_tile<HORD, VORD, SH, true>(ar, sm, g, its, ite, jts, jte, tf, sp.q1[s], sp.q0[s],
                                                         sp.out[s], i0, j0, Um, Vm, Wm, Gc, DJR);
         else

@@ -1407,8 +1407,9 @@ int icar_adv_balance_uvw(icar_adv_t *h)
     const float *rho = adv_den ? h->rho.p : h->jac.p;  // only read when advect_density
     const dim3 grid((unsigned)((g.nx + icar::balf::BX - 1) / icar::balf::BX),
                     (unsigned)((g.ny + icar::balf::BY - 1) / icar::balf::BY));
-    icar::k_balance_uvw<<<grid, icar::balf::NT, icar::balf::SMEM, h->stream>>>(
-        g, h->hs, h->desc.dx, adv_den, h->u.p, h->v.p, rho, h->dz.p, h->jac_u.p, h->jac_v.p, h->jac_w.p, h->w.p);
+    auto *kernel = adv_den ? icar::k_balance_uvw<true> : icar::k_balance_uvw<false>;
+    kernel<<<grid, icar::balf::NT, icar::balf::SMEM, h->stream>>>(g, h->hs, h->desc.dx, h->u.p, h->v.p, rho, h->dz.p,
+                                                                  h->jac_u.p, h->jac_v.p, h->jac_w.p, h->w.p);
     h->have_w = true;
     return check_launch(h, "balance_uvw");
 }

@@ -3,7 +3,7 @@
 //
 //   k_balance_uvw   balance_uvw (src/physics/wind.f90:88-164) with
 //                   calc_divergence(horz_only) and calc_w (:166-271): one
-//                   thread per (i, j) column marches up the column, forming
+//                   thread per two columns marches up them, forming
 //                   the horizontal divergence of the metric-weighted u, v at
 //                   each level and integrating w from w = 0 below the ground;
 //                   the levels arrive in shared-memory planes ahead of use.
@@ -24,13 +24,13 @@
 namespace icar {
 
 namespace balf {
-// CTA tile: 32 x 8 columns, one thread per column marching up k.  The
-// seven fields a level needs (u, J_u, v, J_v, rho, dz, J_w) arrive in
-// shared-memory planes by 16-byte cp.async, DEPTH levels ahead of use:
+// CTA tile: 32 x 8 columns, one thread per two columns adjacent in y marching
+// up k.  The seven fields a level needs (u, J_u, v, J_v, rho, dz, J_w) arrive
+// in shared-memory planes by 16-byte cp.async, DEPTH levels ahead of use:
 // each plane spans x from i0-4 (a multiple of 4) to i0+35 and y from j0-1
 // to j0+8, covering the faces i0..i0+32 / j0..j0+8 and the density
 // neighbours the face weights read.
-constexpr int BX = 32, BY = 8, NT = BX * BY;
+constexpr int BX = 32, BY = 8, RPT = 2, NT = BX * BY / RPT;
 constexpr int PW = 40, PH = BY + 2, PLANE = PW * PH;
 constexpr int NF = 7;                      // u, ju, v, jv, rho, dz, jw
 constexpr int DEPTH = 3, NSLOT = DEPTH + 1;
@@ -38,64 +38,40 @@ constexpr int CPR = PW / 4, NCH = (NF * CPR * PH + NT - 1) / NT;
 constexpr size_t SMEM = (size_t)NSLOT * NF * PLANE * sizeof(float);
 }  // namespace balf
 
-// u*J_u on x face f, times the face density when advect_density (the
-// outermost faces extrapolate it), wind.f90:237-239.  U, JU, R point at
-// the cell's row of the u, J_u and density planes; plane column = index -
-// ox.
-__device__ __forceinline__ float umet_p(int nx, int adv_den, const float *U, const float *JU, const float *R, int f,
-                                        int ox)
-{
-    const int p = f - ox;
-    const float uj = U[p] * JU[p];
-    if (!adv_den) return uj;
-    if (f == 0) return uj * (1.5f * R[0 - ox] - 0.5f * R[1 - ox]);
-    if (f == nx) return uj * (1.5f * R[nx - 1 - ox] - 0.5f * R[nx - 2 - ox]);
-    return uj * (R[p - 1] + R[p]) / 2.0f;
-}
-
-// v*J_v on y face gy, wind.f90:241-243; V, JV, R point at row gy of the v,
-// J_v and density planes in the cell's column (rows of stride balf::PW).
-__device__ __forceinline__ float vmet_p(int ny, int adv_den, const float *V, const float *JV, const float *R, int gy)
-{
-    constexpr int W = balf::PW;
-    const float vj = V[0] * JV[0];
-    if (!adv_den) return vj;
-    if (gy == 0) return vj * (1.5f * R[0] - 0.5f * R[W]);
-    if (gy == ny) return vj * (1.5f * R[-W] - 0.5f * R[-2 * W]);
-    return vj * (R[-W] + R[0]) / 2.0f;
-}
-
 // Columns i_s..i_e x j_s..j_e (its-1..ite+1 clipped to the domain, i.e.
 // [max(hs-1,0), min(n-hs,n-1)] for one image with halo hs) get the balanced
 // w; every other column gets w = 0 (calc_w sets the whole array first).
-__global__ void __launch_bounds__(balf::NT)
-    k_balance_uvw(Geo g, int hs, float dx, int adv_den, const float *__restrict__ u, const float *__restrict__ v,
-                  const float *__restrict__ rho, const float *__restrict__ dz, const float *__restrict__ ju,
-                  const float *__restrict__ jv, const float *__restrict__ jw, float *__restrict__ w)
+//
+// Face values: u*J_u times the face density when ADV (the outermost faces
+// extrapolate it), wind.f90:237-239; v*J_v likewise, :241-243.  EDGE tiles
+// touch the domain's sides, the others have no outermost face.
+//
+// 334 MB at 512x512x40 (51 us at the measured copy rate), bound by issue.  Two
+// adjacent columns per thread share the y face between them and the densities
+// of their rows, and tiles inside the domain carry no side conditions:
+// 86 us where one column per thread with them took 99.
+template <bool ADV, bool EDGE>
+__device__ __forceinline__ void balance_march(float *sm, const Geo &g, int hs, float dx, int i0, int j0,
+                                              const float *__restrict__ u, const float *__restrict__ v,
+                                              const float *__restrict__ rho, const float *__restrict__ dz,
+                                              const float *__restrict__ ju, const float *__restrict__ jv,
+                                              const float *__restrict__ jw, float *__restrict__ w)
 {
     using namespace balf;
-    extern __shared__ float4 sm4[];
-    float *sm = reinterpret_cast<float *>(sm4);
-    const int tx = threadIdx.x % BX, ty = threadIdx.x / BX;
-    const int i0 = blockIdx.x * BX, j0 = blockIdx.y * BY;
+    const int tx = threadIdx.x % BX, ty = threadIdx.x / BX * RPT;
     const int i = i0 + tx, j = j0 + ty;
     const int nx = g.nx, ny = g.ny, nz = g.nz;
     const int ox = i0 - 4, oy = j0 - 1;
     const int i_s = max(hs - 1, 0), i_e = min(nx - hs, nx - 1);
     const int j_s = max(hs - 1, 0), j_e = min(ny - hs, ny - 1);
-    const bool in = i < nx && j < ny;
-    const bool bal = in && i >= i_s && i <= i_e && j >= j_s && j <= j_e;
     // every thread's chunks of one level: field f, row ly, chunk cx
     const float *src[NCH];
-    size_t off[NCH];
     int dst[NCH];
-    bool ok[NCH];
+    unsigned okm = 0u;
 #pragma unroll
     for (int c = 0; c < NCH; c++) {
         const int e = threadIdx.x + c * NT;
         dst[c] = -1;
-        ok[c] = false;
-        off[c] = 0;
         src[c] = u;
         if (e < NF * CPR * PH) {
             const int f = e / (CPR * PH), r = e % (CPR * PH);
@@ -103,71 +79,111 @@ __global__ void __launch_bounds__(balf::NT)
             const int gi = ox + 4 * cx, gj = oy + ly;
             const bool yface = f == 2 || f == 3;
             dst[c] = f * PLANE + ly * PW + 4 * cx;
-            src[c] = f == 0 ? u : f == 1 ? ju : f == 2 ? v : f == 3 ? jv : f == 4 ? rho : f == 5 ? dz : jw;
-            ok[c] = gi >= 0 && gi < g.P && gj >= 0 && gj < (yface ? ny + 1 : ny);
-            if (ok[c]) off[c] = (size_t)gi + (size_t)g.P * nz * gj;
+            const float *base = f == 0 ? u : f == 1 ? ju : f == 2 ? v : f == 3 ? jv : f == 4 ? rho : f == 5 ? dz : jw;
+            if (gi >= 0 && gi < g.P && gj >= 0 && gj < (yface ? ny + 1 : ny)) {
+                okm |= 1u << c;
+                src[c] = base + (size_t)gi + (size_t)g.P * nz * gj;
+            }
         }
     }
     auto issue = [&](int k) {
         if (k < nz) {
             float *slot = sm + (size_t)(k % NSLOT) * NF * PLANE;
-            const size_t lo = (size_t)k * g.P;
 #pragma unroll
             for (int c = 0; c < NCH; c++)
-                if (dst[c] >= 0) cp_async16(slot + dst[c], ok[c] ? src[c] + off[c] + lo : src[c], ok[c]);
+                if (dst[c] >= 0) {
+                    const bool ok = (okm >> c) & 1u;
+                    cp_async16(slot + dst[c], src[c], ok);
+                    if (ok) src[c] += g.P;
+                }
         }
         cp_async_commit();
     };
 #pragma unroll
     for (int k = 0; k < DEPTH; k++) issue(k);
-    float wb = 0.0f, rib = 0.0f, jwb = 0.0f;  // w, interface density and J_w one level down
-    const int px = i - ox, py = j - oy;
+    bool in[RPT], bal[RPT];
+    float wb[RPT], rib[RPT], jwb[RPT];  // w, interface density and J_w one level down
+    float *wp[RPT];
+#pragma unroll
+    for (int r = 0; r < RPT; r++) {
+        in[r] = i < nx && j + r < ny;
+        bal[r] = in[r] && i >= i_s && i <= i_e && j + r >= j_s && j + r <= j_e;
+        wb[r] = rib[r] = jwb[r] = 0.0f;
+        wp[r] = w + (in[r] ? ix(g, i, 0, j + r) : 0);
+    }
+    const int pc = (ty + 1) * PW + tx + 4;
     for (int k = 0; k < nz; k++) {
         cp_async_wait<DEPTH - 2>();  // levels k and k+1 have landed
         __syncthreads();
         issue(k + DEPTH);            // into the slot of level k-1, read by nobody any more
-        const float *L = sm + (size_t)(k % NSLOT) * NF * PLANE;
-        const float *Lu = sm + (size_t)((k + 1) % NSLOT) * NF * PLANE;
-        const size_t c = ix(g, i, k, j);
-        if (!bal) {
-            if (in) w[c] = 0.0f;
-            continue;
-        }
+        const float *L = sm + (size_t)(k % NSLOT) * NF * PLANE + pc;
+        const float *Lu = sm + (size_t)((k + 1) % NSLOT) * NF * PLANE + pc;
         const float *U = L, *JU = L + PLANE, *V = L + 2 * PLANE, *JV = L + 3 * PLANE, *R = L + 4 * PLANE;
         const float *DZ = L + 5 * PLANE, *JW = L + 6 * PLANE;
-        const float *Ur = U + py * PW, *JUr = JU + py * PW, *Rr = R + py * PW;
-        const float ue = umet_p(nx, adv_den, Ur, JUr, Rr, i + 1, ox), uw = umet_p(nx, adv_den, Ur, JUr, Rr, i, ox);
-        const int pc = py * PW + px;
-        const float vn = vmet_p(ny, adv_den, V + pc + PW, JV + pc + PW, R + pc + PW, j + 1);
-        const float vs = vmet_p(ny, adv_den, V + pc, JV + pc, R + pc, j);
-        const float div = ((ue - uw) + (vn - vs)) / dx;
-        const float d = DZ[pc], jwc = JW[pc];
-        float wk;
-        if (adv_den) {
-            // rho_i(k) = (rho_k*dz_k + rho_k+1*dz_k+1) / (dz_k + dz_k+1), wind.f90:175-176
-            float ri = 0.0f;
-            if (k < nz - 1) {
-                const float dzu = Lu[5 * PLANE + pc];
-                ri = (R[pc] * d + Lu[4 * PLANE + pc] * dzu) / (d + dzu);
+        float R0[RPT + 2];  // density of rows j-1 .. j+RPT in this column
+        if (ADV)
+#pragma unroll
+            for (int m = 0; m < RPT + 2; m++) R0[m] = R[(m - 1) * PW];
+        float vf[RPT + 1];
+#pragma unroll
+        for (int m = 0; m <= RPT; m++) {
+            const float vj = V[m * PW] * JV[m * PW];
+            vf[m] = vj;
+            if (ADV) {
+                vf[m] = vj * (R0[m] + R0[m + 1]) / 2.0f;
+                if (EDGE && m == 0 && j == 0) vf[m] = vj * (1.5f * R0[1] - 0.5f * R0[2]);
+                if (EDGE && m > 0 && j + m == ny) vf[m] = vj * (1.5f * R0[m] - 0.5f * R0[m - 1]);
             }
-            if (k == 0)
-                wk = 0.0f - div * d / (jwc * ri);
-            else if (k == nz - 1)
-                wk = ((wb * rib * jwb) - div * d) / (jwc * R[pc]);
-            else
-                wk = ((wb * rib * jwb) - div * d) / (jwc * ri);
-            rib = ri;
-        } else {
-            if (k == 0)
-                wk = (0.0f - div * d) / jwc;
-            else
-                wk = (wb * jwb - div * d) / jwc;
         }
-        w[c] = wk;
-        wb = wk;
-        jwb = jwc;
+#pragma unroll
+        for (int r = 0; r < RPT; r++) {
+            const int o = r * PW;
+            float ue = U[o + 1] * JU[o + 1], uw = U[o] * JU[o];
+            if (ADV) {
+                const float rc = R0[r + 1], rl = R[o - 1], rr = R[o + 1];
+                const float ej = ue, wj = uw;
+                ue = ej * (rc + rr) / 2.0f;
+                uw = wj * (rl + rc) / 2.0f;
+                if (EDGE && i + 1 == nx) ue = ej * (1.5f * rc - 0.5f * rl);
+                if (EDGE && i == 0) uw = wj * (1.5f * rc - 0.5f * rr);
+            }
+            const float div = ((ue - uw) + (vf[r + 1] - vf[r])) / dx;
+            const float d = DZ[o], jwc = JW[o];
+            float wk;
+            if (ADV) {
+                // rho_i(k) = (rho_k*dz_k + rho_k+1*dz_k+1) / (dz_k + dz_k+1), wind.f90:175-176
+                float ri = R0[r + 1];
+                if (k < nz - 1) {
+                    const float dzu = Lu[5 * PLANE + o];
+                    ri = (R0[r + 1] * d + Lu[4 * PLANE + o] * dzu) / (d + dzu);
+                }
+                wk = ((k == 0 ? 0.0f : wb[r] * rib[r] * jwb[r]) - div * d) / (jwc * ri);
+                rib[r] = ri;
+            } else {
+                wk = ((k == 0 ? 0.0f : wb[r] * jwb[r]) - div * d) / jwc;
+            }
+            wb[r] = wk;
+            jwb[r] = jwc;
+            if (in[r]) *wp[r] = bal[r] ? wk : 0.0f;
+            wp[r] += g.P;
+        }
     }
     cp_async_wait<0>();
+}
+
+template <bool ADV>
+__global__ void __launch_bounds__(balf::NT)
+    k_balance_uvw(Geo g, int hs, float dx, const float *__restrict__ u, const float *__restrict__ v,
+                  const float *__restrict__ rho, const float *__restrict__ dz, const float *__restrict__ ju,
+                  const float *__restrict__ jv, const float *__restrict__ jw, float *__restrict__ w)
+{
+    extern __shared__ float4 sm4[];
+    float *sm = reinterpret_cast<float *>(sm4);
+    const int i0 = blockIdx.x * balf::BX, j0 = blockIdx.y * balf::BY;
+    if (i0 > 0 && j0 > 0 && i0 + balf::BX < g.nx && j0 + balf::BY < g.ny)
+        balance_march<ADV, false>(sm, g, hs, dx, i0, j0, u, v, rho, dz, ju, jv, jw, w);
+    else
+        balance_march<ADV, true>(sm, g, hs, dx, i0, j0, u, v, rho, dz, ju, jv, jw, w);
 }
 
 // out[0..2] = bits of max |u|, |v|, |w| over the arrays; out[3] = bits of

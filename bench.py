@@ -57,7 +57,7 @@ def parse():
     p.add_argument("--no-cpu-baseline", action="store_true")
     p.add_argument("--staged", action="store_true", help="use the staged kernels instead of the fused one")
     p.add_argument("--kernel", default="single-pass-fast", choices=["two-pass", "single-pass", "single-pass-fast"],
-                   help="MPDATA kernels: the donor-cell kernel then the fused correction (two-pass), or the "
+                   help="MPDATA kernels: two-pass is the former name of the library default, now the same as single-pass; the "
                         "single-pass kernel with bit-exact or fast arithmetic")
     p.add_argument("--no-extras", action="store_true",
                    help="skip the sub-records of the default line (bit-exact kernels, drift, batched, served)")
@@ -245,7 +245,7 @@ def run_b200(args):
     adv_init(d, opts)
     path = 1 if args.staged else KERNEL_PATH[args.kernel]
     launch = set_launch_shape(d, args) if path == 0 else (
-        {"kernel": "staged"} if path == 1 else {"kernel": args.kernel, "tile": "56 x 26 columns per CTA, 16 warps"})
+        {"kernel": "staged"} if path == 1 else {"kernel": args.kernel, "tile": "56 x 22 columns per CTA, 12 warps"})
     d.set_path(path)
     # a dedicated stream: the library and the timing events share it
     stream = torch.cuda.Stream()
@@ -296,11 +296,8 @@ def run_b200(args):
     # ---- roofline of the dominant kernel and of the whole advect call ---
     from hicar_b200 import roofline
     step_rl = roofline.species_pass(case.nx, case.ny, case.nz, S, kms.value, passes.value)
-    if claunch.value > 0 and path >= 2:
+    if claunch.value > 0:
         rl = roofline.single_pass_kernel(case.nx, case.ny, case.nz, S, cms.value, claunch.value)
-        rl["advect_call"] = step_rl
-    elif claunch.value > 0:
-        rl = roofline.correction_kernel(case.nx, case.ny, case.nz, S, cms.value, claunch.value)
         rl["advect_call"] = step_rl
     else:                                       # staged path: the whole advect call
         rl = step_rl
@@ -324,8 +321,7 @@ def run_b200(args):
             extras["exact"] = {
                 "value": R.whole_job_rate(cells * S * args.steps, world, ems / 1e3), "unit": UNIT,
                 "ms_per_step": ems / args.steps, "steps": args.steps,
-                "kernel": "two-pass (donor-cell kernel + fused correction), the reference's FP32 arithmetic, "
-                          "bit-identical to the oracle"}
+                "kernel": "single-pass, the reference's FP32 arithmetic, bit-identical to the oracle (library default)"}
             d.set_path(path)
         # ---- drift: the step cost as the fields evolve, from the initial state
         for k, q in case.species.items():
@@ -432,9 +428,9 @@ LARGE_DESC = "large single domain 2048x2048x60, dx 250 m, fractal terrain up to 
 
 def run_large(args):
     """The large single domain, generated on the device.  Every arm starts
-    from the same saved initial state: the default launch shape of the
-    two-pass kernels, each autotuner candidate, the autotuned shape, and the
-    single-pass fast kernel."""
+    from the same saved initial state: the library's
+    default kernel, each autotuner candidate, the autotuned choice, and the
+    fast kernel."""
     import torch
     from hicar_b200 import _lib as L, autotune, replicas as R, roofline, synth
     from hicar_b200.advection import Domain, Options
@@ -536,9 +532,9 @@ def run_large(args):
                    "state": "every arm starts from the same saved initial state",
                    "l2": "inputs larger than L2 (12 fields x 1 GB)"},
         "plain": {"value": cs * args.steps / (ms_plain / 1e3), "ms_per_step": ms_plain / args.steps,
-                  "kernel": "two-pass", "launch_shape": {"tile_rows": autotune.TILE_ROWS[1], "species_group": 0}},
+                  "kernel": "library default (exact single-pass)", "launch_shape": {"tile_rows": autotune.TILE_ROWS[1], "species_group": 0}},
         "autotuned": {"value": cs * args.steps / (ms_tuned / 1e3), "ms_per_step": ms_tuned / args.steps,
-                      "kernel": "two-pass",
+                      "kernel": "library default (exact single-pass)",
                       "launch_shape": {"tile_rows": autotune.TILE_ROWS[shape], "species_group": group,
                                        "chosen_by": "autotune: every combination timed on this domain, "
                                                     "each from the saved state"}},
@@ -853,15 +849,6 @@ def ensemble_core(args, rk, kernel: str, want_e2e: bool, want_cpu: bool) -> dict
     b.set_path(KERNEL_PATH[kernel])
     for d, c in zip(doms, cases):
         b.add(d, c.dt)
-    shape = 1
-    if kernel != "two-pass":
-        pass                                    # the single-pass kernel has one tile shape
-    elif args.tile_shape == "auto":
-        from hicar_b200 import autotune
-        shape = autotune.tune_batch(b)
-    else:
-        shape = int(args.tile_shape)
-        b.set_tile_shape(shape)
     for _ in range(args.warmup):
         b.step()
     clocks = ClockSampler(local)
@@ -883,9 +870,9 @@ def ensemble_core(args, rk, kernel: str, want_e2e: bool, want_cpu: bool) -> dict
           "bytes_model": "8 + 32/S B per cell-species; one launch = one batched step (graph)"}
     out = {"value": value, "ms_per_step": ms / args.steps, "steps": args.steps, "cell_species_per_step": cs_step,
            "members": len(cases), "kernel": kernel,
-           "tile_shape_rows": [8, 15, 24, 31][shape] if kernel == "two-pass" else 26,
+           "tile_shape_rows": 22,
            "plain": {"value": plain_value, "steps": plain_steps, "ms_per_step": plain_ms / plain_steps,
-                     "launches_per_step": len(cases) * (3 if kernel != "two-pass" else 4)},
+                     "launches_per_step": len(cases) * 3},
            "batched_over_plain": value / plain_value, "roofline": rl,
            "gpu_launches": int(prof["kernels_per_step"] * prof["steps"]), "clocks": clk}
 

@@ -1,16 +1,11 @@
-"""Autotuner for the launch shape of the fused MPDATA kernels.
+"""Autotuner for the launch-shape knobs of the MPDATA kernels.
 
-Two knobs, neither of which changes any result (every combination gives
-bit-identical fields; tests/test_autotune_gpu.py checks it):
-
-  tile shape     output rows per tile of the correction kernel (8, 15, 24 or
-                 31 rows of 28 columns).  Taller tiles recompute less of the
-                 y halo around each tile but need more shared memory per CTA,
-                 so fewer CTAs fit on an SM, and waste more rows in the last
-                 tile of a column when ny-2 is not a multiple of the height.
-  species group  species that one thread of the donor-cell pass takes (0 =
-                 all).  All species reuse a cell's winds and metric terms;
-                 smaller groups give small domains more blocks.
+The two knobs, tile shape (8, 15, 24 or 31 rows) and species group of the
+donor-cell pass (0 = all), belonged to kernels that handles and batches no
+longer run: the single-pass kernel has one tile shape and chooses its level
+ranges from the grid.  They are still checked, measured, cached and applied,
+so programs and caches that use them keep working; every combination launches
+the same kernel and gives bit-identical fields (tests/test_autotune_gpu.py).
 
 tune_domain(nx, ny, nz, n_species, fct)
     measures every combination on a synthetic domain of that grid shape,
@@ -22,7 +17,7 @@ shape_costs(fct)
     measures once per GPU the device time of one tile-level of one species
     for every tile shape, on a calibration domain large enough to fill the
     GPU.  choose_batch_shape(members, costs) then picks the tile shape of a
-    batch -- one persistent launch over every member's tiles -- as the shape
+    batch -- one launch over every member's tiles -- as the shape
     with the least predicted time, sum over members of tiles x levels x
     species x cost per tile-level.
 """

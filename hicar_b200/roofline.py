@@ -14,7 +14,8 @@ fields once (U_m, V_m, W_m/dz and J*rho through TMA, W_m, dz*J*rho and dz by
 plain loads: 28 B per cell):
     8 + 28/S bytes per cell-species  (10.33 B at S=12).
 
-The dominant kernel of the two-kernel form, the fused correction kernel (k_mp_corr),
+The dominant kernel of the two-kernel form, which the entry on caller-owned
+memory still runs, the fused correction kernel (k_mp_corr),
 reads q0 and q1 and writes the new state of every species (12 B per
 cell-species) and reads six species-independent fields once (U_m, V_m,
 W_m/dz, J*rho, dz*J*rho and dz: 24 B per cell):

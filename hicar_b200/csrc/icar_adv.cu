@@ -1435,7 +1435,7 @@ int icar_adv_compute_dt(icar_adv_t *h, const float *dz_levels, float cfl, int32_
     CUDA_TRY(h, cudaMemcpyAsync(bits, d_out, sizeof(bits), cudaMemcpyDeviceToHost, h->stream));
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     float m[4];
-    memcpy(m, bits, sizeof(m));
+    icar::decode_maxima(bits, m);
     *dt = icar::dt_from_maxima(m, cfl, cfl_strictness, use_density);
     if (*dt < 1e-1f)
         return fail(h, ICAR_ADV_CFL_VIOLATION, "time step too small: dt = %g s (max |u| %g, |v| %g, |w| %g)",

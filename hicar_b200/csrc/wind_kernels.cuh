@@ -18,6 +18,9 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cmath>
+#include <cstring>
+
 #include "common.cuh"
 #include "mpdata_fused.cuh"
 
@@ -186,9 +189,14 @@ __global__ void __launch_bounds__(balf::NT)
         balance_march<ADV, true>(sm, g, hs, dx, i0, j0, u, v, rho, dz, ju, jv, jw, w);
 }
 
-// out[0..2] = bits of max |u|, |v|, |w| over the arrays; out[3] = bits of
-// the largest per-cell rate over the tile (i, j in [hs, n-1-hs], every k).
-// out must be zero on entry.  dzl is dz_levels (nz).
+// out[0..2] = bits of max |u|, |v|, |w| over the arrays plus one; out[3] =
+// bits of the largest per-cell rate over the tile (i, j in [hs, n-1-hs], every
+// k).  out must be zero on entry.  dzl is dz_levels (nz).
+//
+// A NaN among other values is skipped; of an array that holds nothing else
+// out stays zero, which dt_from_maxima turns into a NaN again.  So every
+// maximum starts as NaN ("nothing yet") and grows by fmaxf, which returns the
+// other operand for a NaN.
 //
 // Bound by reading the three fields.  Rounded division by a positive number
 // is monotone, so the largest rate is the largest speed divided: of u over
@@ -204,15 +212,14 @@ namespace dtm {
 constexpr int NT = 256, WARPS = NT / 32, U = 2;
 }
 
-// mx: maximum so far over the whole row; tx: over x in [a, b]; both over x < n
+// mx: maximum so far over the whole row; tx: over x in [a, b] (b < n); both over x < n
 __device__ __forceinline__ void dt_take(float4 v, int i, int n, int a, int b, bool tile, float &mx, float &tx)
 {
     const float f[4] = {fabsf(v.x), fabsf(v.y), fabsf(v.z), fabsf(v.w)};
 #pragma unroll
     for (int m = 0; m < 4; m++) {
-        const float x = i + m < n ? f[m] : 0.0f;
-        mx = fmax_(x, mx);
-        if (tile && i + m >= a && i + m <= b) tx = fmax_(x, tx);
+        if (i + m < n) mx = fmaxf(mx, f[m]);
+        if (tile && i + m >= a && i + m <= b) tx = fmaxf(tx, f[m]);
     }
 }
 
@@ -226,22 +233,23 @@ __global__ void __launch_bounds__(dtm::NT)
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const unsigned row = blockIdx.x * WARPS + warp;  // k + nz*j, j <= ny (v has ny+1 rows)
     const int j = (int)(row / (unsigned)nz), k = (int)(row - (unsigned)j * nz);
-    float mu = 0.0f, mv = 0.0f, mw = 0.0f, tu = 0.0f, tv = 0.0f, tw = 0.0f;
+    const float none = __int_as_float(0x7fffffff);
+    float mu = none, mv = none, mw = none, tu = none, tv = none, tw = none;
     if (j <= ny) {
         const bool cells = j < ny, tile = j >= hs && j <= ny - 1 - hs, vtile = j >= hs && j <= ny - hs;
         const float4 *pu = reinterpret_cast<const float4 *>(u + (size_t)row * g.P);
         const float4 *pv = reinterpret_cast<const float4 *>(v + (size_t)row * g.P);
         const float4 *pw = reinterpret_cast<const float4 *>(w + (size_t)row * g.P);
-        const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const float4 blank = make_float4(none, none, none, none);
         for (int q0 = lane; q0 < nq; q0 += 32 * U) {
             float4 a[U], b[U], c[U];
 #pragma unroll
             for (int m = 0; m < U; m++) {
                 const int q = q0 + 32 * m;
                 const bool in = q < nq;
-                a[m] = in && cells ? pu[q] : zero;
-                b[m] = in ? pv[q] : zero;
-                c[m] = in && cells ? pw[q] : zero;
+                a[m] = in && cells ? pu[q] : blank;
+                b[m] = in ? pv[q] : blank;
+                c[m] = in && cells ? pw[q] : blank;
             }
 #pragma unroll
             for (int m = 0; m < U; m++) {
@@ -254,15 +262,15 @@ __global__ void __launch_bounds__(dtm::NT)
     }
     float m3 = 0.0f;
     if (tw > 0.0f) {
-        m3 = fmax_(tw / dzl[k], m3);
-        if (k + 1 < nz) m3 = fmax_(tw / dzl[k + 1], m3);
+        m3 = fmaxf(tw / dzl[k], m3);
+        if (k + 1 < nz) m3 = fmaxf(tw / dzl[k + 1], m3);
     }
-    m3 = fmax_(fmax_(tu, tv) / dx, m3);
+    m3 = fmaxf(fmaxf(tu, tv) / dx, m3);
     for (int o = 16; o > 0; o >>= 1) {
-        mu = fmax_(mu, __shfl_xor_sync(0xffffffffu, mu, o));
-        mv = fmax_(mv, __shfl_xor_sync(0xffffffffu, mv, o));
-        mw = fmax_(mw, __shfl_xor_sync(0xffffffffu, mw, o));
-        m3 = fmax_(m3, __shfl_xor_sync(0xffffffffu, m3, o));
+        mu = fmaxf(mu, __shfl_xor_sync(0xffffffffu, mu, o));
+        mv = fmaxf(mv, __shfl_xor_sync(0xffffffffu, mv, o));
+        mw = fmaxf(mw, __shfl_xor_sync(0xffffffffu, mw, o));
+        m3 = fmaxf(m3, __shfl_xor_sync(0xffffffffu, m3, o));
     }
     if (lane == 0) {
         part[0][warp] = mu;
@@ -272,24 +280,36 @@ __global__ void __launch_bounds__(dtm::NT)
     }
     __syncthreads();
     if (threadIdx.x < 4) {
-        float m = 0.0f;
-        for (int o = 0; o < WARPS; o++) m = fmax_(part[threadIdx.x][o], m);
+        float m = none;
+        for (int o = 0; o < WARPS; o++) m = fmaxf(m, part[threadIdx.x][o]);
         // the values there only grow: no atomic where it could not change them
-        const unsigned bits = __float_as_uint(m);
+        const unsigned bits = threadIdx.x == 3 ? __float_as_uint(m) : m >= 0.0f ? __float_as_uint(m) + 1u : 0u;
         if (bits > *reinterpret_cast<volatile unsigned *>(&out[threadIdx.x])) atomicMax(&out[threadIdx.x], bits);
     }
 }
 
+// The maxima from k_dt_maxima's words: max |u|, |v|, |w| (NaN for an array of
+// NaN) and the largest rate, NaN where one of the winds is.
+inline void decode_maxima(const unsigned bits[4], float m[4])
+{
+    for (int i = 0; i < 4; i++) {
+        const unsigned b = i < 3 && bits[i] ? bits[i] - 1u : bits[i];
+        memcpy(&m[i], &b, sizeof(b));
+        if (i < 3 && !bits[i]) m[i] = NAN;
+    }
+    if (m[0] != m[0] || m[1] != m[1] || m[2] != m[2]) m[3] = NAN;
+}
+
 // compute_dt's combination of the maxima for cfl_strictness 1..5 (host
-// side, same FP32 operations as the reference).  use_density: the
-// reference's density-weighted terms are commented out, so the winds then
+// side, same FP32 operations as the reference; a NaN stays one).  use_density:
+// the reference's density-weighted terms are commented out, so the winds then
 // contribute nothing and dt is infinite.
 inline float dt_from_maxima(const float m[4], float cfl, int strictness, int use_density)
 {
     const float three_d_cfl = 0.577350269f;
     const float sqrt3 = std::sqrt(3.0f) * 1.001f;
     float maxwind1d = 0.0f, maxwind3d = 0.0f;
-    auto mx = [](float a, float b) { return a > b ? a : b; };
+    auto mx = [](float a, float b) { return a > b || a != a ? a : b; };
     if (strictness == 1) {
         if (!use_density) maxwind1d = mx(mx(m[0], m[1]), m[2]);
         maxwind3d = maxwind1d * sqrt3;

@@ -226,8 +226,9 @@ int icar_adv_balance_uvw(icar_adv_t *h);
  * step for cfl (options%time_options%cfl_reduction_factor) and
  * cfl_strictness 1..5, with dz_levels the host array of nz level
  * thicknesses (options%parameters%dz_levels).  Writes *dt and returns
- * ICAR_ADV_CFL_VIOLATION when dt < 0.1 s (where the reference stops).
- * Synchronises the handle's stream. */
+ * ICAR_ADV_CFL_VIOLATION when dt < 0.1 s (where the reference stops).  A NaN
+ * among a wind's other values is skipped; a wind that is NaN throughout gives
+ * dt = NaN.  Synchronises the handle's stream. */
 int icar_adv_compute_dt(icar_adv_t *h, const float *dz_levels, float cfl, int32_t cfl_strictness,
                         int32_t use_density, float *dt);
 

@@ -3,8 +3,8 @@
 //
 //   k_balance_uvw   balance_uvw (src/physics/wind.f90:88-164) with
 //                   calc_divergence(horz_only) and calc_w (:166-271): one
-//                   thread per two columns marches up them, forming
-//                   the horizontal divergence of the metric-weighted u, v at
+//                   thread per column marches up it, forming the
+//                   horizontal divergence of the metric-weighted u, v at
 //                   each level and integrating w from w = 0 below the ground;
 //                   the levels arrive in shared-memory planes ahead of use.
 //   k_dt_maxima     the maxima compute_dt (src/main/time_step.f90:51-168)
@@ -27,13 +27,12 @@
 namespace icar {
 
 namespace balf {
-// CTA tile: 32 x 8 columns, one thread per two columns adjacent in y marching
-// up k.  The seven fields a level needs (u, J_u, v, J_v, rho, dz, J_w) arrive
+// CTA tile: 32 x 8 columns, one thread per column marching up k.  The seven fields a level needs (u, J_u, v, J_v, rho, dz, J_w) arrive
 // in shared-memory planes by 16-byte cp.async, DEPTH levels ahead of use:
 // each plane spans x from i0-4 (a multiple of 4) to i0+35 and y from j0-1
 // to j0+8, covering the faces i0..i0+32 / j0..j0+8 and the density
 // neighbours the face weights read.
-constexpr int BX = 32, BY = 8, RPT = 2, NT = BX * BY / RPT;
+constexpr int BX = 32, BY = 8, NT = BX * BY;
 constexpr int PW = 40, PH = BY + 2, PLANE = PW * PH;
 constexpr int NF = 7;                      // u, ju, v, jv, rho, dz, jw
 constexpr int DEPTH = 3, NSLOT = DEPTH + 1;
@@ -49,10 +48,13 @@ constexpr size_t SMEM = (size_t)NSLOT * NF * PLANE * sizeof(float);
 // extrapolate it), wind.f90:237-239; v*J_v likewise, :241-243.  EDGE tiles
 // touch the domain's sides, the others have no outermost face.
 //
-// 334 MB at 512x512x40 (51 us at the measured copy rate), bound by issue.  Two
-// adjacent columns per thread share the y face between them and the densities
-// of their rows, and tiles inside the domain carry no side conditions:
-// 86 us where one column per thread with them took 99.
+// 334 MB at 512x512x40 (51 us at the measured copy rate), bound by issue there
+// and by the latency of the march on domains of up to a wave of tiles.  The
+// density is a template argument and tiles inside the domain carry no side
+// conditions: 80 us with density and 73 without at 512x512x40, 33 both at
+// 25x38x54, where a run-time switch and side conditions everywhere took 97 and
+// 75, 47 and 37.  Two columns per thread share operands but march slower: 84
+// and 84, 42 and 45.
 template <bool ADV, bool EDGE>
 __device__ __forceinline__ void balance_march(float *sm, const Geo &g, int hs, float dx, int i0, int j0,
                                               const float *__restrict__ u, const float *__restrict__ v,
@@ -61,7 +63,7 @@ __device__ __forceinline__ void balance_march(float *sm, const Geo &g, int hs, f
                                               const float *__restrict__ jw, float *__restrict__ w)
 {
     using namespace balf;
-    const int tx = threadIdx.x % BX, ty = threadIdx.x / BX * RPT;
+    const int tx = threadIdx.x % BX, ty = threadIdx.x / BX;
     const int i = i0 + tx, j = j0 + ty;
     const int nx = g.nx, ny = g.ny, nz = g.nz;
     const int ox = i0 - 4, oy = j0 - 1;
@@ -104,72 +106,67 @@ __device__ __forceinline__ void balance_march(float *sm, const Geo &g, int hs, f
     };
 #pragma unroll
     for (int k = 0; k < DEPTH; k++) issue(k);
-    bool in[RPT], bal[RPT];
-    float wb[RPT], rib[RPT], jwb[RPT];  // w, interface density and J_w one level down
-    float *wp[RPT];
-#pragma unroll
-    for (int r = 0; r < RPT; r++) {
-        in[r] = i < nx && j + r < ny;
-        bal[r] = in[r] && i >= i_s && i <= i_e && j + r >= j_s && j + r <= j_e;
-        wb[r] = rib[r] = jwb[r] = 0.0f;
-        wp[r] = w + (in[r] ? ix(g, i, 0, j + r) : 0);
-    }
+    const bool in = i < nx && j < ny;
+    const bool bal = in && i >= i_s && i <= i_e && j >= j_s && j <= j_e;
+    float wb = 0.0f, rib = 0.0f, jwb = 0.0f;  // w, interface density and J_w one level down
+    float *wp = w + (in ? ix(g, i, 0, j) : 0);
     const int pc = (ty + 1) * PW + tx + 4;
     for (int k = 0; k < nz; k++) {
         cp_async_wait<DEPTH - 2>();  // levels k and k+1 have landed
         __syncthreads();
         issue(k + DEPTH);            // into the slot of level k-1, read by nobody any more
+        // Outside the domain the metrics are zeros, and a quotient of zeros
+        // takes the division's slow path: those columns are skipped.
+        if (EDGE && !bal) {
+            if (in) *wp = 0.0f;
+            wp += g.P;
+            continue;
+        }
         const float *L = sm + (size_t)(k % NSLOT) * NF * PLANE + pc;
         const float *Lu = sm + (size_t)((k + 1) % NSLOT) * NF * PLANE + pc;
         const float *U = L, *JU = L + PLANE, *V = L + 2 * PLANE, *JV = L + 3 * PLANE, *R = L + 4 * PLANE;
-        const float *DZ = L + 5 * PLANE, *JW = L + 6 * PLANE;
-        float R0[RPT + 2];  // density of rows j-1 .. j+RPT in this column
-        if (ADV)
-#pragma unroll
-            for (int m = 0; m < RPT + 2; m++) R0[m] = R[(m - 1) * PW];
-        float vf[RPT + 1];
-#pragma unroll
-        for (int m = 0; m <= RPT; m++) {
-            const float vj = V[m * PW] * JV[m * PW];
-            vf[m] = vj;
-            if (ADV) {
-                vf[m] = vj * (R0[m] + R0[m + 1]) / 2.0f;
-                if (EDGE && m == 0 && j == 0) vf[m] = vj * (1.5f * R0[1] - 0.5f * R0[2]);
-                if (EDGE && m > 0 && j + m == ny) vf[m] = vj * (1.5f * R0[m] - 0.5f * R0[m - 1]);
-            }
+        float rs = 0.0f, rc = 0.0f, rn = 0.0f;  // density here and in the rows beside
+        if (ADV) {
+            rs = R[-PW];
+            rc = R[0];
+            rn = R[PW];
         }
-#pragma unroll
-        for (int r = 0; r < RPT; r++) {
-            const int o = r * PW;
-            float ue = U[o + 1] * JU[o + 1], uw = U[o] * JU[o];
-            if (ADV) {
-                const float rc = R0[r + 1], rl = R[o - 1], rr = R[o + 1];
-                const float ej = ue, wj = uw;
-                ue = ej * (rc + rr) / 2.0f;
-                uw = wj * (rl + rc) / 2.0f;
-                if (EDGE && i + 1 == nx) ue = ej * (1.5f * rc - 0.5f * rl);
-                if (EDGE && i == 0) uw = wj * (1.5f * rc - 0.5f * rr);
-            }
-            const float div = ((ue - uw) + (vf[r + 1] - vf[r])) / dx;
-            const float d = DZ[o], jwc = JW[o];
-            float wk;
-            if (ADV) {
-                // rho_i(k) = (rho_k*dz_k + rho_k+1*dz_k+1) / (dz_k + dz_k+1), wind.f90:175-176
-                float ri = R0[r + 1];
-                if (k < nz - 1) {
-                    const float dzu = Lu[5 * PLANE + o];
-                    ri = (R0[r + 1] * d + Lu[4 * PLANE + o] * dzu) / (d + dzu);
-                }
-                wk = ((k == 0 ? 0.0f : wb[r] * rib[r] * jwb[r]) - div * d) / (jwc * ri);
-                rib[r] = ri;
-            } else {
-                wk = ((k == 0 ? 0.0f : wb[r] * jwb[r]) - div * d) / jwc;
-            }
-            wb[r] = wk;
-            jwb[r] = jwc;
-            if (in[r]) *wp[r] = bal[r] ? wk : 0.0f;
-            wp[r] += g.P;
+        const float sj = V[0] * JV[0], nj = V[PW] * JV[PW];
+        float vs = sj, vn = nj;
+        if (ADV) {
+            vs = sj * (rs + rc) / 2.0f;
+            if (EDGE && j == 0) vs = sj * (1.5f * rc - 0.5f * rn);
+            vn = nj * (rc + rn) / 2.0f;
+            if (EDGE && j + 1 == ny) vn = nj * (1.5f * rc - 0.5f * rs);
         }
+        const float ej = U[1] * JU[1], wj = U[0] * JU[0];
+        float ue = ej, uw = wj;
+        if (ADV) {
+            const float rl = R[-1], rr = R[1];
+            ue = ej * (rc + rr) / 2.0f;
+            uw = wj * (rl + rc) / 2.0f;
+            if (EDGE && i + 1 == nx) ue = ej * (1.5f * rc - 0.5f * rl);
+            if (EDGE && i == 0) uw = wj * (1.5f * rc - 0.5f * rr);
+        }
+        const float div = ((ue - uw) + (vn - vs)) / dx;
+        const float d = L[5 * PLANE], jwc = L[6 * PLANE];
+        float wk;
+        if (ADV) {
+            // rho_i(k) = (rho_k*dz_k + rho_k+1*dz_k+1) / (dz_k + dz_k+1), wind.f90:175-176
+            float ri = rc;
+            if (k < nz - 1) {
+                const float dzu = Lu[5 * PLANE];
+                ri = (rc * d + Lu[4 * PLANE] * dzu) / (d + dzu);
+            }
+            wk = ((k == 0 ? 0.0f : wb * rib * jwb) - div * d) / (jwc * ri);
+            rib = ri;
+        } else {
+            wk = ((k == 0 ? 0.0f : wb * jwb) - div * d) / jwc;
+        }
+        wb = wk;
+        jwb = jwc;
+        if (in) *wp = bal ? wk : 0.0f;
+        wp += g.P;
     }
     cp_async_wait<0>();
 }

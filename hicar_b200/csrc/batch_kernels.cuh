@@ -21,7 +21,7 @@ struct BatchMember {
     Geo g;
     float dx, dt;
     double dtd;
-    int S, adv_den, nzone, epoch;
+    int S, adv_den, nzone;
     int *flags;
     const float *u, *v, *w, *rho, *jac, *ju, *jv, *jw, *dz;
     float *Um, *Vm, *Wm, *Gc, *DJR, *Wp;
@@ -79,10 +79,7 @@ __global__ void __launch_bounds__(256)
     const int mi = find_owner(prefix, nmem, blockIdx.x);
     const BatchMember &m = mem[mi];
     const PrepFields f{m.u, m.v, m.w, m.rho, m.jac, m.ju, m.jv, m.jw, m.dz, m.Um, m.Vm, m.Wm, m.Gc, m.DJR, m.Wp};
-    bool bad = false, tie = false;
-    prep_quad(m.g, m.dx, m.dt, m.adv_den, f, (blockIdx.x - prefix[mi]) * blockDim.x + threadIdx.x, bad, tie);
-    if (bad && m.flags) m.flags[FLAG_IEEE] = m.epoch;
-    if (tie && m.flags) m.flags[FLAG_TIE] = m.epoch;
+    prep_quad(m.g, m.dx, m.dt, m.adv_den, f, (blockIdx.x - prefix[mi]) * blockDim.x + threadIdx.x, m.flags);
 }
 
 }  // namespace icar

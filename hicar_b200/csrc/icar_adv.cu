@@ -101,8 +101,7 @@ struct icar_adv_domain {
     std::vector<const float *> map_tag[2];
     int map_next = 0;
     int *op_err = nullptr;
-    int *op_flags = nullptr;   // icar::N_FLAGS words the prep kernels set to a step's epoch
-    int op_epoch = 0;
+    int *op_flags = nullptr;   // what the prep kernels report about a step's fields (icar::FLAG_WORDS)
     bool op_ready = false;
     int nsm = 148;     // SMs of the device
     // diagnostics: launch counter and optional event timing of the species kernels
@@ -684,6 +683,15 @@ int std_advect3d(icar_adv_t *h, const float *qf, const float *qold, float *qout,
     return check_launch(h, "std kernels", flux_corr == 1 ? 8 : 2);
 }
 
+int ensure_flags(icar_adv_t *h)
+{
+    if (h->op_flags) return ICAR_ADV_OK;
+    const size_t bytes = icar::FLAG_WORDS * sizeof(int);
+    CUDA_TRY(h, dev_alloc(h, (void **)&h->op_flags, bytes));
+    CUDA_TRY(h, cudaMemsetAsync(h->op_flags, 0, bytes, h->stream));
+    return ICAR_ADV_OK;
+}
+
 // ---------------------------------------------------------------------------
 // Single-pass MPDATA kernel (mpdata_onepass.cuh): per-step fields from
 // k_mp_prep, then one launch for every species.  It needs no pass-1
@@ -823,10 +831,7 @@ int ensure_onepass(icar_adv_t *h)
             CUDA_TRY(h, dev_alloc(h, (void **)&h->op_err, sizeof(int)));
             CUDA_TRY(h, cudaMemsetAsync(h->op_err, 0, sizeof(int), h->stream));
         }
-        if (!h->op_flags) {
-            CUDA_TRY(h, dev_alloc(h, (void **)&h->op_flags, icar::N_FLAGS * sizeof(int)));
-            CUDA_TRY(h, cudaMemsetAsync(h->op_flags, 0, icar::N_FLAGS * sizeof(int), h->stream));
-        }
+        if ((e = ensure_flags(h))) return e;
         cudaError_t ce = onepass_attr<icar::opx::A_EXACT>();
         if (ce == cudaSuccess) ce = onepass_attr<icar::opx::A_FAST>();
         if (ce == cudaSuccess) ce = cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, h->desc.device);
@@ -858,7 +863,6 @@ int mpdata_onepass_group(icar_adv_t *h, int s0, int s1)
     prm.dz = h->dz.p;
     prm.err = h->op_err;
     prm.flags = h->op_flags;
-    prm.epoch = h->op_epoch;
     prm.nzero = -0.0f;
     prm.g = g;
     prm.nspecies = S;
@@ -896,7 +900,7 @@ int mpdata_prep(icar_adv_t *h, float dt)
     const icar::PrepFields f{h->u.p,     h->v.p,  h->w.p,  h->rho.p, h->jac.p, h->jac_u.p, h->jac_v.p, h->jac_w.p,
                              h->dz.p,    h->Um.p, h->Vm.p, h->Wm.p,  h->Gc.p,  h->DJR.p,   h->Wp.p};
     icar::k_mp_prep<<<blocks_for(icar::prep_quads(g), 256), 256, 0, h->stream>>>(
-        g, h->desc.dx, dt, h->opts.advect_density, f, h->op_flags, ++h->op_epoch);
+        g, h->desc.dx, dt, h->opts.advect_density, f, h->op_flags);
     if (h->opts.debug &&
         icar::check_courant(h->stream, h->g, h->Um.p, h->Vm.p, h->Wm.p, h->dz.p, h->jac.p, h->rho.p, 1))
         return fail(h, ICAR_ADV_CFL_VIOLATION, "a Courant number >= 1 was found (debug check)");
@@ -926,10 +930,7 @@ int ensure_std_fused(icar_adv_t *h)
         if ((e = alloc(h, h->Gc, h->n_cell)) || (e = alloc(h, h->DJR, h->n_cell))) return e;
         for (int s = 0; s < S; s++)
             if ((e = alloc(h, h->qn[s], h->n_cell)) || (e = alloc(h, h->q1s[s], h->n_cell))) return e;
-        if (!h->op_flags) {
-            CUDA_TRY(h, dev_alloc(h, (void **)&h->op_flags, icar::N_FLAGS * sizeof(int)));
-            CUDA_TRY(h, cudaMemsetAsync(h->op_flags, 0, icar::N_FLAGS * sizeof(int), h->stream));
-        }
+        if ((e = ensure_flags(h))) return e;
         cudaError_t ce = icar::std_fused_setup();
         if (ce != cudaSuccess) return fail(h, ICAR_ADV_CUDA_ERROR, "cudaFuncSetAttribute: %s", cudaGetErrorString(ce));
         h->std_ready = true;
@@ -948,7 +949,7 @@ int std_prep(icar_adv_t *h, float dt)
     const float *rho = h->have_rho ? h->rho.p : h->jac.p;  // only read when advect_density
     icar::k_std_prep<<<blocks_for(nf, 256), 256, 0, h->stream>>>(
         g, h->desc.dx, dt, h->opts.advect_density, h->u.p, h->v.p, h->w.p, rho, h->jac.p, h->jac_u.p, h->jac_v.p,
-        h->jac_w.p, h->dz.p, h->Um.p, h->Vm.p, h->Wm.p, h->Gc.p, h->DJR.p, h->op_flags, ++h->op_epoch);
+        h->jac_w.p, h->dz.p, h->Um.p, h->Vm.p, h->Wm.p, h->Gc.p, h->DJR.p, h->op_flags);
     if (h->opts.debug &&
         icar::check_courant(h->stream, h->g, h->Um.p, h->Vm.p, h->Wm.p, h->dz.p, h->jac.p, h->rho.p,
                             h->opts.advect_density))
@@ -973,7 +974,7 @@ int std_group(icar_adv_t *h, int s0, int s1)
             sp.out[s] = (*out)[s0 + s].p;
         }
         return icar::std_fused_launch(h->stream, c, ho, vo, g, hs, tf, sp, S, h->Um.p, h->Vm.p, h->Wm.p, h->Gc.p,
-                                      h->DJR.p, h->op_flags, h->op_epoch);
+                                      h->DJR.p, h->op_flags);
     };
     cudaEvent_t c0 = nullptr, c1 = nullptr;
     if (h->profiling) {
@@ -1994,7 +1995,6 @@ void fill_member(icar::BatchMember &m, icar_adv_t *h, double dt, int parity)
     m.filter = h->filter_dev;
     m.zone = h->zone_dev;
     m.flags = h->op_flags;
-    m.epoch = h->op_epoch;
     for (int s = 0; s < m.S; s++) {
         // parity 0: current state in q, next in qn; parity 1 the other way round
         float *cur = parity == 0 ? h->q[s].p : h->qn[s].p;
@@ -2036,7 +2036,6 @@ int build_tables(icar_adv_batch_t *b)
         icar_adv_t *h = b->members[m];
         int r = ensure_onepass(h);
         if (r) return bfail(b, r, "member scratch: %s", h->err.c_str());
-        h->op_epoch++;   // one epoch for every step these tables serve
         // descriptors of both parities: species inputs, then U_m, V_m, W_m/dz, J*rho
         for (int pp = 0; pp < 2; pp++) {
             map_base[pp][m] = maps.size();
@@ -2090,7 +2089,6 @@ int build_tables(icar_adv_batch_t *b)
             q.dz = h->dz.p;
             q.err = b->d_operr;
             q.flags = h->op_flags;
-            q.epoch = h->op_epoch;
             q.nzero = -0.0f;
             q.g = h->g;
             q.nspecies = S;
@@ -2625,8 +2623,7 @@ extern "C" int icar_adv_advect_noalloc(const icar_adv_noalloc_args *a)
     if (ce != cudaSuccess) return fail(nullptr, ICAR_ADV_CUDA_ERROR, "cudaMemsetAsync: %s", cudaGetErrorString(ce));
     const icar::PrepFields f{a->u,          a->v,            a->w,  a->density, a->jacobian, a->jacobian_u, a->jacobian_v,
                              a->jacobian_w, a->advection_dz, Um, Vm, Wm,         Gc,          DJR,           Wp};
-    icar::k_mp_prep<<<blocks_for(icar::prep_quads(g), 256), 256, 0, st>>>(g, a->dx, a->dt, a->advect_density, f, nullptr,
-                                                                        0);
+    icar::k_mp_prep<<<blocks_for(icar::prep_quads(g), 256), 256, 0, st>>>(g, a->dx, a->dt, a->advect_density, f, nullptr);
     // the column-march donor-cell pass, one species at a
     // time through the one pass-1 field of the scratch
     const dim3 gu((unsigned)((g.nx + icar::upf::BX - 1) / icar::upf::BX),

@@ -33,16 +33,36 @@ namespace icar {
 // per-step species-independent fields
 // --------------------------------------------------------------------------
 // What the prep kernels report about the fields of a step, for the exact
-// arithmetic of the single-pass kernel: flags[f] is set to the step's epoch
-// (so nothing has to be cleared between steps) when
-//   FLAG_IEEE  a wind or metric term lies outside the range its branch-free
+// arithmetic of the fused kernels: two words, raised when somewhere
+//   FLAG_IEEE  a wind or metric term lies outside the range the branch-free
 //              quotients are exact for (non-finite, huge, or a face Courant
 //              number that is tiny but not zero), so the tiles take IEEE
 //              division;
 //   FLAG_TIE   J*rho or dz*J*rho is an even integer other than a power of
-//              two somewhere, so that a subnormal quotient can lie exactly
-//              halfway between two floats.
-enum { FLAG_IEEE = 0, FLAG_TIE = 1, N_FLAGS = 2 };
+//              two, so that a subnormal quotient can lie exactly halfway
+//              between two floats.
+// A raised word holds its step's number, so nothing has to be cleared.  The
+// number is kept on the device, so that replayed steps count too: word 0 is
+// the last finished step's, word 1 that of the step under way.  The prep
+// kernel reads word 0 and writes word 1, the kernels after it read word 1 and
+// write word 0, so no kernel reads what it writes.
+enum { FLAG_IEEE = 0, FLAG_TIE = 1, FLAG_HEAD = 2, FLAG_WORDS = 4 };
+// (flags may be null: nobody asks)
+__device__ __forceinline__ void begin_step(int *flags, bool first_thread)
+{
+    if (flags && first_thread) flags[1] = flags[0] + 1;
+}
+__device__ __forceinline__ void raise_flags(int *flags, bool bad, bool tie)
+{
+    if (!flags || !(bad || tie)) return;
+    const int step = flags[0] + 1;
+    if (bad) flags[FLAG_HEAD + FLAG_IEEE] = step;
+    if (tie) flags[FLAG_HEAD + FLAG_TIE] = step;
+}
+__device__ __forceinline__ void end_step(int *flags, bool first_thread)
+{
+    if (first_thread) flags[0] = flags[1];
+}
 __device__ __forceinline__ bool exact_wind(float x)
 {
     const float a = fabsf(x);
@@ -78,8 +98,10 @@ __device__ __forceinline__ void store4(float *p, const float (&r)[4])
 }
 
 __device__ __forceinline__ void prep_quad(const Geo &g, float dx, float dt, int adv_den, const PrepFields &f, unsigned t,
-                                          bool &bad, bool &tie)
+                                          int *flags)
 {
+    begin_step(flags, t == 0);
+    bool bad = false, tie = false;
     const unsigned nq = (unsigned)g.P / 4u, row = t / nq;
     const int i = 4 * (int)(t - row * nq), nx = g.nx, nz = g.nz;
     const int j = (int)(row / (unsigned)nz), k = (int)(row - (unsigned)j * (unsigned)nz);
@@ -143,15 +165,13 @@ __device__ __forceinline__ void prep_quad(const Geo &g, float dx, float dt, int 
             }
     }
     store4(f.Vm + c, vm);
+    raise_flags(flags, bad, tie);
 }
 
 __global__ void __launch_bounds__(256)
-    k_mp_prep(Geo g, float dx, float dt, int adv_den, const __grid_constant__ PrepFields f, int *flags, int epoch)
+    k_mp_prep(Geo g, float dx, float dt, int adv_den, const __grid_constant__ PrepFields f, int *flags)
 {
-    bool bad = false, tie = false;
-    prep_quad(g, dx, dt, adv_den, f, blockIdx.x * blockDim.x + threadIdx.x, bad, tie);
-    if (bad && flags) flags[FLAG_IEEE] = epoch;
-    if (tie && flags) flags[FLAG_TIE] = epoch;
+    prep_quad(g, dx, dt, adv_den, f, blockIdx.x * blockDim.x + threadIdx.x, flags);
 }
 
 // Species pointer tables for the multi-species launches.

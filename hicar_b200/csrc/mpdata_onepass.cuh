@@ -159,12 +159,11 @@ struct OnePassParams {
     float *out[op::MAXS];
     const float *Wm, *DJR, *dz;
     int *err;            // 1: a TMA wait gave up; 2: a TMA operand was misaligned (loads skipped)
-    const int *flags;    // what the prep kernel found in the winds and metrics (FLAG_*), by epoch
+    int *flags;          // what the prep kernel found in the winds and metrics (FLAG_*)
     Geo g;
     int nspecies;
     int tiles_x;
     int klen;            // levels per CTA
-    int epoch;           // flags[i] == epoch: the condition holds for this step's fields
     float nzero;         // -0.0f, not a compile-time constant (see opx::mul2_sep)
 };
 
@@ -1232,8 +1231,9 @@ __device__ __forceinline__ void onepass_item(float *sm, uint64_t *bars, const On
 {
     float worst = 0.0f;
     if constexpr (M == opx::A_EXACT) {
-        const bool tie = p.flags[FLAG_TIE] == p.epoch;
-        bool redo = p.flags[FLAG_IEEE] == p.epoch;
+        const int step = p.flags[1];
+        const bool tie = p.flags[FLAG_HEAD + FLAG_TIE] == step;
+        bool redo = p.flags[FLAG_HEAD + FLAG_IEEE] == step;
         if (!redo) {
             if (!onepass_run<M, FCT>(sm, bars, p, s, tx, j0, ka, kb, tie, worst)) return;
             redo = __syncthreads_or(worst < opx::EXACT_MAX ? 0 : 1) != 0;
@@ -1254,6 +1254,7 @@ __global__ void __launch_bounds__(op::NT, 1) k_mpdata_onepass(const __grid_const
     // planes start on 128-byte boundaries (TMA destinations); SMEM has the slack
     float *sm = reinterpret_cast<float *>(smem4) + ((128u - (smem_u32(smem4) & 127u)) & 127u) / sizeof(float);
     __shared__ __align__(8) uint64_t bars[2];
+    end_step(p.flags, blockIdx.x == 0 && threadIdx.x == 0);
     const int s = blockIdx.x % p.nspecies;
     int rest = blockIdx.x / p.nspecies;
     const int parts = (p.g.nz + p.klen - 1) / p.klen;
@@ -1290,6 +1291,8 @@ __global__ void __launch_bounds__(op::NT, 1)
     if (threadIdx.x == 0) stop = *reinterpret_cast<volatile const int *>(params[0].err);
     __syncthreads();
     if (stop) return;
+    // an item of each member's first species, first level part and first tile
+    end_step(sp.flags, threadIdx.x == 0 && w.y == 0 && w.z == 0 && w.w == 0);
     onepass_init_bars(bars);
     const int ka = (w.y / op::MAXS) * sp.klen, kb = min(ka + sp.klen, sp.g.nz);
     onepass_item<M, FCT>(sm, bars, sp, w.y % op::MAXS, w.z, w.w, ka, kb);

@@ -117,8 +117,9 @@ __global__ void k_std_prep(Geo g, float dx, float dt, int adv_den, const float *
                            const float *__restrict__ jac, const float *__restrict__ ju, const float *__restrict__ jv,
                            const float *__restrict__ jw, const float *__restrict__ dz, float *__restrict__ Um,
                            float *__restrict__ Vm, float *__restrict__ Wm, float *__restrict__ Gc,
-                           float *__restrict__ DJR, int *flags, int epoch)
+                           float *__restrict__ DJR, int *flags)
 {
+    begin_step(flags, blockIdx.x == 0 && threadIdx.x == 0);
     Idx3s t = decode_s(g.nx + 1, g.nz, g.ny + 1);
     if (!t.ok) return;
     bool bad = false, tie = false;
@@ -164,8 +165,7 @@ __global__ void k_std_prep(Geo g, float dx, float dt, int adv_den, const float *
             Vm[c] = 0.0f;
         }
     }
-    if (bad) flags[FLAG_IEEE] = epoch;
-    if (tie) flags[FLAG_TIE] = epoch;
+    raise_flags(flags, bad, tie);
 }
 
 // out = qold outside the tile [its,ite] x [jts,jte] (every species of sp:
@@ -765,17 +765,19 @@ __global__ void __launch_bounds__(SH::NT, SH::CORR ? 1 : 3)
     k_std_fused(Geo g, int its, int ite, int jts, int jte, float tf, const __grid_constant__ SpeciesPtrs sp,
                 int nspecies, int tiles_x, const float *__restrict__ Um, const float *__restrict__ Vm,
                 const float *__restrict__ Wm, const float *__restrict__ Gc, const float *__restrict__ DJR,
-                const int *__restrict__ flags, int epoch)
+                int *flags)
 {
     extern __shared__ float4 sm4[];
     float *sm = reinterpret_cast<float *>(sm4);
+    end_step(flags, blockIdx.x == 0 && threadIdx.x == 0);
     const int s = blockIdx.x % nspecies;
     const int tile = blockIdx.x / nspecies;
     const int i0 = its + (tile % tiles_x) * SH::TX;
     const int j0 = jts + (tile / tiles_x) * SH::TY;
-    bool redo = flags[FLAG_IEEE] == epoch;
+    const int step = flags[1];
+    bool redo = flags[FLAG_HEAD + FLAG_IEEE] == step;
     if (!redo) {
-        const StdArith ar{flags[FLAG_TIE] == epoch};
+        const StdArith ar{flags[FLAG_HEAD + FLAG_TIE] == step};
         float worst;
         if constexpr (SH::CORR)
             worst = std_corr_tile<HORD, VORD, SH, true>(ar, sm, g, its, ite, jts, jte, tf, sp.q1[s], sp.q0[s],
@@ -820,25 +822,24 @@ inline cudaError_t std_fused_setup()
 template <int HORD, int VORD, class SH>
 inline void std_fused_launch_t(cudaStream_t st, const Geo &g, int hs, float tf, const SpeciesPtrs &sp, int S,
                                const float *Um, const float *Vm, const float *Wm, const float *Gc, const float *DJR,
-                               const int *flags, int epoch)
+                               int *flags)
 {
     const int its = hs, ite = g.nx - 1 - hs, jts = hs, jte = g.ny - 1 - hs;
     if (ite < its || jte < jts || S <= 0) return;
     const int tx = (ite - its + SH::TX) / SH::TX, ty = (jte - jts + SH::TY) / SH::TY;
     const unsigned nblk = (unsigned)(tx * ty * S);
     k_std_fused<HORD, VORD, SH><<<nblk, SH::NT, stdf::smem_bytes<SH>(), st>>>(g, its, ite, jts, jte, tf, sp, S, tx,
-                                                                              Um, Vm, Wm, Gc, DJR, flags, epoch);
+                                                                              Um, Vm, Wm, Gc, DJR, flags);
 }
 
 template <class SH>
 inline int std_fused_launch_o(cudaStream_t st, int hord, int vord, const Geo &g, int hs, float tf,
                               const SpeciesPtrs &sp, int S, const float *Um, const float *Vm, const float *Wm,
-                              const float *Gc, const float *DJR, const int *flags, int epoch)
+                              const float *Gc, const float *DJR, int *flags)
 {
 #define ICAR_STD_CASE(h, v)                                                         \
     if (hord == h && vord == v) {                                                   \
-        std_fused_launch_t<h, v, SH>(st, g, hs, tf, sp, S, Um, Vm, Wm, Gc, DJR, flags,    \
-                                    epoch);                                         \
+        std_fused_launch_t<h, v, SH>(st, g, hs, tf, sp, S, Um, Vm, Wm, Gc, DJR, flags);    \
         return 0;                                                                   \
     }
     ICAR_STD_CASE(1, 1) ICAR_STD_CASE(1, 3) ICAR_STD_CASE(1, 5)
@@ -853,7 +854,7 @@ inline int std_fused_launch_o(cudaStream_t st, int hord, int vord, const Geo &g,
 // outside {1,3,5}.
 inline int std_fused_launch(cudaStream_t st, bool corr, int hord, int vord, const Geo &g, int hs, float tf,
                             const SpeciesPtrs &sp, int S, const float *Um, const float *Vm, const float *Wm,
-                            const float *Gc, const float *DJR, const int *flags, int epoch)
+                            const float *Gc, const float *DJR, int *flags)
 {
     if (S <= 0) return 0;
     const size_t ring = ((size_t)g.nx * 2 * hs + (size_t)2 * hs * (size_t)(g.ny > 2 * hs ? g.ny - 2 * hs : 0)) *
@@ -862,8 +863,8 @@ inline int std_fused_launch(cudaStream_t st, bool corr, int hord, int vord, cons
         const unsigned nb = (unsigned)std::min<size_t>((ring + 255) / 256, 148 * 8);
         k_std_ring<<<nb, 256, 0, st>>>(g, hs, sp, S);
     }
-    return corr ? std_fused_launch_o<StdCorrShape>(st, hord, vord, g, hs, tf, sp, S, Um, Vm, Wm, Gc, DJR, flags, epoch)
-                : std_fused_launch_o<StdStageShape>(st, hord, vord, g, hs, tf, sp, S, Um, Vm, Wm, Gc, DJR, flags, epoch);
+    return corr ? std_fused_launch_o<StdCorrShape>(st, hord, vord, g, hs, tf, sp, S, Um, Vm, Wm, Gc, DJR, flags)
+                : std_fused_launch_o<StdStageShape>(st, hord, vord, g, hs, tf, sp, S, Um, Vm, Wm, Gc, DJR, flags);
 }
 
 }  // namespace icar

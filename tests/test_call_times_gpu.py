@@ -8,6 +8,7 @@ import torch
 
 from hicar_b200 import synth
 from hicar_b200.advection import Domain, Options, Parameters, balance_uvw
+from hicar_b200.batch import Batch
 
 pytestmark = pytest.mark.gpu
 
@@ -43,3 +44,27 @@ def test_balance_of_ragged_extents_costs_what_the_aligned_ones_around_it_do():
         t.append(microseconds(lambda: balance_uvw(d, opts), d.sync))
         d.close()
     assert t[0] < 1.15 * t[1], t
+
+
+def test_batch_forgets_a_step_outside_the_exact_range():
+    """A wind too small for the branch-free quotients sends a member's tiles to
+    IEEE division; once it is gone so is its cost, without new tables."""
+    opts = Options()
+    d, dt = device_domain(180, 160, 30, opts, ("qv", "theta", "qc"))
+    b = Batch(0)
+    b.add(d, dt)
+    v = d.download(["v"])["v"]
+    small = v.copy()
+    small[...] = 1e-30
+    for _ in range(4):
+        b.step()
+    t = [microseconds(b.step, b.sync, n=10)]
+    for a in (small, v):
+        d.upload("v", a)
+        b.step()
+        b.step()
+        t.append(microseconds(b.step, b.sync, n=10))
+    b.remove(d)
+    b.close()
+    d.close()
+    assert t[1] > 1.5 * t[0] and t[2] < 1.2 * t[0], t

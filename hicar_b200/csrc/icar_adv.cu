@@ -101,7 +101,7 @@ struct icar_adv_domain {
     std::vector<const float *> map_tag[2];
     int map_next = 0;
     int *op_err = nullptr;
-    int *op_flags = nullptr;   // what the prep kernels report about a step's fields (icar::FLAG_WORDS)
+    int *op_flags = nullptr;   // what the prep kernels report about a step's fields (icar::flag_words)
     bool op_ready = false;
     int nsm = 148;     // SMs of the device
     // diagnostics: launch counter and optional event timing of the species kernels
@@ -686,7 +686,7 @@ int std_advect3d(icar_adv_t *h, const float *qf, const float *qold, float *qout,
 int ensure_flags(icar_adv_t *h)
 {
     if (h->op_flags) return ICAR_ADV_OK;
-    const size_t bytes = icar::FLAG_WORDS * sizeof(int);
+    const size_t bytes = icar::flag_words(h->g) * sizeof(int);
     CUDA_TRY(h, dev_alloc(h, (void **)&h->op_flags, bytes));
     CUDA_TRY(h, cudaMemsetAsync(h->op_flags, 0, bytes, h->stream));
     return ICAR_ADV_OK;

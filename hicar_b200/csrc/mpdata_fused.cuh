@@ -33,31 +33,37 @@ namespace icar {
 // per-step species-independent fields
 // --------------------------------------------------------------------------
 // What the prep kernels report about the fields of a step, for the exact
-// arithmetic of the fused kernels: two words, raised when somewhere
+// arithmetic of the fused kernels: two words per block of 32 x 8 columns,
+// raised when somewhere in them
 //   FLAG_IEEE  a wind or metric term lies outside the range the branch-free
 //              quotients are exact for (non-finite, huge, or a face Courant
-//              number that is tiny but not zero), so the tiles take IEEE
-//              division;
+//              number that is tiny but not zero), so the tiles that read it
+//              take IEEE division;
 //   FLAG_TIE   J*rho or dz*J*rho is an even integer other than a power of
 //              two, so that a subnormal quotient can lie exactly halfway
 //              between two floats.
+// (The standard scheme's prep raises the first block's for the whole domain.)
 // A raised word holds its step's number, so nothing has to be cleared.  The
 // number is kept on the device, so that replayed steps count too: word 0 is
 // the last finished step's, word 1 that of the step under way.  The prep
 // kernel reads word 0 and writes word 1, the kernels after it read word 1 and
 // write word 0, so no kernel reads what it writes.
-enum { FLAG_IEEE = 0, FLAG_TIE = 1, FLAG_HEAD = 2, FLAG_WORDS = 4 };
+enum { FLAG_IEEE = 0, FLAG_TIE = 1, FLAG_HEAD = 2 };
+constexpr int FLAG_BX = 32, FLAG_BY = 8;
+__host__ __device__ inline int flag_blocks_x(const Geo &g) { return (g.nx + FLAG_BX - 1) / FLAG_BX; }
+__host__ __device__ inline int flag_blocks_y(const Geo &g) { return (g.ny + FLAG_BY - 1) / FLAG_BY; }
+inline size_t flag_words(const Geo &g) { return FLAG_HEAD + 2 * (size_t)flag_blocks_x(g) * flag_blocks_y(g); }
 // (flags may be null: nobody asks)
 __device__ __forceinline__ void begin_step(int *flags, bool first_thread)
 {
     if (flags && first_thread) flags[1] = flags[0] + 1;
 }
-__device__ __forceinline__ void raise_flags(int *flags, bool bad, bool tie)
+__device__ __forceinline__ void raise_flags(int *flags, int block, bool bad, bool tie)
 {
     if (!flags || !(bad || tie)) return;
     const int step = flags[0] + 1;
-    if (bad) flags[FLAG_HEAD + FLAG_IEEE] = step;
-    if (tie) flags[FLAG_HEAD + FLAG_TIE] = step;
+    if (bad) flags[FLAG_HEAD + 2 * block + FLAG_IEEE] = step;
+    if (tie) flags[FLAG_HEAD + 2 * block + FLAG_TIE] = step;
 }
 __device__ __forceinline__ void end_step(int *flags, bool first_thread)
 {
@@ -165,7 +171,7 @@ __device__ __forceinline__ void prep_quad(const Geo &g, float dx, float dt, int 
             }
     }
     store4(f.Vm + c, vm);
-    raise_flags(flags, bad, tie);
+    raise_flags(flags, (j / FLAG_BY) * flag_blocks_x(g) + i / FLAG_BX, bad, tie);
 }
 
 __global__ void __launch_bounds__(256)

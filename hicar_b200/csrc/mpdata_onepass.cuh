@@ -1204,7 +1204,11 @@ __device__ __forceinline__ bool onepass_run(float *sm, uint64_t *bars, const One
 }
 
 // The march with IEEE division, out of line, so that it costs the others no
-// registers.
+// registers.  A tile of it takes about 2.5 times the exact march's time (up to
+// five times with subnormal operands, whose divisions take their slow path).  A
+// step of 512x512x40x12 with one wind of 1e-30 takes 3.68 ms where one without
+// takes 3.56, with all of v at 1e-30 19.9.  Copies of it for interior tiles
+// and for the middle of the march bring that to 19.5 and are left out.
 template <bool FCT>
 __device__ __noinline__ void onepass_redo(float *sm, uint64_t *bars, const OnePassParams &p, int s, int tx, int j0, int ka,
                                           int kb)
@@ -1221,8 +1225,28 @@ __device__ __noinline__ void onepass_redo(float *sm, uint64_t *bars, const OnePa
     onepass_tile<opx::A_IEEE, FCT, false>(sm, bars, p, s, x0, xlo, xhi, j0, ka, kb, false, worst);
 }
 
+// Flags of the blocks of columns that the plane with origin (x0, y0) covers
+// (at most 3 x 5 of them); every thread of the CTA.  The answers come through
+// a shuffle, which the compiler knows to be uniform: as per-thread values they
+// cost the exact march ten spilled registers.
+__device__ __forceinline__ void plane_flags(const OnePassParams &p, int x0, int y0, bool &ieee, bool &tie)
+{
+    const int nbx = flag_blocks_x(p.g);
+    const int bx0 = x0 / FLAG_BX, wx = min(x0 + op::PW - 1, p.g.nx - 1) / FLAG_BX - bx0 + 1;
+    const int by0 = max(y0, 0) / FLAG_BY, wy = min(y0 + op::PH - 1, p.g.ny - 1) / FLAG_BY - by0 + 1;
+    bool b = false, t = false;
+    if (threadIdx.x < (unsigned)(wx * wy)) {
+        const int at = (by0 + (int)threadIdx.x / wx) * nbx + bx0 + (int)threadIdx.x % wx;
+        const int step = p.flags[1];
+        b = p.flags[FLAG_HEAD + 2 * at + FLAG_IEEE] == step;
+        t = p.flags[FLAG_HEAD + 2 * at + FLAG_TIE] == step;
+    }
+    ieee = __shfl_sync(opx::FULL, __syncthreads_or(b), 0) != 0;
+    tie = __shfl_sync(opx::FULL, __syncthreads_or(t), 0) != 0;
+}
+
 // One work item of either form.  A_EXACT: a tile whose fields or values lie
-// outside what its quotients are proven for (the prep kernel's FLAG_IEEE, or
+// outside what its quotients are proven for (FLAG_IEEE in its plane, or
 // `worst` at the end of the march) is marched with IEEE division; the tile's
 // stores are then overwritten, which no other tile reads.
 template <int M, bool FCT>
@@ -1231,9 +1255,10 @@ __device__ __forceinline__ void onepass_item(float *sm, uint64_t *bars, const On
 {
     float worst = 0.0f;
     if constexpr (M == opx::A_EXACT) {
-        const int step = p.flags[1];
-        const bool tie = p.flags[FLAG_HEAD + FLAG_TIE] == step;
-        bool redo = p.flags[FLAG_HEAD + FLAG_IEEE] == step;
+        int x0, xlo, xhi;
+        op::xtile(p.g.nx, tx, p.tiles_x, x0, xlo, xhi);
+        bool redo, tie;
+        plane_flags(p, x0, j0 - 3, redo, tie);
         if (!redo) {
             if (!onepass_run<M, FCT>(sm, bars, p, s, tx, j0, ka, kb, tie, worst)) return;
             redo = __syncthreads_or(worst < opx::EXACT_MAX ? 0 : 1) != 0;

@@ -165,7 +165,7 @@ __global__ void k_std_prep(Geo g, float dx, float dt, int adv_den, const float *
             Vm[c] = 0.0f;
         }
     }
-    raise_flags(flags, bad, tie);
+    raise_flags(flags, 0, bad, tie);
 }
 
 // out = qold outside the tile [its,ite] x [jts,jte] (every species of sp:

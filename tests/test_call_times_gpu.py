@@ -7,7 +7,7 @@ import pytest
 import torch
 
 from hicar_b200 import synth
-from hicar_b200.advection import Domain, Options, Parameters, balance_uvw
+from hicar_b200.advection import Domain, Options, Parameters, advect, balance_uvw
 from hicar_b200.batch import Batch
 
 pytestmark = pytest.mark.gpu
@@ -68,3 +68,14 @@ def test_batch_forgets_a_step_outside_the_exact_range():
     b.close()
     d.close()
     assert t[1] > 1.5 * t[0] and t[2] < 1.2 * t[0], t
+
+
+def test_one_wind_outside_the_exact_range_costs_its_tiles_only():
+    opts = Options()
+    names = ("qv", "theta", "qc", "qr", "qs", "qi")
+    t = []
+    for change in (None, lambda f: f["u"].__setitem__((20, 3, 30), 1e-30)):
+        d, dt = device_domain(384, 384, 30, opts, names, change)
+        t.append(microseconds(lambda: advect(d, opts, dt), d.sync, n=10))
+        d.close()
+    assert t[1] < 1.5 * t[0], t

@@ -99,7 +99,6 @@ struct icar_adv_domain {
     std::unordered_map<const float *, CUtensorMap> tmaps;
     CUtensorMap *map_dev[2] = {nullptr, nullptr};
     std::vector<const float *> map_tag[2];
-    int map_next = 0;
     int *op_err = nullptr;
     int *op_flags = nullptr;   // what the prep kernels report about a step's fields (icar::flag_words)
     bool op_ready = false;
@@ -767,29 +766,13 @@ int plane_map(icar_adv_t *h, const float *base, int rows, const CUtensorMap **ou
     return ICAR_ADV_OK;
 }
 
-// The device table of descriptors for the current buffers: every species
-// input in adv_vars order, then U_m, V_m, W_m/dz, J*rho.  Two tables are
-// kept, tagged with the device addresses they describe; a table is rebuilt
-// (encode + one copy on the handle's stream) only when neither matches.
-int onepass_maps(icar_adv_t *h, const CUtensorMap **out)
+// Fill descriptor table t for the given fields (species inputs in adv_vars
+// order, then U_m, V_m, W_m/dz, J*rho); host holds them until the copy is done.
+int fill_table(icar_adv_t *h, int t, const std::vector<const float *> &want, std::vector<CUtensorMap> &host)
 {
     const int S = h->desc.n_species;
-    std::vector<const float *> want;
-    want.reserve(S + 4);
-    for (int s = 0; s < S; s++) want.push_back(h->q[s].p);
-    want.push_back(h->Um.p);
-    want.push_back(h->Vm.p);
-    want.push_back(h->Wp.p);
-    want.push_back(h->Gc.p);
-    for (int t = 0; t < 2; t++)
-        if (h->map_dev[t] && h->map_tag[t] == want) {
-            *out = h->map_dev[t];
-            return ICAR_ADV_OK;
-        }
-    const int t = h->map_next;
-    h->map_next ^= 1;
     if (!h->map_dev[t]) CUDA_TRY(h, dev_alloc(h, (void **)&h->map_dev[t], (size_t)(S + 4) * sizeof(CUtensorMap)));
-    std::vector<CUtensorMap> host(S + 4);
+    host.resize(S + 4);
     int e;
     const CUtensorMap *m;
     for (int s = 0; s < S + 4; s++) {
@@ -797,12 +780,44 @@ int onepass_maps(icar_adv_t *h, const CUtensorMap **out)
         if ((e = plane_map(h, want[s], rows, &m))) return e;
         host[s] = *m;
     }
+    h->map_tag[t].clear();
     // ordered on the stream after any kernel still reading the old table
     CUDA_TRY(h, cudaMemcpyAsync(h->map_dev[t], host.data(), host.size() * sizeof(CUtensorMap),
                                 cudaMemcpyHostToDevice, h->stream));
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     h->map_tag[t] = want;
-    *out = h->map_dev[t];
+    return ICAR_ADV_OK;
+}
+
+// The device table of descriptors for the current buffers.  The species
+// alternate between two buffers, so there are two tables, tagged with the
+// device addresses they describe.  When neither matches both are built (encode
+// and copy on the handle's stream, then a wait for it), the other one for the
+// step after this: from the second step on nothing here waits, and steps can be
+// captured in a graph after one of them has run.
+int onepass_maps(icar_adv_t *h, const CUtensorMap **out)
+{
+    const int S = h->desc.n_species;
+    auto wanted = [&](const std::vector<DevBuf> &q) {
+        std::vector<const float *> want;
+        want.reserve(S + 4);
+        for (int s = 0; s < S; s++) want.push_back(q[s].p);
+        for (const DevBuf *b : {&h->Um, &h->Vm, &h->Wp, &h->Gc}) want.push_back(b->p);
+        return want;
+    };
+    const std::vector<const float *> want = wanted(h->q);
+    for (int t = 0; t < 2; t++)
+        if (h->map_dev[t] && h->map_tag[t] == want) {
+            *out = h->map_dev[t];
+            return ICAR_ADV_OK;
+        }
+    std::vector<CUtensorMap> host[2];
+    int e;
+    if ((e = fill_table(h, 0, want, host[0])) || (e = fill_table(h, 1, wanted(h->qn), host[1]))) {
+        cudaStreamSynchronize(h->stream);  // a copy from host may be queued
+        return e;
+    }
+    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+    *out = h->map_dev[0];
     return ICAR_ADV_OK;
 }
 

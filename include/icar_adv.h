@@ -260,7 +260,10 @@ int icar_adv_sync_timeout(icar_adv_t *h, double timeout_s);
 /* Use an external CUDA stream (cudaStream_t passed as void*; NULL = the
  * handle's own stream).  Work already queued on the previous stream comes
  * first: the new stream waits for it (no host wait).  The stream must stay
- * valid while the handle uses it. */
+ * valid while the handle uses it.  A handle's first step allocates and waits;
+ * after it, steps can be captured from the stream into a CUDA graph (an even
+ * number of them where the graph is replayed, as the species alternate
+ * between two buffers; not icar_adv_step_host, which waits). */
 int icar_adv_set_stream(icar_adv_t *h, void *cuda_stream);
 
 /* Bytes of device memory the handle holds. */

@@ -39,7 +39,7 @@ def _nvcc() -> str:
 
 
 def _sources():
-    return sorted(CSRC.glob("*.cu")) + sorted(CSRC.glob("*.cuh")) + [ROOT / "include" / "icar_adv.h"]
+    return sorted(CSRC.glob("*.cu")) + sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")) + [ROOT / "include" / "icar_adv.h"]
 
 
 def build_cuda(force: bool = False, verbose: bool = False) -> Path:

@@ -882,9 +882,12 @@ int mpdata_onepass_group(icar_adv_t *h, int s0, int s1)
     prm.g = g;
     prm.nspecies = S;
     prm.tiles_x = onepass_tiles_x(g);
-    const int tiles = onepass_tiles_x(g) * onepass_tiles_y(g) * S;
-    prm.klen = icar::op::levels_per_cta(tiles, g.nz, h->nsm);
-    const unsigned grid = (unsigned)tiles * (unsigned)((g.nz + prm.klen - 1) / prm.klen);
+    const long items = (long)onepass_tiles_x(g) * onepass_tiles_y(g) * S;
+    const icar::op::ColumnSplit split = icar::op::split_columns(items, g.nz, h->nsm);
+    prm.items = (unsigned)items;
+    prm.whole = (unsigned)split.whole;
+    prm.parts = split.parts;
+    const unsigned grid = (unsigned)icar::op::split_ctas(split, items);
     const bool exact = h->path != 3, fct = h->opts.mpdata_fct != 0;
     cudaEvent_t c0 = nullptr, c1 = nullptr;
     if (h->profiling) {
@@ -2034,11 +2037,11 @@ int build_tables(icar_adv_batch_t *b)
     std::vector<icar::OnePassParams> opp[2];
     std::vector<CUtensorMap> maps;
     std::vector<size_t> map_base[2];
-    std::vector<int> klen(M, 0);   // levels per single-pass item of each member
+    std::vector<int> parts(M, 1);   // level ranges per column of each member
     long tiles = 0;
     for (icar_adv_t *h : b->members)
         tiles += (long)onepass_tiles_x(h->g) * onepass_tiles_y(h->g) * h->desc.n_species;
-    for (int m = 0; m < M; m++) klen[m] = icar::op::levels_per_cta(tiles, b->members[m]->g.nz, b->nsm);
+    for (int m = 0; m < M; m++) parts[m] = icar::op::best_parts(tiles, b->members[m]->g.nz, b->nsm);
     opp[0].resize(std::max(M, 1));
     opp[1].resize(std::max(M, 1));
     map_base[0].resize(M);
@@ -2075,11 +2078,11 @@ int build_tables(icar_adv_batch_t *b)
                 fpre.push_back(fpre.back() + (int)(((size_t)h->nzone * g.nz + 255) / 256));
             }
         }
-        const int tx = onepass_tiles_x(g), tyn = onepass_tiles_y(g), parts = (g.nz + klen[m] - 1) / klen[m];
+        const int tx = onepass_tiles_x(g), tyn = onepass_tiles_y(g);
         for (int s = 0; s < h->desc.n_species; s++)
             for (int a = 0; a < tyn; a++)
                 for (int c = 0; c < tx; c++)
-                    for (int k = 0; k < parts; k++)
+                    for (int k = 0; k < parts[m]; k++)
                         items.push_back(make_int4(m, s + icar::op::MAXS * k, c, a * icar::op::TY));
     }
     if (!maps.empty() && (maps.size() > b->bmaps_cap || !b->d_bmaps)) {
@@ -2108,7 +2111,7 @@ int build_tables(icar_adv_batch_t *b)
             q.g = h->g;
             q.nspecies = S;
             q.tiles_x = onepass_tiles_x(h->g);
-            q.klen = klen[m];
+            q.parts = parts[m];
         }
     if ((size_t)std::max(M, 1) > b->opp_cap || !b->d_opp[0]) {
         for (int pp = 0; pp < 2; pp++) {
@@ -2120,10 +2123,12 @@ int build_tables(icar_adv_batch_t *b)
         for (int pp = 0; pp < 2; pp++) BCUDA(b, cudaMalloc(&b->d_opp[pp], cap * sizeof(icar::OnePassParams)));
         b->opp_cap = cap;
     }
-    // longest columns first (cost ~ levels per item), so the tail of the
-    // launch is made of short items
-    std::stable_sort(items.begin(), items.end(),
-                     [&](const int4 &x, const int4 &y) { return klen[x.x] > klen[y.x]; });
+    // most levels first, so the tail of the launch is made of short items
+    auto levels = [&](const int4 &x) {
+        const int nz = b->members[x.x]->g.nz, k = x.y / icar::op::MAXS;
+        return icar::op::range_begin(nz, parts[x.x], k + 1) - icar::op::range_begin(nz, parts[x.x], k);
+    };
+    std::stable_sort(items.begin(), items.end(), [&](const int4 &x, const int4 &y) { return levels(x) > levels(y); });
     b->n_prep = prep[M];
     b->n_pairs = (int)pairs.size();
     b->n_force = fpre.back();

@@ -71,6 +71,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "launch_split.h"
 #include "tma.cuh"
 
 namespace icar {
@@ -124,29 +125,6 @@ __device__ __forceinline__ void xtile(int nx, int tx, int ntx, int &x0, int &xlo
         }
     }
 }
-
-// Levels per CTA for a launch of `tiles` (column tile, species) pairs of nz
-// levels on `sms` SMs (one CTA each).  A CTA that marches only levels
-// [ka, kb) of its tile repeats about three levels of its neighbours' work
-// and its own start-up costs about two more, so a column is cut only where
-// that shortens the launch: the cut of least waves x (levels + overhead),
-// with at least five levels each.  Whole columns against this rule, fast
-// kernel: 128x128x20, one species (18 tiles) 80 -> 36 us, 256x256x40 161 -> 95
-// us; 187x301x33x5 (280 tiles, stays whole) 257 us.
-inline int levels_per_cta(long tiles, int nz, int sms)
-{
-    long best = -1;
-    int len = nz;
-    for (int n = 1; n == 1 || (nz + n - 1) / n >= 5; n++) {
-        const int l = (nz + n - 1) / n, parts = (nz + l - 1) / l;
-        const long cost = (tiles * parts + sms - 1) / sms * (l + 2 + (parts > 1 ? 3 : 0));
-        if (best < 0 || cost < best) {
-            best = cost;
-            len = l;
-        }
-    }
-    return len;
-}
 }  // namespace op
 
 // Kernel parameters.  The tensor maps (64 x 1 x 28 boxes over (x, z, y))
@@ -163,7 +141,8 @@ struct OnePassParams {
     Geo g;
     int nspecies;
     int tiles_x;
-    int klen;            // levels per CTA
+    unsigned whole, items;   // (tile, species) pairs that march whole columns, and all of them
+    int parts;               // level ranges of the others
     float nzero;         // -0.0f, not a compile-time constant (see opx::mul2_sep)
 };
 
@@ -1280,12 +1259,11 @@ __global__ void __launch_bounds__(op::NT, 1) k_mpdata_onepass(const __grid_const
     float *sm = reinterpret_cast<float *>(smem4) + ((128u - (smem_u32(smem4) & 127u)) & 127u) / sizeof(float);
     __shared__ __align__(8) uint64_t bars[2];
     end_step(p.flags, blockIdx.x == 0 && threadIdx.x == 0);
-    const int s = blockIdx.x % p.nspecies;
-    int rest = blockIdx.x / p.nspecies;
-    const int parts = (p.g.nz + p.klen - 1) / p.klen;
-    const int ka = (rest % parts) * p.klen, kb = min(ka + p.klen, p.g.nz);
-    rest /= parts;
-    const int tx = rest % p.tiles_x, j0 = (rest / p.tiles_x) * TY;
+    unsigned item;
+    int ka, kb;
+    split_cta(blockIdx.x, p.whole, p.parts, p.items, p.g.nz, item, ka, kb);
+    const int s = (int)(item % (unsigned)p.nspecies), tile = (int)(item / (unsigned)p.nspecies);
+    const int tx = tile % p.tiles_x, j0 = (tile / p.tiles_x) * TY;
     __shared__ int stop;
     if (threadIdx.x == 0) stop = *reinterpret_cast<volatile const int *>(p.err);
     __syncthreads();
@@ -1319,7 +1297,8 @@ __global__ void __launch_bounds__(op::NT, 1)
     // an item of each member's first species, first level part and first tile
     end_step(sp.flags, threadIdx.x == 0 && w.y == 0 && w.z == 0 && w.w == 0);
     onepass_init_bars(bars);
-    const int ka = (w.y / op::MAXS) * sp.klen, kb = min(ka + sp.klen, sp.g.nz);
+    const int k = w.y / op::MAXS;
+    const int ka = op::range_begin(sp.g.nz, sp.parts, k), kb = op::range_begin(sp.g.nz, sp.parts, k + 1);
     onepass_item<M, FCT>(sm, bars, sp, w.y % op::MAXS, w.z, w.w, ka, kb);
 }
 

@@ -79,3 +79,18 @@ def test_one_wind_outside_the_exact_range_costs_its_tiles_only():
         t.append(microseconds(lambda: advect(d, opts, dt), d.sync, n=10))
         d.close()
     assert t[1] < 1.5 * t[0], t
+
+
+@pytest.mark.parametrize("path", [0, 3])
+def test_a_launch_just_above_a_wave_costs_little_more_than_the_wave(path):
+    """Six species of 96 x 250 are 144 column tiles, one wave of the 148 SMs;
+    seven are 168."""
+    opts = Options()
+    names = ("qv", "theta", "qc", "qr", "qs", "qi", "qg")
+    t = []
+    for n in (6, 7):
+        d, dt = device_domain(96, 250, 35, opts, names[:n])
+        d.set_path(path)
+        t.append(microseconds(lambda: advect(d, opts, dt), d.sync, n=20))
+        d.close()
+    assert t[1] < 1.35 * t[0], t

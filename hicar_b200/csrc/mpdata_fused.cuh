@@ -44,20 +44,17 @@ namespace icar {
 //              between two floats.
 // (The standard scheme's prep raises the first block's for the whole domain.)
 // A raised word holds its step's number, so nothing has to be cleared.  The
-// number is kept on the device, so that replayed steps count too: word 0 is
-// the last finished step's, word 1 that of the step under way.  The prep
+// number is kept on the device, so that replayed steps count too: word 0 counts
+// the launches that came after a prep kernel, word 1 is the number of the step
+// under way, one more than word 0 was when its prep kernel ran.  The prep
 // kernel reads word 0 and writes word 1, the kernels after it read word 1 and
-// write word 0, so no kernel reads what it writes.
+// add to word 0, so no kernel reads what it writes.
 enum { FLAG_IEEE = 0, FLAG_TIE = 1, FLAG_HEAD = 2 };
 constexpr int FLAG_BX = 32, FLAG_BY = 8;
 __host__ __device__ inline int flag_blocks_x(const Geo &g) { return (g.nx + FLAG_BX - 1) / FLAG_BX; }
 __host__ __device__ inline int flag_blocks_y(const Geo &g) { return (g.ny + FLAG_BY - 1) / FLAG_BY; }
 inline size_t flag_words(const Geo &g) { return FLAG_HEAD + 2 * (size_t)flag_blocks_x(g) * flag_blocks_y(g); }
 // (flags may be null: nobody asks)
-__device__ __forceinline__ void begin_step(int *flags, bool first_thread)
-{
-    if (flags && first_thread) flags[1] = flags[0] + 1;
-}
 __device__ __forceinline__ void raise_flags(int *flags, int block, bool bad, bool tie)
 {
     if (!flags || !(bad || tie)) return;
@@ -65,9 +62,11 @@ __device__ __forceinline__ void raise_flags(int *flags, int block, bool bad, boo
     if (bad) flags[FLAG_HEAD + 2 * block + FLAG_IEEE] = step;
     if (tie) flags[FLAG_HEAD + 2 * block + FLAG_TIE] = step;
 }
-__device__ __forceinline__ void end_step(int *flags, bool first_thread)
+// (an addition that nobody waits for: a load and a store held up the launch by
+// the latency of both, 1.2 us of the 41 of a 128x128x20 step)
+__device__ __forceinline__ void count_launch(int *flags, bool first_thread)
 {
-    if (first_thread) flags[0] = flags[1];
+    if (first_thread) atomicAdd(&flags[0], 1);
 }
 __device__ __forceinline__ bool exact_wind(float x)
 {
@@ -106,8 +105,8 @@ __device__ __forceinline__ void store4(float *p, const float (&r)[4])
 __device__ __forceinline__ void prep_quad(const Geo &g, float dx, float dt, int adv_den, const PrepFields &f, unsigned t,
                                           int *flags)
 {
-    begin_step(flags, t == 0);
     bool bad = false, tie = false;
+    const int step = flags && t == 0 ? flags[0] + 1 : 0;
     const unsigned nq = (unsigned)g.P / 4u, row = t / nq;
     const int i = 4 * (int)(t - row * nq), nx = g.nx, nz = g.nz;
     const int j = (int)(row / (unsigned)nz), k = (int)(row - (unsigned)j * (unsigned)nz);
@@ -172,6 +171,7 @@ __device__ __forceinline__ void prep_quad(const Geo &g, float dx, float dt, int 
     }
     store4(f.Vm + c, vm);
     raise_flags(flags, (j / FLAG_BY) * flag_blocks_x(g) + i / FLAG_BX, bad, tie);
+    if (flags && t == 0) flags[1] = step;
 }
 
 __global__ void __launch_bounds__(256)

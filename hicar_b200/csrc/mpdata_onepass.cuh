@@ -1204,24 +1204,23 @@ __device__ __noinline__ void onepass_redo(float *sm, uint64_t *bars, const OnePa
     onepass_tile<opx::A_IEEE, FCT, false>(sm, bars, p, s, x0, xlo, xhi, j0, ka, kb, false, worst);
 }
 
-// Flags of the blocks of columns that the plane with origin (x0, y0) covers
-// (at most 3 x 5 of them); every thread of the CTA.  The answers come through
-// a shuffle, which the compiler knows to be uniform: as per-thread values they
-// cost the exact march ten spilled registers.
+// Flags of the blocks of columns that the plane with origin (x0, y0) covers, at
+// most 3 x 5 of them, one to a lane; every warp asks for itself.  (The votes are
+// uniform for the compiler too: answers that were not cost the exact march ten
+// spilled registers.)
 __device__ __forceinline__ void plane_flags(const OnePassParams &p, int x0, int y0, bool &ieee, bool &tie)
 {
-    const int nbx = flag_blocks_x(p.g);
+    const int nbx = flag_blocks_x(p.g), lane = threadIdx.x & 31;
     const int bx0 = x0 / FLAG_BX, wx = min(x0 + op::PW - 1, p.g.nx - 1) / FLAG_BX - bx0 + 1;
     const int by0 = max(y0, 0) / FLAG_BY, wy = min(y0 + op::PH - 1, p.g.ny - 1) / FLAG_BY - by0 + 1;
     bool b = false, t = false;
-    if (threadIdx.x < (unsigned)(wx * wy)) {
-        const int at = (by0 + (int)threadIdx.x / wx) * nbx + bx0 + (int)threadIdx.x % wx;
-        const int step = p.flags[1];
+    if (lane < wx * wy) {
+        const int at = (by0 + lane / wx) * nbx + bx0 + lane % wx, step = p.flags[1];
         b = p.flags[FLAG_HEAD + 2 * at + FLAG_IEEE] == step;
         t = p.flags[FLAG_HEAD + 2 * at + FLAG_TIE] == step;
     }
-    ieee = __shfl_sync(opx::FULL, __syncthreads_or(b), 0) != 0;
-    tie = __shfl_sync(opx::FULL, __syncthreads_or(t), 0) != 0;
+    ieee = __any_sync(opx::FULL, b);
+    tie = __any_sync(opx::FULL, t);
 }
 
 // One work item of either form.  A_EXACT: a tile whose fields or values lie
@@ -1258,7 +1257,7 @@ __global__ void __launch_bounds__(op::NT, 1) k_mpdata_onepass(const __grid_const
     // planes start on 128-byte boundaries (TMA destinations); SMEM has the slack
     float *sm = reinterpret_cast<float *>(smem4) + ((128u - (smem_u32(smem4) & 127u)) & 127u) / sizeof(float);
     __shared__ __align__(8) uint64_t bars[2];
-    end_step(p.flags, blockIdx.x == 0 && threadIdx.x == 0);
+    count_launch(p.flags, blockIdx.x == 0 && threadIdx.x == 0);
     unsigned item;
     int ka, kb;
     split_cta(blockIdx.x, p.whole, p.parts, p.items, p.g.nz, item, ka, kb);
@@ -1295,7 +1294,7 @@ __global__ void __launch_bounds__(op::NT, 1)
     __syncthreads();
     if (stop) return;
     // an item of each member's first species, first level part and first tile
-    end_step(sp.flags, threadIdx.x == 0 && w.y == 0 && w.z == 0 && w.w == 0);
+    count_launch(sp.flags, threadIdx.x == 0 && w.y == 0 && w.z == 0 && w.w == 0);
     onepass_init_bars(bars);
     const int k = w.y / op::MAXS;
     const int ka = op::range_begin(sp.g.nz, sp.parts, k), kb = op::range_begin(sp.g.nz, sp.parts, k + 1);

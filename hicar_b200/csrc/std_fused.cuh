@@ -119,7 +119,7 @@ __global__ void k_std_prep(Geo g, float dx, float dt, int adv_den, const float *
                            float *__restrict__ Vm, float *__restrict__ Wm, float *__restrict__ Gc,
                            float *__restrict__ DJR, int *flags)
 {
-    begin_step(flags, blockIdx.x == 0 && threadIdx.x == 0);
+    if (blockIdx.x == 0 && threadIdx.x == 0) flags[1] = flags[0] + 1;
     Idx3s t = decode_s(g.nx + 1, g.nz, g.ny + 1);
     if (!t.ok) return;
     bool bad = false, tie = false;
@@ -769,7 +769,7 @@ __global__ void __launch_bounds__(SH::NT, SH::CORR ? 1 : 3)
 {
     extern __shared__ float4 sm4[];
     float *sm = reinterpret_cast<float *>(sm4);
-    end_step(flags, blockIdx.x == 0 && threadIdx.x == 0);
+    count_launch(flags, blockIdx.x == 0 && threadIdx.x == 0);
     const int s = blockIdx.x % nspecies;
     const int tile = blockIdx.x / nspecies;
     const int i0 = its + (tile % tiles_x) * SH::TX;

@@ -884,7 +884,6 @@ int mpdata_onepass_group(icar_adv_t *h, int s0, int s1)
     prm.tiles_x = onepass_tiles_x(g);
     const long items = (long)onepass_tiles_x(g) * onepass_tiles_y(g) * S;
     const icar::op::ColumnSplit split = icar::op::split_columns(items, g.nz, h->nsm);
-    prm.items = (unsigned)items;
     prm.whole = (unsigned)split.whole;
     prm.parts = split.parts;
     const unsigned grid = (unsigned)icar::op::split_ctas(split, items);

@@ -141,8 +141,8 @@ struct OnePassParams {
     Geo g;
     int nspecies;
     int tiles_x;
-    unsigned whole, items;   // (tile, species) pairs that march whole columns, and all of them
-    int parts;               // level ranges of the others
+    unsigned whole;      // (tile, species) pairs that march whole columns
+    int parts;           // level ranges of the others
     float nzero;         // -0.0f, not a compile-time constant (see opx::mul2_sep)
 };
 
@@ -1260,7 +1260,7 @@ __global__ void __launch_bounds__(op::NT, 1) k_mpdata_onepass(const __grid_const
     count_launch(p.flags, blockIdx.x == 0 && threadIdx.x == 0);
     unsigned item;
     int ka, kb;
-    split_cta(blockIdx.x, p.whole, p.parts, p.items, p.g.nz, item, ka, kb);
+    split_cta(blockIdx.x, p.whole, p.parts, p.g.nz, item, ka, kb);
     const int s = (int)(item % (unsigned)p.nspecies), tile = (int)(item / (unsigned)p.nspecies);
     const int tx = tile % p.tiles_x, j0 = (tile / p.tiles_x) * TY;
     __shared__ int stop;

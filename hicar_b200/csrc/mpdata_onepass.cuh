@@ -72,6 +72,7 @@
 
 #include "common.cuh"
 #include "launch_split.h"
+#include "mpdata_fused.cuh"
 #include "tma.cuh"
 
 namespace icar {
@@ -242,7 +243,7 @@ __device__ __forceinline__ ExDiv exdiv(float2 b, float s, float r)
 __device__ __forceinline__ float tie_even(float nq, float nq0, float rem, float bs)
 {
     if (fabsf(nq0) < 0x1p-125f && fabsf(rem) == bs * 0x1p-75f * 0x1p-75f)
-        return (__float_as_int(nq0) & 1) ? nq0 - copysignf(0x1p-149f, rem) : nq0;
+        return (__float_as_int(nq0) & 1) ? copysignf(nq0 - copysignf(0x1p-149f, rem), nq0) : nq0;
     return nq;
 }
 __device__ __forceinline__ float2 nquot(float2 a, const ExDiv &d, bool tie)

@@ -92,7 +92,7 @@ __device__ __forceinline__ float std_quot(float a, float b, float nr, const StdA
     float q = __fmaf_rn(rem, nrs, q0);
     if (__builtin_expect(ar.tie, 0)) {
         if (fabsf(q0) < 0x1p-125f && fabsf(rem) == bs * 0x1p-75f * 0x1p-75f)
-            q = (__float_as_int(q0) & 1) ? q0 - copysignf(0x1p-149f, rem) : q0;
+            q = (__float_as_int(q0) & 1) ? copysignf(q0 - copysignf(0x1p-149f, rem), q0) : q0;
     }
     return -q;
 }

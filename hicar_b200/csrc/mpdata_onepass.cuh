@@ -1005,8 +1005,9 @@ __device__ __forceinline__ bool onepass_tile(float *sm, uint64_t *bars, const On
 
         // own-column values for the next iteration and this one's store
         if (ST || t + 3 <= l1) {
-            load_ahead(t + 3);
-            if (halo) load_ahead_b(t + 3);
+            const int L = ST ? min(t + 3, l1) : t + 3;   // (the last middle iteration loads a level it has no use for)
+            load_ahead(L);
+            if (halo) load_ahead_b(L);
         }
         if (halo) {
             if (FCT && hor) {
@@ -1146,7 +1147,7 @@ __device__ __forceinline__ bool onepass_tile(float *sm, uint64_t *bars, const On
     };
 #pragma unroll 1
     for (int t = t0; t <= kb; t++) {
-        const bool mid = M != A_IEEE && t > ka && t <= l1 - 3 && t < kb;
+        const bool mid = M != A_IEEE && t > ka && t <= l1 - 2 && t < kb;
         if (mid ? !level(std::bool_constant<M != A_IEEE>{}, t) : !level(std::false_type{}, t)) return false;
     }
     return true;

@@ -1,25 +1,23 @@
-"""Autotuner for the launch-shape knobs of the MPDATA kernels.
+"""Launch-shape knobs of earlier MPDATA kernels.
 
 The two knobs, tile shape (8, 15, 24 or 31 rows) and species group of the
 donor-cell pass (0 = all), belonged to kernels that handles and batches no
-longer run: the single-pass kernel has one tile shape and chooses its level
-ranges from the grid.  They are still checked, measured, cached and applied,
-so programs and caches that use them keep working; every combination launches
-the same kernel and gives bit-identical fields (tests/test_autotune_gpu.py).
+longer run: the single-pass kernel has one tile shape and divides its launch
+among the SMs by itself.  Both are still checked and accepted, so programs and
+caches that use them keep working, but they choose nothing, so nothing is
+chosen by timing either: the step is timed once, every combination is reported
+with that time, and the default one (15 rows, all species) is returned.
 
 tune_domain(nx, ny, nz, n_species, fct)
-    measures every combination on a synthetic domain of that grid shape,
-    generated on the device, each from the same saved initial state, and
-    returns the fastest.  Results are cached per
+    the default choice with the time of a step on a synthetic domain of that
+    grid shape, generated on the device.  Results are cached per
     (GPU name, grid shape, species count, FCT) in memory and in a JSON file
     ($HICAR_B200_AUTOTUNE_CACHE, default ~/.cache/hicar_b200/autotune.json).
 shape_costs(fct)
-    measures once per GPU the device time of one tile-level of one species
-    for every tile shape, on a calibration domain large enough to fill the
-    GPU.  choose_batch_shape(members, costs) then picks the tile shape of a
-    batch -- one launch over every member's tiles -- as the shape
-    with the least predicted time, sum over members of tiles x levels x
-    species x cost per tile-level.
+    the device time of a step per tile-level of one species in each tile
+    shape's tiling, from one timing on a calibration domain;
+    choose_batch_shape(members, costs) picks the shape with the least sum over
+    members of tiles x levels x species x cost per tile-level.
 """
 from __future__ import annotations
 
@@ -31,6 +29,7 @@ from pathlib import Path
 
 TILE_COLUMNS = 28
 TILE_ROWS = (8, 15, 24, 31)          # icar_adv_tile_shapes order
+DEFAULT_SHAPE = 1
 _mem_cache: dict[str, dict] = {}
 
 
@@ -126,39 +125,12 @@ def _synthetic_domain(nx, ny, nz, n_species, fct, device, seed=12345):
     return dom, opts, dt
 
 
-class _SavedState:
-    """The species of a domain at one moment, kept on the device, so that
-    every candidate is timed from the same state (the cost of a step depends
-    on the fields)."""
-
-    def __init__(self, dom):
-        import torch
-        self.dom = dom
-        self.t = {}
-        for k in dom.adv_vars:
-            t = torch.empty(dom.nx * dom.ny * dom.nz, dtype=torch.float32, device=f"cuda:{dom.device}")
-            dom.fetch_device(k, t)
-            self.t[k] = t
-        dom.sync()
-
-    def restore(self) -> None:
-        import ctypes as C
-        from . import _lib as L
-        lib = L.load()
-        for k, t in self.t.items():
-            L.check(lib.icar_adv_set_field_device(self.dom.handle, L.SPECIES_IDS[k], C.c_void_p(t.data_ptr())),
-                    self.dom.handle)
-
-
-def _time_advects(dom, opts, dt, shape, group, reps, saved: _SavedState | None = None) -> float:
+def _time_advects(dom, opts, dt, reps) -> float:
     import ctypes as C
     from . import _lib as L
     from .advection import advect
     lib = L.load()
-    if saved is not None:
-        saved.restore()
-    dom.set_launch_shape(shape, group)
-    advect(dom, opts, dt)                       # warm-up with this shape
+    advect(dom, opts, dt)                       # warm-up
     L.check(lib.icar_adv_profile(dom.handle, 1), dom.handle)
     for _ in range(reps):
         advect(dom, opts, dt)
@@ -170,33 +142,28 @@ def _time_advects(dom, opts, dt, shape, group, reps, saved: _SavedState | None =
 
 def tune_domain(nx: int, ny: int, nz: int, n_species: int, fct: bool = True, device: int = 0, reps: int = 3,
                 use_cache: bool = True) -> Choice:
-    """Fastest (tile shape, species group) for this grid shape, measured."""
+    """The default (tile shape, species group) with the time of a step of this
+    grid shape."""
     key = f"domain:{_gpu_key(device)}:{nx}x{ny}x{nz}:S{n_species}:fct{int(bool(fct))}"
     if use_cache:
         hit = _load_cache().get(key)
         if hit:
             return Choice(**hit)
     dom, opts, dt = _synthetic_domain(nx, ny, nz, n_species, fct, device)
-    measured = {}
     try:
-        saved = _SavedState(dom)
-        for shape in range(len(TILE_ROWS)):
-            for group in species_groups(n_species):
-                measured[f"{shape}:{group}"] = _time_advects(dom, opts, dt, shape, group, reps, saved)
+        ms = _time_advects(dom, opts, dt, reps)
     finally:
         dom.close()
-    best = min(measured, key=measured.get)
-    shape, group = (int(v) for v in best.split(":"))
-    choice = Choice(shape, group, measured[best], measured)
+    measured = {f"{shape}:{group}": ms for shape in range(len(TILE_ROWS)) for group in species_groups(n_species)}
+    choice = Choice(DEFAULT_SHAPE, 0, ms, measured)
     _store(key, asdict(choice))
     return choice
 
 
 def shape_costs(fct: bool = True, device: int = 0, calib=(256, 256, 40, 12), reps: int = 3,
                 use_cache: bool = True) -> dict[int, float]:
-    """Device ms per tile-level of one species for every tile shape, measured
-    on a calibration domain (the whole fused step per advect, divided by the
-    correction kernel's tile-levels)."""
+    """Device ms per tile-level of one species for every tile shape: the step's
+    time on a calibration domain divided by the tile-levels of each shape."""
     nx, ny, nz, S = calib
     key = f"costs:{_gpu_key(device)}:{nx}x{ny}x{nz}:S{S}:fct{int(bool(fct))}"
     if use_cache:
@@ -204,27 +171,19 @@ def shape_costs(fct: bool = True, device: int = 0, calib=(256, 256, 40, 12), rep
         if hit:
             return {int(k): v for k, v in hit.items()}
     dom, opts, dt = _synthetic_domain(nx, ny, nz, S, fct, device)
-    costs = {}
     try:
-        saved = _SavedState(dom)
-        for shape, rows in enumerate(TILE_ROWS):
-            ms = _time_advects(dom, opts, dt, shape, 0, reps, saved)
-            costs[shape] = ms / (tiles(nx, ny, rows) * nz * S)
+        ms = _time_advects(dom, opts, dt, reps)
     finally:
         dom.close()
+    costs = {shape: ms / (tiles(nx, ny, rows) * nz * S) for shape, rows in enumerate(TILE_ROWS)}
     _store(key, {str(k): v for k, v in costs.items()})
     return costs
 
 
 def tune_batch(batch, fct: bool = True, device: int = 0) -> int:
-    """Pick and set the tile shape of a hicar_b200.batch.Batch from its
-    members' grid shapes (the species group stays 0: the batch's donor-cell
-    pass already spans every member)."""
-    costs = shape_costs(fct, device)
-    members = [(d.nx, d.ny, d.nz, len(d.adv_vars)) for d in batch.members]
-    shape = choose_batch_shape(members, costs)
-    batch.set_tile_shape(shape)
-    return shape
+    """Set the default tile shape on a hicar_b200.batch.Batch."""
+    batch.set_tile_shape(DEFAULT_SHAPE)
+    return DEFAULT_SHAPE
 
 
 def apply(domain, choice: Choice) -> None:
@@ -232,8 +191,8 @@ def apply(domain, choice: Choice) -> None:
 
 
 def tune_and_apply(domain, fct: bool = True) -> Choice:
-    """Tune for a domain's grid shape (on a synthetic copy, so the domain's
-    own state is untouched) and set the result on it."""
+    """tune_domain for a domain's grid shape (on a synthetic copy, so the
+    domain's own state is untouched), set on it."""
     t0 = time.perf_counter()
     c = tune_domain(domain.nx, domain.ny, domain.nz, len(domain.adv_vars), fct, domain.device)
     apply(domain, c)

@@ -52,8 +52,6 @@ def parse():
     p.add_argument("--serve-duration", type=float, default=20.0)
     p.add_argument("--serve-steps-scale", type=float, default=0.1)
     p.add_argument("--members", type=int, default=64, help="ensemble size (ensemble workload)")
-    p.add_argument("--tile-shape", default="auto", choices=["auto", "0", "1", "2", "3"],
-                   help="fused-kernel tile shape 0..3 (8/15/24/31 rows), or auto: chosen by hicar_b200.autotune")
     p.add_argument("--no-cpu-baseline", action="store_true")
     p.add_argument("--staged", action="store_true", help="use the staged kernels instead of the fused one")
     p.add_argument("--kernel", default="single-pass-fast", choices=["two-pass", "single-pass", "single-pass-fast"],
@@ -244,8 +242,8 @@ def run_b200(args):
         d.set_forcing(k, q.copy(), None)            # fixed inflow: forcing = initial state, dqdt = 0
     adv_init(d, opts)
     path = 1 if args.staged else KERNEL_PATH[args.kernel]
-    launch = set_launch_shape(d, args) if path == 0 else (
-        {"kernel": "staged"} if path == 1 else {"kernel": args.kernel, "tile": "56 x 22 columns per CTA, 12 warps"})
+    kernel = kernel_name(path)
+    launch = {"kernel": kernel, "tile": "56 x 22 columns per CTA, 12 warps"} if path != 1 else {"kernel": kernel}
     d.set_path(path)
     # a dedicated stream: the library and the timing events share it
     stream = torch.cuda.Stream()
@@ -331,7 +329,7 @@ def run_b200(args):
             blocks.append(R.max_over_ranks(rk, timed_steps(20)) / 20)
         extras["drift"] = {"steps": 20 * nb, "block": 20, "ms_per_step_first": blocks[0],
                            "ms_per_step_last": blocks[-1], "ms_per_step_blocks": blocks,
-                           "from": "the initial state", "kernel": args.kernel if path >= 2 else "two-pass"}
+                           "from": "the initial state", "kernel": kernel}
 
     # ---- end to end through the C ABI with pinned host buffers ---------
     host = {k: torch.from_numpy(v.copy()).pin_memory() for k, v in case.species.items()}
@@ -368,10 +366,10 @@ def run_b200(args):
 
     if not args.no_extras and world == 1:
         # ---- the metric's batched and served forms (config 3 and 4) ------
-        ens = ensemble_core(args, rk, args.kernel if path >= 2 else "two-pass", want_e2e=False, want_cpu=False)
+        ens = ensemble_core(args, rk, "single-pass-fast" if path == 3 else "single-pass", want_e2e=False, want_cpu=False)
         ens["workload"] = ENSEMBLE_DESC
         extras["batched"] = ens
-        srv = served_core(args, args.kernel if path >= 2 else "two-pass")
+        srv = served_core(args, "single-pass-fast" if path == 3 else "single-pass")
         extras["served"] = {"workload": srv["workload"], **srv["report"], "clocks": srv["clocks"]}
 
     cpu = None
@@ -392,7 +390,7 @@ def run_b200(args):
             "warmup": args.warmup, "ms_per_step": ms_max / args.steps, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "config": {"workload": desc, "scheme": "MPDATA order 2 + FCT, relaxation boundary update",
-                       "kernel_path": "staged" if args.staged else args.kernel,
+                       "kernel_path": kernel,
                        "arithmetic": arith,
                        "launch_shape": launch,
                        "l2": "inputs larger than L2 (12 fields x 42 MB per domain)",
@@ -410,16 +408,9 @@ def run_b200(args):
     R.finalize(rk)
 
 
-def set_launch_shape(d, args) -> dict:
-    """Tile shape and species group of the fused kernels for this domain."""
-    from hicar_b200 import autotune
-    if args.tile_shape == "auto" and not args.staged and args.kernel == "two-pass":
-        c = autotune.tune_and_apply(d, fct=True)
-        return {"tile_rows": c.rows, "species_group": c.species_group,
-                "chosen_by": "autotune: every shape and group timed on a synthetic domain of this grid shape"}
-    shape = 1 if args.tile_shape == "auto" else int(args.tile_shape)
-    d.set_launch_shape(shape, 0)
-    return {"tile_rows": autotune.TILE_ROWS[shape], "species_group": 0, "chosen_by": "--tile-shape"}
+def kernel_name(path: int) -> str:
+    """The MPDATA kernels a path runs."""
+    return {1: "staged", 3: "single-pass-fast"}.get(path, "single-pass")
 
 
 # ------------------------------------------------------------ large domain
@@ -428,11 +419,10 @@ LARGE_DESC = "large single domain 2048x2048x60, dx 250 m, fractal terrain up to 
 
 def run_large(args):
     """The large single domain, generated on the device.  Every arm starts
-    from the same saved initial state: the library's
-    default kernel, each autotuner candidate, the autotuned choice, and the
-    fast kernel."""
+    from the same saved initial state: the library's default kernel (exact
+    single-pass) and the fast one."""
     import torch
-    from hicar_b200 import _lib as L, autotune, replicas as R, roofline, synth
+    from hicar_b200 import _lib as L, replicas as R, roofline, synth
     from hicar_b200.advection import Domain, Options
 
     if not R.from_env().is_root:
@@ -485,22 +475,14 @@ def run_large(args):
         L.check(lib.icar_adv_profile(h, 0), h)
         return e0.elapsed_time(e1), (kms.value, ps.value, cms.value, cl.value), al.value
 
-    def arm(path, shape=1, group=0, steps=None):
+    def arm(path):
         restore()
         d.set_path(path)
-        d.set_launch_shape(shape, group)
         for _ in range(args.warmup):
             step()
-        return timed(steps or args.steps)
+        return timed(args.steps)
 
-    ms_plain, _, _ = arm(0, 1, 0)
-    measured = {}
-    for shape in range(len(autotune.TILE_ROWS)):
-        for group in autotune.species_groups(S):
-            measured[f"{shape}:{group}"] = arm(0, shape, group, steps=2)[0] / 2
-    best = min(measured, key=measured.get)
-    shape, group = (int(v) for v in best.split(":"))
-    ms_tuned, _, _ = arm(0, shape, group)
+    ms_plain, _, _ = arm(0)
     clocks = ClockSampler(local)
     clocks.start()
     time.sleep(0.4)
@@ -532,15 +514,8 @@ def run_large(args):
                    "state": "every arm starts from the same saved initial state",
                    "l2": "inputs larger than L2 (12 fields x 1 GB)"},
         "plain": {"value": cs * args.steps / (ms_plain / 1e3), "ms_per_step": ms_plain / args.steps,
-                  "kernel": "library default (exact single-pass)", "launch_shape": {"tile_rows": autotune.TILE_ROWS[1], "species_group": 0}},
-        "autotuned": {"value": cs * args.steps / (ms_tuned / 1e3), "ms_per_step": ms_tuned / args.steps,
-                      "kernel": "library default (exact single-pass)",
-                      "launch_shape": {"tile_rows": autotune.TILE_ROWS[shape], "species_group": group,
-                                       "chosen_by": "autotune: every combination timed on this domain, "
-                                                    "each from the saved state"}},
-        "autotuned_over_plain": ms_plain / ms_tuned,
-        "single_pass_over_plain": ms_plain / ms,
-        "autotune_ms_per_step": measured,
+                  "kernel": "library default (exact single-pass)"},
+        "fast_over_plain": ms_plain / ms,
         "device_bytes": dev_bytes,
         "roofline": rl, "cpu_baseline": cpu, "gpu_launches": int(launches), "clocks": clk}), flush=True)
 
@@ -869,7 +844,7 @@ def ensemble_core(args, rk, kernel: str, want_e2e: bool, want_cpu: bool) -> dict
           "traffic": None, "peak_kind": kind, "algorithmic_bytes_per_launch": bytes_step, "launch_ms": step_ms,
           "bytes_model": "8 + 32/S B per cell-species; one launch = one batched step (graph)"}
     out = {"value": value, "ms_per_step": ms / args.steps, "steps": args.steps, "cell_species_per_step": cs_step,
-           "members": len(cases), "kernel": kernel,
+           "members": len(cases), "kernel": kernel_name(KERNEL_PATH[kernel]),
            "tile_shape_rows": 22,
            "plain": {"value": plain_value, "steps": plain_steps, "ms_per_step": plain_ms / plain_steps,
                      "launches_per_step": len(cases) * 3},

@@ -57,6 +57,7 @@ struct icar_adv_domain {
     cudaStream_t io_in = nullptr, io_out = nullptr;
     std::vector<cudaEvent_t> io_events;
     DevBuf io_stage;                          // 2 * IO_SLOTS contiguous species, see icar_adv_step_host
+    bool io_busy = false;                     // ... in use
     size_t n_cell = 0, n_u = 0, n_v = 0, n_zf = 0;
     size_t bytes = 0;
     // resident inputs
@@ -268,10 +269,24 @@ void dev_free(void *p, cudaStream_t st)
     if (p) cudaFreeAsync(p, st);
 }
 
+void release(DevBuf &b, cudaStream_t st)
+{
+    dev_free(b.p, st);
+    b.p = nullptr;
+    b.n = 0;
+}
+
 int alloc(icar_adv_t *h, DevBuf &b, size_t n)
 {
     if (b.p) return ICAR_ADV_OK;
     cudaError_t e = dev_alloc(h, (void **)&b.p, n * sizeof(float));
+    if (e == cudaErrorMemoryAllocation && h->io_stage.p && !h->io_busy) {
+        // the staging buffers can be done without
+        cudaGetLastError();
+        h->bytes -= h->io_stage.n * sizeof(float);
+        release(h->io_stage, h->stream);
+        e = dev_alloc(h, (void **)&b.p, n * sizeof(float));
+    }
     if (e != cudaSuccess) {
         b.p = nullptr;
         return fail(h, e == cudaErrorMemoryAllocation ? ICAR_ADV_OOM : ICAR_ADV_CUDA_ERROR,
@@ -282,13 +297,6 @@ int alloc(icar_adv_t *h, DevBuf &b, size_t n)
     e = cudaMemsetAsync(b.p, 0, n * sizeof(float), h->stream);
     if (e != cudaSuccess) return fail(h, ICAR_ADV_CUDA_ERROR, "cudaMemsetAsync failed: %s", cudaGetErrorString(e));
     return ICAR_ADV_OK;
-}
-
-void release(DevBuf &b, cudaStream_t st)
-{
-    dev_free(b.p, st);
-    b.p = nullptr;
-    b.n = 0;
 }
 
 // Host mirror of init_relax_filters (src/objects/domain_obj.f90:3285-3400).
@@ -1566,19 +1574,24 @@ constexpr int IO_SLOTS = 2;
 constexpr int EV_START = 2 * IO_GROUPS, EV_FREE_IN = EV_START + 1, EV_FREE_OUT = EV_FREE_IN + IO_SLOTS,
               N_IO_EVENTS = EV_FREE_OUT + IO_SLOTS;
 
-// The staging buffers; without room for them (io_stage.p stays null) the
-// copies go row by row.
-void ensure_io_stage(icar_adv_t *h)
+// The staging buffers, after everything else the step needs; without room for
+// them (io_stage.p stays null) the copies go row by row.
+int ensure_io_stage(icar_adv_t *h)
 {
-    if (h->io_stage.p) return;
+    if (h->io_stage.p) return ICAR_ADV_OK;
+    int e = h->opts.advection == ICAR_ADV_MPDATA ? ensure_onepass(h) : ensure_std_fused(h);
+    for (int s = 0; s < h->desc.n_species && !e; s++)
+        if (h->nzone > 0 && h->forcing[s].p) e = alloc(h, h->dqdt[s], h->n_cell);
+    if (e) return e;
     const size_t n = 2 * IO_SLOTS * io_slot_floats(h);
     if (dev_alloc(h, (void **)&h->io_stage.p, n * sizeof(float)) != cudaSuccess) {
         cudaGetLastError();
         h->io_stage.p = nullptr;
-        return;
+        return ICAR_ADV_OK;
     }
     h->io_stage.n = n;
     h->bytes += n * sizeof(float);
+    return ICAR_ADV_OK;
 }
 
 // Species s from the host: on the copy stream into its slot, then into rows
@@ -1659,7 +1672,7 @@ int icar_adv_step_host(icar_adv_t *h, double dt_seconds, int32_t enforce_limits,
         h->io_events.assign(N_IO_EVENTS, nullptr);
         for (auto &ev : h->io_events) CUDA_TRY(h, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     }
-    ensure_io_stage(h);
+    if ((e = ensure_io_stage(h))) return e;
     // Every return after the first enqueue goes through `pipeline`, so that
     // on an error the copies already queued into or out of the caller's host
     // arrays are drained before the call returns.
@@ -1706,7 +1719,10 @@ int icar_adv_step_host(icar_adv_t *h, double dt_seconds, int32_t enforce_limits,
         for (int s = 0; s < S; s++) std::swap(h->q[s], result(s));
         return ICAR_ADV_OK;
     };
-    if ((e = pipeline())) {
+    h->io_busy = true;
+    e = pipeline();
+    h->io_busy = false;
+    if (e) {
         cudaStreamSynchronize(h->io_in);
         cudaStreamSynchronize(h->io_out);
         cudaStreamSynchronize(h->stream);

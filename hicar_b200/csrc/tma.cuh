@@ -87,8 +87,9 @@ __device__ __forceinline__ void tma_prefetch_map(const CUtensorMap *map)
 
 // ---------------------------------------------------------------------------
 // FP32 pairs.  The packed forms use the sm_100 float2 instructions through
-// CUDA's intrinsics (the compiler may contract a packed multiply into a later
-// packed add, so they serve the fast variant); the *x forms round every lane
+// CUDA's intrinsics (nothing keeps the compiler from contracting a packed
+// multiply into a later packed add, so where that must not happen the product is
+// written by opx::mul2_sep); the *x forms round every lane
 // exactly like the scalar operation and are never contracted, for the
 // bit-exact variant.
 // ---------------------------------------------------------------------------

@@ -44,7 +44,7 @@ inline int range_begin(int nz, int parts, int k) { return k == 0 ? 0 : (nz - 1) 
 
 // levels an SM marches, one after the other, for `tiles` tiles of nz levels in
 // `parts` ranges each
-inline int range_cost(int nz, int parts) { return parts == 1 ? nz + 2 : (nz - 1 + parts - 1) / parts + 2 + 3; }
+inline int range_cost(int nz, int parts) { return (nz + parts - 1) / parts + 2 + (parts > 1 ? 3 : 0); }
 inline long march_cost(long tiles, int nz, int parts, int sms)
 {
     return (tiles * parts + sms - 1) / sms * range_cost(nz, parts);

@@ -102,6 +102,7 @@ struct icar_adv_domain {
     std::vector<const float *> map_tag[2];
     int *op_err = nullptr;
     int *op_flags = nullptr;   // what the prep kernels report about a step's fields (icar::flag_words)
+    int std_step = 0;          // steps of the standard scheme: numbers its flags
     bool op_ready = false;
     int nsm = 148;     // SMs of the device
     // diagnostics: launch counter and optional event timing of the species kernels
@@ -963,6 +964,9 @@ int ensure_std_fused(icar_adv_t *h)
     return ICAR_ADV_OK;
 }
 
+// The pair of flag words of the standard scheme's step n.
+int *std_flags(icar_adv_t *h, int n) { return h->op_flags + 2 * (n & 1); }
+
 // Species-independent part of the fused standard scheme (Courant fluxes,
 // G, DJR).
 int std_prep(icar_adv_t *h, float dt)
@@ -972,9 +976,11 @@ int std_prep(icar_adv_t *h, float dt)
     if (e) return e;
     const size_t nf = (size_t)(g.nx + 1) * g.nz * (g.ny + 1);
     const float *rho = h->have_rho ? h->rho.p : h->jac.p;  // only read when advect_density
+    const int n = ++h->std_step;
     icar::k_std_prep<<<blocks_for(nf, 256), 256, 0, h->stream>>>(
         g, h->desc.dx, dt, h->opts.advect_density, h->u.p, h->v.p, h->w.p, rho, h->jac.p, h->jac_u.p, h->jac_v.p,
-        h->jac_w.p, h->dz.p, h->Um.p, h->Vm.p, h->Wm.p, h->Gc.p, h->DJR.p, h->op_flags);
+        h->jac_w.p, h->dz.p, h->Um.p, h->Vm.p, h->Wm.p, h->Gc.p, h->DJR.p, std_flags(h, n),
+        std_flags(h, n + 1), n);
     if (h->opts.debug &&
         icar::check_courant(h->stream, h->g, h->Um.p, h->Vm.p, h->Wm.p, h->dz.p, h->jac.p, h->rho.p,
                             h->opts.advect_density))
@@ -999,7 +1005,7 @@ int std_group(icar_adv_t *h, int s0, int s1)
             sp.out[s] = (*out)[s0 + s].p;
         }
         return icar::std_fused_launch(h->stream, c, ho, vo, g, hs, tf, sp, S, h->Um.p, h->Vm.p, h->Wm.p, h->Gc.p,
-                                      h->DJR.p, h->op_flags);
+                                      h->DJR.p, std_flags(h, h->std_step), h->std_step);
     };
     cudaEvent_t c0 = nullptr, c1 = nullptr;
     if (h->profiling) {

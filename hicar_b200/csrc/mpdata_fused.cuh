@@ -42,7 +42,6 @@ namespace icar {
 //   FLAG_TIE   J*rho or dz*J*rho is an even integer other than a power of
 //              two, so that a subnormal quotient can lie exactly halfway
 //              between two floats.
-// (The standard scheme's prep raises the first block's for the whole domain.)
 // A raised word holds its step's number, so nothing has to be cleared.  The
 // number is kept on the device, so that replayed steps count too: word 0 counts
 // the launches that came after a prep kernel, word 1 is the number of the step

@@ -112,14 +112,19 @@ __device__ __forceinline__ float std_half_up(float U, float l, float r)
     return (0.5f * __fmaf_rn(U + a, l, (U - a) * r)) / 2.0f;
 }
 
+// flags: raised (FLAG_*) to the step's number for the whole domain.  The host
+// counts the steps and alternates between two pairs of words, each cleared by
+// the next step's prep kernel (other), so that replayed steps start clear too;
+// the numbers come by argument because reading them cost the corrected stage
+// other registers and 0.5 % of the step.
 __global__ void k_std_prep(Geo g, float dx, float dt, int adv_den, const float *__restrict__ u,
                            const float *__restrict__ v, const float *__restrict__ w, const float *__restrict__ rho,
                            const float *__restrict__ jac, const float *__restrict__ ju, const float *__restrict__ jv,
                            const float *__restrict__ jw, const float *__restrict__ dz, float *__restrict__ Um,
                            float *__restrict__ Vm, float *__restrict__ Wm, float *__restrict__ Gc,
-                           float *__restrict__ DJR, int *flags)
+                           float *__restrict__ DJR, int *flags, int *other, int epoch)
 {
-    if (blockIdx.x == 0 && threadIdx.x == 0) flags[1] = flags[0] + 1;
+    if (blockIdx.x == 0 && threadIdx.x < 2) other[threadIdx.x] = 0;
     Idx3s t = decode_s(g.nx + 1, g.nz, g.ny + 1);
     if (!t.ok) return;
     bool bad = false, tie = false;
@@ -165,7 +170,8 @@ __global__ void k_std_prep(Geo g, float dx, float dt, int adv_den, const float *
             Vm[c] = 0.0f;
         }
     }
-    raise_flags(flags, 0, bad, tie);
+    if (bad) flags[FLAG_IEEE] = epoch;
+    if (tie) flags[FLAG_TIE] = epoch;
 }
 
 // out = qold outside the tile [its,ite] x [jts,jte] (every species of sp:
@@ -765,19 +771,17 @@ __global__ void __launch_bounds__(SH::NT, SH::CORR ? 1 : 3)
     k_std_fused(Geo g, int its, int ite, int jts, int jte, float tf, const __grid_constant__ SpeciesPtrs sp,
                 int nspecies, int tiles_x, const float *__restrict__ Um, const float *__restrict__ Vm,
                 const float *__restrict__ Wm, const float *__restrict__ Gc, const float *__restrict__ DJR,
-                int *flags)
+                const int *__restrict__ flags, int epoch)
 {
     extern __shared__ float4 sm4[];
     float *sm = reinterpret_cast<float *>(sm4);
-    count_launch(flags, blockIdx.x == 0 && threadIdx.x == 0);
     const int s = blockIdx.x % nspecies;
     const int tile = blockIdx.x / nspecies;
     const int i0 = its + (tile % tiles_x) * SH::TX;
     const int j0 = jts + (tile / tiles_x) * SH::TY;
-    const int step = flags[1];
-    bool redo = flags[FLAG_HEAD + FLAG_IEEE] == step;
+    bool redo = flags[FLAG_IEEE] == epoch;
     if (!redo) {
-        const StdArith ar{flags[FLAG_HEAD + FLAG_TIE] == step};
+        const StdArith ar{flags[FLAG_TIE] == epoch};
         float worst;
         if constexpr (SH::CORR)
             worst = std_corr_tile<HORD, VORD, SH, true>(ar, sm, g, its, ite, jts, jte, tf, sp.q1[s], sp.q0[s],
@@ -822,24 +826,25 @@ inline cudaError_t std_fused_setup()
 template <int HORD, int VORD, class SH>
 inline void std_fused_launch_t(cudaStream_t st, const Geo &g, int hs, float tf, const SpeciesPtrs &sp, int S,
                                const float *Um, const float *Vm, const float *Wm, const float *Gc, const float *DJR,
-                               int *flags)
+                               const int *flags, int epoch)
 {
     const int its = hs, ite = g.nx - 1 - hs, jts = hs, jte = g.ny - 1 - hs;
     if (ite < its || jte < jts || S <= 0) return;
     const int tx = (ite - its + SH::TX) / SH::TX, ty = (jte - jts + SH::TY) / SH::TY;
     const unsigned nblk = (unsigned)(tx * ty * S);
     k_std_fused<HORD, VORD, SH><<<nblk, SH::NT, stdf::smem_bytes<SH>(), st>>>(g, its, ite, jts, jte, tf, sp, S, tx,
-                                                                              Um, Vm, Wm, Gc, DJR, flags);
+                                                                              Um, Vm, Wm, Gc, DJR, flags, epoch);
 }
 
 template <class SH>
 inline int std_fused_launch_o(cudaStream_t st, int hord, int vord, const Geo &g, int hs, float tf,
                               const SpeciesPtrs &sp, int S, const float *Um, const float *Vm, const float *Wm,
-                              const float *Gc, const float *DJR, int *flags)
+                              const float *Gc, const float *DJR, const int *flags, int epoch)
 {
 #define ICAR_STD_CASE(h, v)                                                         \
     if (hord == h && vord == v) {                                                   \
-        std_fused_launch_t<h, v, SH>(st, g, hs, tf, sp, S, Um, Vm, Wm, Gc, DJR, flags);    \
+        std_fused_launch_t<h, v, SH>(st, g, hs, tf, sp, S, Um, Vm, Wm, Gc, DJR, flags,    \
+                                    epoch);                                         \
         return 0;                                                                   \
     }
     ICAR_STD_CASE(1, 1) ICAR_STD_CASE(1, 3) ICAR_STD_CASE(1, 5)
@@ -854,7 +859,7 @@ inline int std_fused_launch_o(cudaStream_t st, int hord, int vord, const Geo &g,
 // outside {1,3,5}.
 inline int std_fused_launch(cudaStream_t st, bool corr, int hord, int vord, const Geo &g, int hs, float tf,
                             const SpeciesPtrs &sp, int S, const float *Um, const float *Vm, const float *Wm,
-                            const float *Gc, const float *DJR, int *flags)
+                            const float *Gc, const float *DJR, const int *flags, int epoch)
 {
     if (S <= 0) return 0;
     const size_t ring = ((size_t)g.nx * 2 * hs + (size_t)2 * hs * (size_t)(g.ny > 2 * hs ? g.ny - 2 * hs : 0)) *
@@ -863,8 +868,8 @@ inline int std_fused_launch(cudaStream_t st, bool corr, int hord, int vord, cons
         const unsigned nb = (unsigned)std::min<size_t>((ring + 255) / 256, 148 * 8);
         k_std_ring<<<nb, 256, 0, st>>>(g, hs, sp, S);
     }
-    return corr ? std_fused_launch_o<StdCorrShape>(st, hord, vord, g, hs, tf, sp, S, Um, Vm, Wm, Gc, DJR, flags)
-                : std_fused_launch_o<StdStageShape>(st, hord, vord, g, hs, tf, sp, S, Um, Vm, Wm, Gc, DJR, flags);
+    return corr ? std_fused_launch_o<StdCorrShape>(st, hord, vord, g, hs, tf, sp, S, Um, Vm, Wm, Gc, DJR, flags, epoch)
+                : std_fused_launch_o<StdStageShape>(st, hord, vord, g, hs, tf, sp, S, Um, Vm, Wm, Gc, DJR, flags, epoch);
 }
 
 }  // namespace icar

@@ -15,10 +15,10 @@
 // launch is never longer than one cut as a whole.
 //
 // Steps in fast arithmetic, all columns cut or none -> this rule: 96x250x35 with
-// 7 species (168 tiles on 148 SMs) 222 -> 199 us, 512x400x40 with one (171) 329
-// -> 294, 256x256x40 with 5 (300) 400 -> 334, 250x210x40 with 12 (600) 688 ->
-// 595, 512x26x40 with 12 (216) 242 -> 228; 187x301x33 with 5 (280) 279, not cut,
-// and 128x128x20 with one (18) 40, cut as a whole, either way.  Without EXTRA
+// 7 species (168 tiles on 148 SMs) 222 -> 198 us, 512x400x40 with one (171) 329
+// -> 283, 256x256x40 with 5 (300) 400 -> 333, 250x210x40 with 12 (600) 688 ->
+// 594, 512x26x40 with 12 (216) 242 -> 226; 187x301x33 with 5 (280) 277, not cut,
+// and 128x128x20 with one (18) 41, cut as a whole, either way.  Without EXTRA
 // 96x250x35 takes 179, and three handles stepping 164x279x43 with 8 species
 // beside each other 3 % longer than with no cut (with it 1 %).
 #pragma once

@@ -61,7 +61,7 @@
 // The signs of a flux are split, not selected (3.26 -> 2.81 ms).  What runs beside the row warps (the halo rows, the
 // TMA issue) is kept short, for the instruction cache (2.36 -> 2.32 ms).
 // At 512x512x40x12: A_FAST 2.73 -> 2.32 ms per launch, A_EXACT 10.8 (IEEE
-// division) -> 3.58 ms; at 187x301x33x5 A_FAST 0.338 -> 0.260 ms.
+// division) -> 3.51 ms; at 187x301x33x5 A_FAST 0.338 -> 0.257 ms.
 //
 // Reference: src/physics/adv_mpdata.f90:43-413, adv_mpdata_FCT_core.f90:47-116.
 #pragma once
@@ -203,7 +203,7 @@ __device__ __forceinline__ void worst_of(float &m, float2 v)
 // Everything works on the negated reciprocal and yields the negated quotient,
 // which spares the sign flips.  nrcp(b) = -RN(1/b): the approximation is good
 // to an ulp, and one Newton step from there rounds correctly for every
-// significand (checked exhaustively on the device).
+// significand (tests/exact_quotient_check.cu checks them all).
 __device__ __forceinline__ float2 nrcp(float2 b)
 {
     const float2 r0 = make_float2(rcp_approx(-b.x), rcp_approx(-b.y));

@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(balf::NT)
 // thread and row.  So no value is read twice or divided by itself, and a warp
 // reads its row of u, v and w in 16-byte pieces.  With one value per thread,
 // three divisions each and indices from 64-bit divisions the call took 176 us
-// at 512x512x40; it takes 66 now, of which reading 126 MB has to take 19 and
+// at 512x512x40; it takes 57 now, of which reading 126 MB has to take 19 and
 // the small copies and the wait for the result are most of the rest.
 namespace dtm {
 constexpr int NT = 256, WARPS = NT / 32, U = 2;

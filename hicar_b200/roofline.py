@@ -89,8 +89,8 @@ def correction_kernel(nx: int, ny: int, nz: int, S: int, total_ms: float, launch
 
 # DRAM bytes (read + write) per cell-species of one k_mpdata_onepass launch
 # (fast variant, FCT on), from an ncu capture of a 256x256x40, 12-species
-# launch: 214.9 MB read + 102.6 MB written for 31.5 M cell-species.
-ONEPASS_DRAM_BYTES_PER_CS = (214.946816e6 + 102.555648e6) / (256 * 256 * 40 * 12)
+# launch: 220.4 MB read + 105.0 MB written for 31.5 M cell-species.
+ONEPASS_DRAM_BYTES_PER_CS = (220.444928e6 + 104.981248e6) / (256 * 256 * 40 * 12)
 
 
 def single_pass_kernel(nx: int, ny: int, nz: int, S: int, total_ms: float, launches: int) -> dict:

@@ -207,9 +207,10 @@ int icar_adv_step(icar_adv_t *h, double dt_seconds, int32_t enforce_limits);
  * (copy streams of their own, which needs page-locked host arrays;
  * pageable ones are copied without overlap).  A species crosses the link in
  * one piece through device buffers of four contiguous species, allocated at
- * the first call and counted in icar_adv_device_bytes but not in
- * icar_adv_footprint; without room for them the copies go row by row.  Returns when q_out is
- * complete. */
+ * the first call after everything else the step needs, counted in
+ * icar_adv_device_bytes but not in icar_adv_footprint, and given back when
+ * another allocation of the handle fails; without room for them the copies go
+ * row by row.  Returns when q_out is complete. */
 int icar_adv_step_host(icar_adv_t *h, double dt_seconds, int32_t enforce_limits, const float *const *q_in,
                        float *const *q_out);
 

@@ -93,4 +93,4 @@ def test_a_launch_just_above_a_wave_costs_little_more_than_the_wave(path):
         d.set_path(path)
         t.append(microseconds(lambda: advect(d, opts, dt), d.sync, n=20))
         d.close()
-    assert t[1] < 1.35 * t[0], t
+    assert t[1] < 1.38 * t[0], t   # a sixth more tiles; with a second wave of whole columns 1.42 and 1.47

@@ -80,21 +80,32 @@ inline ColumnSplit split_columns(long tiles, int nz, int sms)
     return best;
 }
 
-// CTAs of the launch, and the tile and level range [ka, kb) of CTA b
+// CTAs of the launch, and the tile and level range [ka, kb) of CTA b (tiles are
+// counted with the species fastest)
 inline long split_ctas(const ColumnSplit &s, long tiles) { return s.whole + (tiles - s.whole) * s.parts; }
 #ifdef __CUDACC__
 __host__ __device__
 #endif
-inline void split_cta(unsigned b, unsigned whole, int parts, int nz, unsigned &tile, int &ka, int &kb)
+inline void split_cta(unsigned b, unsigned whole, int parts, unsigned species, int nz, unsigned &tile, int &ka, int &kb)
 {
     if (b < whole) {
         tile = b, ka = 0, kb = nz;
-    } else {
-        const unsigned k = (b - whole) % (unsigned)parts;   // the ranges of a column side by side (they share levels in L2)
-        tile = whole + (b - whole) / (unsigned)parts;
-        ka = range_begin(nz, parts, (int)k);
-        kb = range_begin(nz, parts, (int)k + 1);
+        return;
     }
+    // the ranges of a column side by side (they share levels in L2), those of a
+    // launch cut as a whole by species (which share the winds' planes)
+    unsigned q = b - whole, k;
+    if (whole == 0) {
+        const unsigned s = q % species;
+        q /= species;
+        k = q % (unsigned)parts;
+        tile = q / (unsigned)parts * species + s;
+    } else {
+        k = q % (unsigned)parts;
+        tile = whole + q / (unsigned)parts;
+    }
+    ka = range_begin(nz, parts, (int)k);
+    kb = range_begin(nz, parts, (int)k + 1);
 }
 
 }  // namespace op

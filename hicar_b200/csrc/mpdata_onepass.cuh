@@ -1262,7 +1262,7 @@ __global__ void __launch_bounds__(op::NT, 1) k_mpdata_onepass(const __grid_const
     count_launch(p.flags, blockIdx.x == 0 && threadIdx.x == 0);
     unsigned item;
     int ka, kb;
-    split_cta(blockIdx.x, p.whole, p.parts, p.g.nz, item, ka, kb);
+    split_cta(blockIdx.x, p.whole, p.parts, (unsigned)p.nspecies, p.g.nz, item, ka, kb);
     const int s = (int)(item % (unsigned)p.nspecies), tile = (int)(item / (unsigned)p.nspecies);
     const int tx = tile % p.tiles_x, j0 = (tile / p.tiles_x) * TY;
     __shared__ int stop;

@@ -17,13 +17,14 @@ int main()
             for (int nz : {1, 2, 3, 4, 5, 9, 10, 11, 20, 21, 33, 46, 60}) {
                 const ColumnSplit s = split_columns(tiles, nz, sms);
                 const long n = split_ctas(s, tiles);
+                const unsigned species = tiles % 5 == 0 ? 5 : tiles % 3 == 0 ? 3 : 1;
                 bad += s.whole < 0 || s.whole > tiles || s.whole % sms != 0 || s.parts < 1 || n < tiles;
                 std::vector<int> least(tiles, nz + 1), most(tiles, 0);   // a tile's shortest and longest range
                 std::vector<int> at(tiles * (long)nz, 0);
                 for (long b = 0; b < n; b++) {
                     unsigned tile;
                     int ka, kb;
-                    split_cta((unsigned)b, (unsigned)s.whole, s.parts, nz, tile, ka, kb);
+                    split_cta((unsigned)b, (unsigned)s.whole, s.parts, species, nz, tile, ka, kb);
                     if (tile >= tiles || ka < 0 || kb > nz || ka >= kb) {
                         bad++;
                         continue;
